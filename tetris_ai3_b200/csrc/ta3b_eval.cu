@@ -516,8 +516,12 @@ struct alignas(16) WarpShared {
     unsigned long long t_start;        // the launch's start on this warp (time budget)
     Engine eng;                        // the committed game
     Stats st;
-    uint32_t seg_off[65];              // a level's candidate segments (parent rank, child list)
-    uint32_t seg_info[64];             // rec (6) | rank k << 8 | piece << 16 | held-is-I << 20 | child << 21
+    uint32_t seg_off[65];              // a level's candidate segments (the distinct child lists)
+    uint32_t seg_info[64];             // rec (6) | list (rank * 2 + child, 6) << 8 | piece << 16 | held-is-I << 20
+                                       // | lists it stands for << 22
+    uint32_t grp0[32], grp1[32];       // per parent: the parents whose child list 0 / 1 equals its own
+                                       // (grp1 = 0: list 1 equals the parent's own list 0)
+    uint32_t merged;                   // parents whose list 1 equals their list 0
     uint32_t defer[64];                // queued (segment << 8 | placement) for the full path
     alignas(8) uint64_t kbuf[WARP];    // a level's keys above the top-K threshold, not yet merged
     // team kernels (TEAM warps per game; the game lives in the leader's area)
@@ -616,7 +620,7 @@ struct LevelAcc {
     uint64_t list;                     // top-K list (STAGE_TOPK)
     uint64_t best;                     // argmax of leaf keys and fallbacks (STAGE_LEAF)
     uint64_t best2;                    // the second-largest leaf key (tracing flavour only)
-    uint32_t lo, hi;                   // TOPK: bit k = parent k has a legal child; LEAF: bit = list legal
+    uint32_t lo, hi;                   // bit (rank * 2 + child): that child list has a legal placement
 };
 
 // keep the two largest keys (keys are unique per move, 0 = none)
@@ -642,8 +646,7 @@ __device__ __forceinline__ void warp_top2(uint64_t& b1, uint64_t& b2) {
 }
 
 __device__ __forceinline__ uint64_t candidate_key(bool leaf, float v, uint32_t info, uint32_t i) {
-    uint32_t const k = (info >> 8) & 31u, child = (info >> 21) & 1u;
-    uint32_t const pos = (k * 2u + child) * MP + i;                        // beam.hpp:296,360,423
+    uint32_t const pos = ((info >> 8) & 63u) * MP + i;                     // beam.hpp:296,360,423
     uint32_t const low = leaf ? uint32_t(ORDER_SPAN) - pos : 0xFFFFFFFFu - pos;   // beam.hpp:217-219
     return (uint64_t(ordered_bits(v)) << 32) | uint64_t(low);
 }
@@ -706,10 +709,10 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
     constexpr bool TEAMED = TEAM > 1;
     constexpr bool LAZY = TEAMED;
     LevelAcc acc{0, 0, 0, 0, 0, 0};
-    auto consume = [&](uint64_t key, uint32_t seg, uint32_t info) {
+    auto consume = [&](uint64_t key, uint32_t info) {
         if (key) {
-            ++evals;
-            uint32_t const bit = leaf ? seg : (info >> 8) & 31u;
+            evals += info >> 22;
+            uint32_t const bit = (info >> 8) & 63u;
             if (bit < 32) acc.lo |= 1u << bit;
             else acc.hi |= 1u << (bit - 32);
         }
@@ -750,12 +753,12 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
                 if (legal) {
                     uint32_t const info = ws.seg_info[entry >> 8];
                     key = candidate_key(leaf, v, info, entry & 0xFFu);
-                    consume(key, entry >> 8, info);
+                    consume(key, info);
                 }
             } else if (uint32_t(lane) < n) {
                 uint32_t const entry = dq[lane];
                 key = full_key(&ws, lut, leaf, entry);
-                consume(key, entry >> 8, ws.seg_info[entry >> 8]);
+                consume(key, ws.seg_info[entry >> 8]);
             }
             uint32_t const rem = queued - n;
             uint32_t t = 0;
@@ -784,7 +787,7 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
             bool const def = valid && st != FAST_OK;
             if (valid && st == FAST_OK) {
                 key = candidate_key(leaf, v, info, idx);
-                consume(key, sg, info);
+                consume(key, info);
             }
             uint32_t const dm = __ballot_sync(FULL_MASK, def);
             if (def) dq[queued + __popc(dm & ((1u << lane) - 1u))] = (sg << 8) | idx;
@@ -816,36 +819,135 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
     return acc;
 }
 
-// Segment table of one level: segment j = (parent rank j/2, child list j%2),
-// spanning the child piece's placement count. Returns the candidate total.
+// Segment table of one level: one segment per distinct child list, in list order (list j = parent
+// rank j / 2, child j % 2), spanning the child piece's placement count. Returns the candidate total.
+//
+// Two kept nodes often hold the same board and clear histogram: the same placements reached in another
+// order through the hold slot. Their child lists with the same piece and held-is-I flag then hold the
+// same candidates with the same values, so one of them (the lowest list, the representative) is evaluated
+// and stands for all: its evaluations count once per list (seg_info), its legality holds for each
+// (list_legal), its leaf keys beat the copies' (lower position), and in the other levels the copies of the
+// kept keys enter the top-K afterwards (expand_copies). Equality is exact: nodes are grouped by a hash of
+// the record's board words and compared word by word with their group's first node. On the generation
+// 21 % of all candidates are such copies (5 / 20 / 29 % at levels 1 / 2 / 3; 26 % in a champion's games).
+// Measured, start -> grouped: generation (10,000 sims, cap 2,000) 330.5 -> 311.5 ms, widened 64 (2,000 sims,
+// cap 200) 414.8 -> 335.1 ms, widened 32 (cap 300) 243.2 -> 194.0 ms.
+// dedup = false: every list stands for itself (the key-tracing flavour, whose second-best key may be a copy;
+// level 1 unless both root groups place the same piece, the only way to the same board there but for clears).
 __device__ __forceinline__ uint32_t build_segments(WarpShared& ws, uint32_t const* slot_piece, int tree, int level,
-                                                   uint32_t fnode, int kept, int lane) {
-    uint32_t base = 0;
+                                                   uint32_t fnode, int kept, bool dedup, int lane) {
+    bool const active = lane < kept;
+    uint32_t piece[2], held[2];
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        int const j = lane + 32 * half;
-        int const k = j >> 1;
-        uint32_t const pnode = __shfl_sync(FULL_MASK, fnode, k & 31);
-        uint32_t const cnode = (2u * pnode + uint32_t(j & 1)) & 15u;
-        uint32_t const nd = c_tables.node[tree][level][cnode];
-        uint32_t const piece = slot_piece[nd & 0xFu];
+    for (int c = 0; c < 2; ++c) {
+        uint32_t const nd = c_tables.node[tree][level][((2u * fnode) & 15u) + uint32_t(c)];
+        piece[c] = slot_piece[nd & 0xFu];
         uint32_t const held_slot = (nd >> 4) & 0xFu;
-        uint32_t const held_i = held_slot != HELD_NONE && slot_piece[held_slot] == 0u;
-        uint32_t const cnt = k < kept ? c_tables.nplace[piece] : 0u;
-        uint32_t incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t const n = __shfl_up_sync(FULL_MASK, incl, o);
-            if (lane >= o) incl += n;
-        }
-        ws.seg_off[j] = base + incl - cnt;
-        ws.seg_info[j] = uint32_t(k & 31) | (uint32_t(k & 31) << 8) | (piece << 16) | (held_i << 20) |
-                         (uint32_t(j & 1) << 21);
-        base += __shfl_sync(FULL_MASK, incl, 31);
+        held[c] = held_slot != HELD_NONE && slot_piece[held_slot] == 0u;
     }
-    if (lane == 0) ws.seg_off[64] = base;
+    uint32_t const self = 1u << lane;
+    uint32_t m0 = self, m1 = self, merged = 0;
+    if (dedup) {
+        uint32_t const* const r = ws.rec[lane];           // words 8..19: board, clears, feature totals
+        uint4 const a0 = *reinterpret_cast<uint4 const*>(r + R_BOARD), a1 = *reinterpret_cast<uint4 const*>(r + R_BOARD + 4),
+                    a2 = *reinterpret_cast<uint4 const*>(r + R_BOARD + 8);
+        uint32_t h = a0.x;
+        for (uint32_t const v : {a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z}) h = h * 0x9E3779B1u + v;
+        uint32_t const same_hash = __match_any_sync(FULL_MASK, h) & __ballot_sync(FULL_MASK, active);
+        int const first = active ? __ffs(int(same_hash)) - 1 : lane;
+        uint32_t const* const f = ws.rec[first];
+        uint4 const b0 = *reinterpret_cast<uint4 const*>(f + R_BOARD), b1 = *reinterpret_cast<uint4 const*>(f + R_BOARD + 4),
+                    b2 = *reinterpret_cast<uint4 const*>(f + R_BOARD + 8);
+        bool const same = active && ((a0.x ^ b0.x) | (a0.y ^ b0.y) | (a0.z ^ b0.z) | (a0.w ^ b0.w) | (a1.x ^ b1.x) |
+                                     (a1.y ^ b1.y) | (a1.z ^ b1.z) | (a1.w ^ b1.w) | (a2.x ^ b2.x) | (a2.y ^ b2.y) |
+                                     (a2.z ^ b2.z)) == 0u;
+        uint32_t const matches = __ballot_sync(FULL_MASK, same);
+        uint32_t const v0 = (piece[0] << 1) | held[0], v1 = (piece[1] << 1) | held[1];
+        merged = __ballot_sync(FULL_MASK, active && v0 == v1);
+        m0 = same ? same_hash & matches : self;
+        m1 = m0 & ~merged;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {                     // ... with the same piece (3 bits) and held-is-I flag
+            uint32_t const x0 = __ballot_sync(FULL_MASK, (v0 >> t) & 1u), x1 = __ballot_sync(FULL_MASK, (v1 >> t) & 1u);
+            m0 &= (v0 >> t) & 1u ? x0 : ~x0;
+            m1 &= (v1 >> t) & 1u ? x1 : ~x1;
+        }
+        if (v0 == v1) m1 = 0;
+    }
+    uint32_t const cnt0 = active && (m0 & (self - 1u)) == 0 ? c_tables.nplace[piece[0]] : 0u;
+    uint32_t const cnt1 = active && m1 && (m1 & (self - 1u)) == 0 ? c_tables.nplace[piece[1]] : 0u;
+    // candidates (low half) and segments (high half) before this lane's
+    uint32_t const own = (cnt0 + cnt1) | ((uint32_t(cnt0 != 0) + uint32_t(cnt1 != 0)) << 16);
+    uint32_t incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        uint32_t const n = __shfl_up_sync(FULL_MASK, incl, o);
+        if (lane >= o) incl += n;
+    }
+    uint32_t off = (incl - own) & 0xFFFFu, s = (incl - own) >> 16;
+    uint32_t const list = uint32_t(lane) | (uint32_t(2 * lane) << 8);
+    if (cnt0) {
+        ws.seg_off[s] = off;
+        ws.seg_info[s++] = list | (piece[0] << 16) | (held[0] << 20) | (uint32_t(__popc(m0) + __popc(m0 & merged)) << 22);
+        off += cnt0;
+    }
+    if (cnt1) {
+        ws.seg_off[s] = off;
+        ws.seg_info[s] = list | (1u << 8) | (piece[1] << 16) | (held[1] << 20) | (uint32_t(__popc(m1)) << 22);
+    }
+    ws.grp0[lane] = m0;
+    ws.grp1[lane] = m1;
+    uint32_t const all = __shfl_sync(FULL_MASK, incl, 31);
+    if (lane == 0) {
+        ws.merged = merged;
+        ws.seg_off[all >> 16] = all & 0xFFFFu;
+    }
     __syncwarp();
-    return base;
+    return all & 0xFFFFu;
+}
+
+// Bit c: parent `lane`'s child list c has a legal placement (lo, hi: the warp's bits of the lists evaluated).
+__device__ __forceinline__ uint32_t list_legal(WarpShared const& ws, uint32_t lo, uint32_t hi, int lane) {
+    uint32_t const g0 = ws.grp0[lane], g1 = ws.grp1[lane];
+    uint64_t const bits = (uint64_t(hi) << 32) | lo;
+    uint32_t const l0 = uint32_t(bits >> (2 * (__ffs(int(g0)) - 1))) & 1u;
+    uint32_t const l1 = g1 ? uint32_t(bits >> (2 * (__ffs(int(g1)) - 1) + 1)) & 1u : l0;
+    return l0 | (l1 << 1);
+}
+
+// A level's kept keys of the evaluated lists -> the kept keys of all its lists: each key's copies (the same
+// value at every other list its own stands for) enter the top-kl list. No copy can be missed: a copy ranks
+// below its original, so an original outside the top kl has no copy inside it. SORTED: copies are sorted and
+// merged in (team kernels: 3.2 us against 4.4 us a move); otherwise inserted one by one, which takes less
+// code (at 16 warps per SM, where instruction fetch counts, the sort costs 4 % of a generation).
+template <bool SORTED>
+__device__ __noinline__ uint64_t expand_copies(WarpShared const* ws, uint64_t list, int kl, int lane) {
+    uint64_t const key = list;
+    uint32_t const slot = 0xFFFFFFFFu - uint32_t(key), j = key ? slot / MP : 0u, i = slot % MP, k = j >> 1;
+    uint32_t c0 = 0, c1 = 0;                              // the parents whose list 0 / 1 is a copy
+    if (key) {
+        if (j & 1u) {
+            c1 = ws->grp1[k] & ~(1u << k);
+        } else {
+            c0 = ws->grp0[k];
+            c1 = c0 & ws->merged;
+            c0 &= ~(1u << k);
+        }
+    }
+    uint64_t thr = SORTED ? 0ull : shfl64(list, kl - 1);
+    while (__any_sync(FULL_MASK, (c0 | c1) != 0)) {       // one copy per key and turn
+        uint64_t copy = 0;
+        if (c0 | c1) {
+            uint32_t const m = c0 ? c0 : c1;
+            uint32_t const pos = (2u * uint32_t(__ffs(int(m)) - 1) + (c0 ? 0u : 1u)) * MP + i;
+            if (c0) c0 &= c0 - 1u;
+            else c1 &= c1 - 1u;
+            copy = (key & 0xFFFFFFFF00000000ull) | uint64_t(0xFFFFFFFFu - pos);
+        }
+        if (SORTED) list = merge_topk(list, warp_sort_desc(copy, lane), kl, lane);
+        else topk_fold(list, thr, copy, kl, lane);
+    }
+    return list;
 }
 
 // lane j builds kept node j (when active): parent record `prec`, placement (piece, i); with
@@ -917,6 +1019,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
     for (int stage = 0;; ++stage) {
         // ---- segments of this stage
         uint32_t total;
+        bool dedup = false;
         if (partner) {                         // the stage the leader posts, or the end of the game
             if (!team_sync(pr, rank, status, lane)) return mv;
             uint32_t const cmd = ws.team_cmd;
@@ -931,7 +1034,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
                 uint32_t const nd = lane ? r1 : r0;
                 uint32_t const held_slot = (nd >> 4) & 0xFu;
                 uint32_t const held_i = held_slot != HELD_NONE && slot_piece[held_slot] == 0u;
-                ws.seg_info[lane] = 32u | ((lane ? p1 : p0) << 16) | (held_i << 20) | (uint32_t(lane) << 21);
+                ws.seg_info[lane] = 32u | (uint32_t(lane) << 8) | ((lane ? p1 : p0) << 16) | (held_i << 20) | (1u << 22);
             }
             total = c_tables.nplace[p0] + c_tables.nplace[p1];
             if (lane == 0) {
@@ -942,7 +1045,11 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             }
             __syncwarp();
         } else {
-            total = build_segments(ws, slot_piece, tree, stage, fnode, kept, lane);
+            // teams of four share a pass's rounds, but not the serial grouping and copying (5 us a move
+            // against the 5 us that the copies' rounds take there: 18.3 against 17.9 ms for 30 champion
+            // games), so they evaluate every list
+            dedup = !KEYS && TEAM < 4 && (stage > 1 || p0 == p1);
+            total = build_segments(ws, slot_piece, tree, stage, fnode, kept, dedup, lane);
         }
         if (TEAMED && !partner) {                // post the stage
             if (lane == 0) {
@@ -994,9 +1101,10 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             fnode = g;
             materialize<WIDE>(&ws, lut, lane < kept, 32u, g ? p1 : p0, root_slot % MP, lane);
         } else if (!leaf) {
-            uint32_t const has_child = __reduce_or_sync(FULL_MASK, a.lo);
+            uint32_t const legal = list_legal(ws, __reduce_or_sync(FULL_MASK, a.lo), __reduce_or_sync(FULL_MASK, a.hi), lane);
+            if (dedup) a.list = expand_copies<TEAMED>(&ws, a.list, kl, lane);
             // kept nodes with no legal continuation become leaves at this depth (beam.hpp:549-551)
-            if (lane < kept && !((has_child >> lane) & 1u)) {
+            if (lane < kept && !legal) {
                 uint64_t const fk = (uint64_t(fscore) << 32) | uint64_t(ORDER_SPAN - (LEAF_ORDERS + frank));
                 if (KEYS) top2_insert(best, best2, fk);
                 else best = fk > best ? fk : best;
@@ -1017,8 +1125,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             kept = next;
         } else {
             // ---- leaf stage (beam.hpp:407-443): a list whose piece never fit scores the frontier board
-            uint32_t const legal_lo = __reduce_or_sync(FULL_MASK, a.lo);
-            uint32_t const legal_hi = __reduce_or_sync(FULL_MASK, a.hi);
+            uint32_t const legal = list_legal(ws, __reduce_or_sync(FULL_MASK, a.lo), __reduce_or_sync(FULL_MASK, a.hi), lane);
             if (KEYS) {
                 top2_insert(best, best2, a.best);
                 top2_insert(best, best2, a.best2);
@@ -1026,13 +1133,9 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
                 best = a.best > best ? a.best : best;
             }
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                int const j = lane + 32 * half;
-                int const k = j >> 1;
-                uint32_t const sc = __shfl_sync(FULL_MASK, fscore, k & 31);
-                bool const legal = ((half ? legal_hi : legal_lo) >> lane) & 1u;
-                if (k < kept && !legal) {
-                    uint64_t const key = (uint64_t(sc) << 32) | uint64_t(ORDER_SPAN - uint32_t(j) * MP);
+            for (int c = 0; c < 2; ++c) {
+                if (lane < kept && !((legal >> c) & 1u)) {
+                    uint64_t const key = (uint64_t(fscore) << 32) | uint64_t(ORDER_SPAN - uint32_t(2 * lane + c) * MP);
                     if (KEYS) top2_insert(best, best2, key);
                     else best = key > best ? key : best;
                 }
