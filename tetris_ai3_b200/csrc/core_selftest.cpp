@@ -30,14 +30,8 @@ int ta3bt_fast(uint32_t const* rec, uint32_t piece, uint32_t idx, int held, floa
     ta3b::load_fast_weights(HostW{w97}, fw);
     ta3b::RecView r;
     for (int o = 0; o < ta3b::NHID; ++o) __builtin_memcpy(&r.P[o], &rec[ta3b::R_P + o], 4);
-    r.tot = rec[ta3b::R_TOT];
-    r.hd = rec[ta3b::R_HD];
-    r.rc0 = rec[ta3b::R_RC];
-    r.rc1 = rec[ta3b::R_RC + 1];
-    r.rc2 = rec[ta3b::R_RC + 2];
     ta3b::PlaceFast const pf = ta3b::FAST.place[piece][idx];
-    ta3b::span_of(rec, int((pf.m >> 27) & 0xFu), r.h4, r.hm4);
-    r.combo = rec[ta3b::R_COMBO + ((pf.m >> 16) & 63u)];
+    ta3b::load_view(rec, pf, r);
     return ta3b::fast_eval<ta3b::MLP_SCALAR>(r, pf, held != 0, fw, *value, dbg);
 }
 
@@ -137,9 +131,7 @@ Cand candidate(uint32_t const* rec, int piece, int i, bool held, bool leaf, uint
     PlaceFast const pf = FAST.place[piece][i];
     RecView r;
     for (int o = 0; o < NHID; ++o) __builtin_memcpy(&r.P[o], &rec[R_P + o], 4);
-    r.tot = rec[R_TOT]; r.hd = rec[R_HD]; r.rc0 = rec[R_RC]; r.rc1 = rec[R_RC + 1]; r.rc2 = rec[R_RC + 2];
-    span_of(rec, int((pf.m >> 27) & 0xFu), r.h4, r.hm4);
-    r.combo = rec[R_COMBO + ((pf.m >> 16) & 63u)];
+    load_view(rec, pf, r);
     float v;
     bool const fast = fast_eval<MLP_SCALAR>(r, pf, held, fw, v) == FAST_OK;
     ++(fast ? g_fast_count : g_defer_count);
@@ -212,36 +204,16 @@ void ta3bt_topk_counts(unsigned long long* ins, unsigned long long* rounds, unsi
     *cands = g_cands;
 }
 
-// root record the way the warp builds it (each "lane" writes its own words)
+// the committed board's record: no path clears
 void ta3bt_root_record(uint32_t const* b10, float const* w97, uint32_t* rec) {
     uint32_t b[W];
     for (int x = 0; x < W; ++x) b[x] = b10[x];
-    HostW const w{w97};
-    for (int lane = 0; lane < 32; ++lane) {
-        ColumnData c;
-        column_data(b, c);
-        if (lane < W) rec[R_BOARD + lane] = b[lane];
-        if (lane == 22) {
-            uint32_t hb[4], hmb[4];
-            span_bytes(c, hb, hmb);
-            for (int q = 0; q < 4; ++q) {
-                rec[R_HB + q] = hb[q];
-                rec[R_HMB + q] = hmb[q];
-            }
-        }
-        for (int id = lane; id < NCOMBO; id += 32) {
-            int c0, wd;
-            combo_of(id, c0, wd);
-            rec[R_COMBO + id] = combo_word(c, c0, wd);
-        }
-        if (lane < NHID) rec[R_P + lane] = partial_word(0u, lane, w);
-        if (lane >= 16 && lane < 19) rec[R_RC + lane - 16] = row_counts(b, lane - 16);
-        if (lane == 20) rec[R_HD] = hole_depths_total(b);
-        if (lane == 21) {
-            rec[R_CLEARS] = 0;
-            rec[R_TOT] = c.holes | (c.maxh << 8) | (uint32_t(c.pw[W]) << 13) | (uint32_t(c.pp[W]) << 17);
-        }
-    }
+    build_record(b, 0u, HostW{w97}, rec);
+}
+
+// the surface input of every possible surface sum
+void ta3bt_surface_table(float* out) {
+    for (int s = 0; s <= SURF_MAX; ++s) out[s] = surface_input(s);
 }
 
 // a whole game through the kernel's algorithm; trace = 3 bytes per move

@@ -22,10 +22,11 @@
 //
 // Floating-point rules (both paths, host and device): every multiply and add
 // rounds separately (__fmul_rn / __fadd_rn on the device; the host build uses
-// -ffp-contract=off); sqrt is the correctly rounded sqrtf; divisions by the
-// feature constants 20, 200, 5 and 100 use the FMA-corrected reciprocal
-// quotient (Markstein), which tests/test_exact_division.py proves equal to
-// the IEEE quotient over every value the features can take.
+// -ffp-contract=off); v11's surface input sqrt(s) / 100 comes from a table of
+// correctly rounded values, the widened networks compute it (sqrtf correctly
+// rounded); divisions by the feature constants 20, 200, 5 and 100 use the FMA-corrected reciprocal quotient (Markstein), which
+// tests/test_exact_division.py proves equal to the IEEE quotient over every
+// value the features can take.
 #pragma once
 #include "tables.h"
 
@@ -103,6 +104,56 @@ TA3B_HD float div_exact(float x, float d, float r) {
 }
 constexpr float R20 = 0.05f, R200 = 0.005f, R5 = 0.2f, R100 = 0.01f;
 
+// The surface input sqrt(s) / 100 for every integer surface sum s, both operations rounded to
+// nearest: one load instead of a conversion, a square root and a quotient per candidate. The root
+// is exact integer arithmetic: m = floor(sqrt(s * 4^k)) with 24 bits, rounded up when the
+// remainder exceeds m (a tie is impossible: (m + 1/2)^2 is not an integer).
+constexpr int SURF_MAX = 4761;                                   // 9 * 23^2
+struct SurfaceTable {
+    float in[SURF_MAX + 1];
+};
+constexpr SurfaceTable make_surface_table() {
+    SurfaceTable t{};
+    uint64_t m = 1;
+    int k = 23;                                                  // s * 4^k in [2^46, 2^48)
+    for (int s = 1; s <= SURF_MAX; ++s) {
+        while ((uint64_t(s) << (2 * k)) >= (uint64_t(1) << 48)) {
+            --k;
+            m >>= 1;
+        }
+        uint64_t const n = uint64_t(s) << (2 * k);
+        uint64_t r = m < (uint64_t(1) << 23) ? (uint64_t(1) << 23) : m;
+        for (int i = 0; i < 64; ++i) {                           // Newton's iteration, from any start
+            uint64_t const q = (r + n / r) / 2;
+            if (q == r || q == r + 1 || q + 1 == r) {
+                r = q;
+                break;
+            }
+            r = q;
+        }
+        while (r * r > n) --r;
+        while ((r + 1) * (r + 1) <= n) ++r;
+        m = r;
+        uint64_t const root = n - r * r > r ? r + 1 : r;
+        t.in[s] = float(root) / float(uint64_t(1) << k) / 100.0f;
+    }
+    return t;
+}
+#if defined(__CUDACC__)
+__device__ SurfaceTable const g_surface = make_surface_table();
+#endif
+inline SurfaceTable const& host_surface() {
+    static SurfaceTable const t = make_surface_table();
+    return t;
+}
+TA3B_HD float surface_input(int s) {
+#if defined(__CUDA_ARCH__)
+    return __ldg(&g_surface.in[s]);
+#else
+    return host_surface().in[s];
+#endif
+}
+
 TA3B_HD uint32_t ordered_bits(float v) {                         // beam.hpp:204-207
     uint32_t u;
 #if defined(__CUDA_ARCH__)
@@ -131,69 +182,90 @@ struct BoardInts {
     int surf_sq;
 };
 
-TA3B_HD int col_hole_depth(uint32_t col) {
-    // occupied cells' count of empty cells below them: (H-1)n + n(n+1)/2 - (s + n^2),
-    // s = sum of occupied row indices, taken from the 5 bit planes of the index
-    int const n = b_popc(col);
-    int const s = b_popc(col & 0x2AAAAAu) + 2 * b_popc(col & 0x4CCCCCu) + 4 * b_popc(col & 0x70F0F0u) +
-                  8 * b_popc(col & 0x00FF00u) + 16 * b_popc(col & 0x7F0000u);
-    return (H - 1) * n + n * (n + 1) / 2 - (s + n * n);
+// The occupied cells' counts of empty cells below them, summed over the board: a column of n cells
+// at rows r_i has sum (22 - r_i) cells below them, less the n (n - 1) / 2 occupied ones:
+// n (45 - n) / 2 - sum r_i. The row indices are summed over all columns at once, from the number of
+// occupied cells per row as bit planes (planes[p] bit y = bit p of row y's count).
+TA3B_HD void row_planes(uint32_t const (&b)[W], uint32_t (&p)[4]) {
+    // ten one-bit numbers per row: full adders (three of a weight -> sum, carry), then half adders
+    auto sum3 = [](uint32_t x, uint32_t y, uint32_t z) { return x ^ y ^ z; };
+    auto maj3 = [](uint32_t x, uint32_t y, uint32_t z) { return (x & y) | (z & (x | y)); };
+    uint32_t const s1 = sum3(b[0], b[1], b[2]), c1 = maj3(b[0], b[1], b[2]);
+    uint32_t const s2 = sum3(b[3], b[4], b[5]), c2 = maj3(b[3], b[4], b[5]);
+    uint32_t const s3 = sum3(b[6], b[7], b[8]), c3 = maj3(b[6], b[7], b[8]);
+    uint32_t const s4 = sum3(s1, s2, s3), c4 = maj3(s1, s2, s3);
+    uint32_t const c5 = s4 & b[9];
+    uint32_t const t1 = sum3(c1, c2, c3), d1 = maj3(c1, c2, c3);
+    uint32_t const d2 = maj3(t1, c4, c5);
+    p[0] = s4 ^ b[9];
+    p[1] = sum3(t1, c4, c5);
+    p[2] = d1 ^ d2;
+    p[3] = d1 & d2;
 }
 
 TA3B_HD BoardInts board_ints(uint32_t const (&b)[W]) {
     BoardInts r{0, 0, 0, 0, 0};
     int h[W];
+    uint32_t pairs = 0;                                // sum of n (45 - n)
 #pragma unroll
     for (int x = 0; x < W; ++x) {
+        uint32_t const n = uint32_t(b_popc(b[x]));
         h[x] = H - column_top(b[x]);
-        r.holes += uint32_t(h[x] - b_popc(b[x]));
+        r.holes += uint32_t(h[x]) - n;
         r.max_height = uint32_t(h[x]) > r.max_height ? uint32_t(h[x]) : r.max_height;
-        r.hole_depths += uint32_t(col_hole_depth(b[x]));
+        pairs += n * (45u - n);
     }
+    uint32_t p[4];
+    row_planes(b, p);
+    uint32_t rows = 0;                                 // sum of the occupied cells' row indices
+#pragma unroll
+    for (int q = 3; q >= 0; --q)
+        rows = 2 * rows + uint32_t(b_popc(p[q] & 0x2AAAAAu) + 2 * b_popc(p[q] & 0x4CCCCCu) + 4 * b_popc(p[q] & 0x70F0F0u) +
+                                   8 * b_popc(p[q] & 0x00FF00u) + 16 * b_popc(p[q] & 0x7F0000u));
+    r.hole_depths = pairs / 2 - rows;
 #pragma unroll
     for (int x = 1; x < W; ++x) r.surf_sq += (h[x] - h[x - 1]) * (h[x] - h[x - 1]);
     uint32_t wells = uint32_t(h[1] >= h[0] + 3) + uint32_t(h[W - 2] >= h[W - 1] + 3);
 #pragma unroll
-    for (int x = 1; x < W - 1; ++x) wells += uint32_t(h[x - 1] >= h[x] + 3 && h[x + 1] >= h[x] + 3);
+    for (int x = 1; x < W - 1; ++x) wells += uint32_t((h[x - 1] < h[x + 1] ? h[x - 1] : h[x + 1]) >= h[x] + 3);
     r.wells = wells;
     return r;
 }
 
-// search.hpp:61-70: returns legality; nb = resulting board, cleared = rows removed
-TA3B_HD bool apply_full(uint32_t const (&b)[W], uint32_t cols, int col0, uint32_t (&nb)[W], int& cleared) {
+// search.hpp:61-70: returns legality; nb = resulting board, cleared = rows removed. src: the same
+// board as b in memory (the piece's columns are read from it by index)
+TA3B_HD bool apply_full(uint32_t const* src, uint32_t const (&b)[W], uint32_t cols, int col0, uint32_t (&nb)[W],
+                        int& cleared) {
     uint32_t hit = 0;
     int drop = H;
-    uint32_t nib[W];
 #pragma unroll
-    for (int x = 0; x < W; ++x) {
-        uint32_t const d = uint32_t(x - col0);
-        nib[x] = d < 4u ? (cols >> (4u * d)) & 0xFu : 0u;
-        hit |= b[x] & nib[x];
-        int const low = b_msb_nz(nib[x] | 1u);
-        int const dd = column_top(b[x] & ~((2u << low) - 1u)) - low - 1;
-        drop = (nib[x] != 0u && dd < drop) ? dd : drop;
+    for (int i = 0; i < 4; ++i) {
+        uint32_t const nib = (cols >> (4 * i)) & 0xFu;
+        uint32_t const col = src[col0 + i < W ? col0 + i : W - 1];
+        hit |= col & nib;
+        int const low = b_msb_nz(nib | 1u);
+        int const dd = column_top(col & ~((2u << low) - 1u)) - low - 1;
+        drop = (nib != 0u && dd < drop) ? dd : drop;
     }
     if (hit) return false;
+    uint64_t const piece = uint64_t(cols) << (4 * col0);       // nibble x = board column x
     uint32_t full = FIELD;
 #pragma unroll
     for (int x = 0; x < W; ++x) {
-        nb[x] = b[x] | (nib[x] << drop);
+        nb[x] = b[x] | ((uint32_t(piece >> (4 * x)) & 0xFu) << drop);
         full &= nb[x];
     }
     cleared = b_popc(full);
-    if (full) {
+    while (full) {                                             // the lowest set bit is the top row: rows above move down
+        uint32_t const above = (full & (~full + 1u)) - 1u;
+        full &= full - 1u;
 #pragma unroll
-        for (int x = 0; x < W; ++x) {
-            uint32_t col = nb[x], fl = full;
-            while (fl) {
-                uint32_t const row = fl & (~fl + 1u);
-                col = ((col & (row - 1u)) << 1) | (col & ~((row << 1) - 1u));
-                fl ^= row;
-            }
-            nb[x] = col;
-        }
+        for (int x = 0; x < W; ++x) nb[x] = ((nb[x] & above) << 1) | (nb[x] & ~(2u * above + 1u));
     }
     return true;
+}
+TA3B_HD bool apply_full(uint32_t const (&b)[W], uint32_t cols, int col0, uint32_t (&nb)[W], int& cleared) {
+    return apply_full(b, b, cols, col0, nb, cleared);
 }
 
 // model_v11.hpp:63-91 inputs + forward, every operation in the reference order
@@ -202,7 +274,7 @@ TA3B_HD float value_full(uint32_t clear_bits, BoardInts const& bi, bool held_i, 
     float in[NIN];
 #pragma unroll
     for (int k = 0; k < 4; ++k) in[k] = f_mul(float((clear_bits >> (8 * k)) & 0xFFu), 0.25f);
-    in[4] = div_exact(bi.surf_sq > 0 ? f_sqrt(float(bi.surf_sq)) : 0.0f, 100.0f, R100);
+    in[4] = surface_input(bi.surf_sq);
     in[5] = div_exact(float(bi.holes), 20.0f, R20);
     in[6] = div_exact(float(bi.hole_depths), 200.0f, R200);
     in[7] = float(bi.max_height);
@@ -252,7 +324,8 @@ static_assert(NPARAMS_WIDE == 4929 && NPARAMS_WIDE32 == 1441 && Wide64::STRIDE =
 
 TA3B_HD float relu(float v) { return v > 0.0f ? v : 0.0f; }    // std::max<float>(0, v)
 
-// model_v11.hpp:63-91 inputs of the widened network
+// model_v11.hpp:63-91 inputs of the widened network. The surface input is computed: L1, which
+// would hold its table, is full of the models' weights
 TA3B_HD void wide_inputs(uint32_t clear_bits, BoardInts const& bi, bool held_i, float (&in)[NIN]) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) in[k] = f_mul(float((clear_bits >> (8 * k)) & 0xFFu), 0.25f);
@@ -324,17 +397,17 @@ TA3B_HD float2 p2_add(float2 a, float2 b) {
 #endif
 }
 
-// two correctly rounded quotients x / d (div_exact per component)
+// two correctly rounded quotients x / d (div_exact per component; -q * d = q * -d)
 TA3B_HD float2 div2_exact(float2 x, float2 d, float2 r) {
     float2 const q = f2_mul(x, r);
-    float2 const e = f2_fma(make_float2(-q.x, -q.y), d, x);
+    float2 const e = f2_fma(q, make_float2(-d.x, -d.y), x);
     return f2_fma(e, r, q);
 }
-TA3B_HD int dot4_s8(uint32_t a, uint32_t b) {                   // sum of 4 signed byte products
+TA3B_HD int dot4_s8(uint32_t a, uint32_t b, int c) {            // c + sum of 4 signed byte products
 #if defined(__CUDA_ARCH__)
-    return __dp4a(int(a), int(b), 0);
+    return __dp4a(int(a), int(b), c);
 #else
-    int s = 0;
+    int s = c;
     for (int i = 0; i < 4; ++i) s += int(int8_t(a >> (8 * i))) * int(int8_t(b >> (8 * i)));
     return s;
 #endif
@@ -342,94 +415,23 @@ TA3B_HD int dot4_s8(uint32_t a, uint32_t b) {                   // sum of 4 sign
 
 // ------------------------------------------------------ parent record ---
 // One kept frontier node (or the committed board), in 68 u32 words (a 16-byte
-// multiple; 68 = 4 mod 32 staggers the records across shared-memory banks):
+// multiple; 68 = 4 mod 32 staggers the records across shared-memory banks, and
+// eight lanes' 16-byte stores cover all 32):
 constexpr int REC_WORDS = 68;
 constexpr int R_P = 0;        // float[8]: hidden partial sums after the 4 clear inputs
 constexpr int R_BOARD = 8;    // 10 bit-columns
 constexpr int R_CLEARS = 18;  // path clear histogram (4 x 8-bit lanes)
-constexpr int R_TOT = 19;     // holes (8) | max height (5) << 8 | wells (4) << 13 | surface sum (13) << 17
-constexpr int R_HD = 20;      // hole depths total
-constexpr int R_RC = 21;      // 3 words: occupied cells per row, 4 bits per row, rows 0..22
-constexpr int R_HB = 24;      // 4 words: column heights as bytes (byte x = column x, bytes 10..15 zero)
-constexpr int R_HMB = 28;     // 4 words: (holes - height) per column as signed bytes (bytes 10..15 zero)
-constexpr int R_COMBO = 32;   // 34 words, per (c0, width) combo: the old surface terms of the window's pairs (12)
-                              // | old wells of the window's columns (3) << 12 | left-well precondition << 15
-                              // | height of column c0-1 (5) << 16 | right-well precondition << 21
-                              // | height of column c0+w (5) << 22
-static_assert(R_COMBO + NCOMBO <= REC_WORDS && REC_WORDS % 4 == 0, "record layout");
+constexpr int R_TOT = 20;     // holes (8) | max height (5) << 8 | hole depths (12) << 16
+constexpr int R_RE = 21;      // 3 words: empty cells per row, 4 bits per row, rows 0..22; then rows 23.. as empty
+constexpr int R_SPAN = 26;    // 4 pairs of words: column heights as bytes (byte x = column x), then
+                              // (holes - height) per column as signed bytes; bytes 10..15 zero
+constexpr int R_COMBO = 34;   // 34 words, per (c0, width) combo: height of column c0-1, 31 at the wall (5)
+                              // | left-well precondition << 5 | height of column c0+w, 31 at the wall (5) << 8
+                              // | right-well precondition << 13 | wells outside the window's columns (3) << 16
+                              // | surface sum without the window's pairs (13) << 19
+static_assert(R_COMBO + NCOMBO <= REC_WORDS && REC_WORDS % 4 == 0 && R_SPAN % 2 == 0, "record layout");
 constexpr uint32_t WALL = 31; // height outside the board: satisfies every well-edge rule
-
-// Column data a record is derived from: heights with walls (h[x + 2] = column x),
-// holes per column, prefix sums of pair terms (pp[x+1] = sum over pairs (t-1, t),
-// t <= x) and of well flags (pw[x+1] = wells among columns <= x).
-struct ColumnData {
-    int h[W + 4];
-    int ho[W];
-    int pp[W + 1], pw[W + 1];
-    uint32_t holes, hd, maxh;
-};
-
-TA3B_HD void column_data(uint32_t const (&b)[W], ColumnData& c) {
-    c.holes = c.hd = c.maxh = 0;
-    c.h[0] = c.h[1] = c.h[W + 2] = c.h[W + 3] = int(WALL);
-#pragma unroll
-    for (int x = 0; x < W; ++x) {
-        int const hx = H - column_top(b[x]);
-        c.h[x + 2] = hx;
-        c.ho[x] = hx - b_popc(b[x]);
-        c.holes += uint32_t(c.ho[x]);
-        c.maxh = uint32_t(hx) > c.maxh ? uint32_t(hx) : c.maxh;
-    }
-    c.pp[0] = c.pp[1] = c.pw[0] = 0;
-#pragma unroll
-    for (int x = 0; x < W; ++x) {
-        int const l = c.h[x + 1], m = c.h[x + 2], r = c.h[x + 3];
-        c.pw[x + 1] = c.pw[x] + int((l < r ? l : r) >= m + 3);
-        if (x > 0) c.pp[x + 1] = c.pp[x] + (m - l) * (m - l);
-    }
-}
-
-TA3B_HD uint32_t hole_depths_total(uint32_t const (&b)[W]) {
-    uint32_t hd = 0;
-#pragma unroll
-    for (int x = 0; x < W; ++x) hd += uint32_t(col_hole_depth(b[x]));
-    return hd;
-}
-
-TA3B_HD uint32_t row_counts(uint32_t const (&b)[W], int q) {
-    // occupied cells per row, 4 bits per row, rows 8q..8q+7; summed bit-sliced
-    uint32_t s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-#pragma unroll
-    for (int x = 0; x < W; ++x) {
-        uint32_t const c0 = s0 & b[x];
-        s0 ^= b[x];
-        uint32_t const c1 = s1 & c0;
-        s1 ^= c0;
-        uint32_t const c2 = s2 & c1;
-        s2 ^= c1;
-        s3 ^= c2;
-    }
-    auto spread = [](uint32_t v) {              // 8 bits -> bit 4t of a word
-        v &= 0xFFu;
-        v = (v | (v << 12)) & 0x000F000Fu;
-        v = (v | (v << 6)) & 0x03030303u;
-        v = (v | (v << 3)) & 0x11111111u;
-        return v;
-    };
-    return spread(s0 >> (8 * q)) | (spread(s1 >> (8 * q)) << 1) | (spread(s2 >> (8 * q)) << 2) |
-           (spread(s3 >> (8 * q)) << 3);
-}
-
-// the byte arrays R_HB / R_HMB of a record
-TA3B_HD void span_bytes(ColumnData const& c, uint32_t (&hb)[4], uint32_t (&hmb)[4]) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) hb[q] = hmb[q] = 0;
-#pragma unroll
-    for (int x = 0; x < W; ++x) {
-        hb[x >> 2] |= uint32_t(c.h[x + 2]) << (8 * (x & 3));
-        hmb[x >> 2] |= (uint32_t(c.ho[x] - c.h[x + 2]) & 0xFFu) << (8 * (x & 3));
-    }
-}
+constexpr uint32_t ROWS_EMPTY = 0xAAAAAAAAu;
 
 TA3B_HD uint32_t fshr32(uint32_t lo, uint32_t hi, uint32_t sh) {     // low word of (hi:lo) >> sh, sh < 32
 #if defined(__CUDA_ARCH__)
@@ -438,33 +440,21 @@ TA3B_HD uint32_t fshr32(uint32_t lo, uint32_t hi, uint32_t sh) {     // low word
     return sh ? (lo >> sh) | (hi << (32u - sh)) : lo;
 #endif
 }
-
-// window words for origin c0: bytes i = column c0+i (0 past the edge) of the two byte arrays
-TA3B_HD void span_of(uint32_t const* rec, int c0, uint32_t& h4, uint32_t& hm4) {
-    uint32_t const wi = uint32_t(c0) >> 2, sh = (uint32_t(c0) & 3u) * 8u;
-    h4 = fshr32(rec[R_HB + wi], rec[R_HB + wi + 1], sh);
-    hm4 = fshr32(rec[R_HMB + wi], rec[R_HMB + wi + 1], sh);
+TA3B_HD uint32_t dot4_u8(uint32_t a, uint32_t b, uint32_t c) {       // c + sum of 4 unsigned byte products
+#if defined(__CUDA_ARCH__)
+    return __dp4a(a, b, c);
+#else
+    for (int i = 0; i < 4; ++i) c += ((a >> (8 * i)) & 0xFFu) * ((b >> (8 * i)) & 0xFFu);
+    return c;
+#endif
 }
 
-TA3B_HD uint32_t combo_word(ColumnData const& c, int c0, int wd) {
-    int const last = c0 + wd < W - 1 ? c0 + wd : W - 1;                // window columns [c0-1, c0+w] in the board
-    int const pairs = c.pp[last + 1] - c.pp[c0 > 1 ? c0 : 1];
-    int const wells = c.pw[last + 1] - c.pw[c0 > 0 ? c0 - 1 : 0];
-    uint32_t v = uint32_t(pairs) | (uint32_t(wells) << 12);
-    if (c0 > 0) {
-        int const hl = c.h[c0 + 1];                                     // column c0-1
-        v |= (uint32_t(c.h[c0] >= hl + 3) << 15) | (uint32_t(hl) << 16);
-    }
-    if (c0 + wd < W) {
-        int const hr = c.h[c0 + wd + 2];                                // column c0+w
-        v |= (uint32_t(c.h[c0 + wd + 3] >= hr + 3) << 21) | (uint32_t(hr) << 22);
-    }
-    return v;
-}
-
-TA3B_HD void combo_of(int id, int& c0, int& wd) {
-    wd = id < 10 ? 1 : id < 19 ? 2 : id < 27 ? 3 : 4;
-    c0 = id - (wd == 1 ? 0 : wd == 2 ? 10 : wd == 3 ? 19 : 27);
+TA3B_HD void store4(uint32_t* dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {   // dst 16-byte aligned
+#if defined(__CUDA_ARCH__)
+    *reinterpret_cast<uint4*>(dst) = make_uint4(a, b, c, d);
+#else
+    dst[0] = a; dst[1] = b; dst[2] = c; dst[3] = d;
+#endif
 }
 
 template <class WF>
@@ -485,45 +475,98 @@ TA3B_HD uint32_t partial_word(uint32_t clear_bits, int o, WF const& w) {
 // PARTIALS: the v11 hidden partial sums (the widened network recomputes its own per candidate)
 template <class WF, bool PARTIALS = true>
 TA3B_HD void build_record(uint32_t const (&b)[W], uint32_t clear_bits, WF const& w, uint32_t* rec) {
-    ColumnData c;
-    column_data(b, c);
-#pragma unroll
-    for (int x = 0; x < W; ++x) rec[R_BOARD + x] = b[x];
-    rec[R_CLEARS] = clear_bits;
-    rec[R_TOT] = c.holes | (c.maxh << 8) | (uint32_t(c.pw[W]) << 13) | (uint32_t(c.pp[W]) << 17);
-    rec[R_HD] = hole_depths_total(b);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) rec[R_RC + q] = row_counts(b, q);
-    // fully unrolled: every column index is a constant, so the column data stays in registers
-    uint32_t hb[4], hmb[4];
-    span_bytes(c, hb, hmb);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        rec[R_HB + q] = hb[q];
-        rec[R_HMB + q] = hmb[q];
-    }
-#pragma unroll
-    for (int id = 0; id < NCOMBO; ++id) {
-        int c0, wd;
-        combo_of(id, c0, wd);
-        rec[R_COMBO + id] = combo_word(c, c0, wd);
-    }
     if (PARTIALS) {
+        uint32_t p[NHID];
 #pragma unroll
-        for (int o = 0; o < NHID; ++o) rec[R_P + o] = partial_word(clear_bits, o, w);
+        for (int o = 0; o < NHID; ++o) p[o] = partial_word(clear_bits, o, w);
+        store4(rec + R_P, p[0], p[1], p[2], p[3]);
+        store4(rec + R_P + 4, p[4], p[5], p[6], p[7]);
+    }
+    store4(rec + R_BOARD, b[0], b[1], b[2], b[3]);
+    store4(rec + R_BOARD + 4, b[4], b[5], b[6], b[7]);
+    store4(rec + R_BOARD + 8, b[8], b[9], clear_bits, 0u);
+    // per column: height, holes; h[x + 2] with walls
+    int h[W + 4];
+    h[0] = h[1] = h[W + 2] = h[W + 3] = int(WALL);
+    uint32_t holes = 0, maxh = 0, pairs = 0, hb[3] = {0, 0, 0}, hmb[3] = {0, 0, 0};
+#pragma unroll
+    for (int x = 0; x < W; ++x) {
+        uint32_t const n = uint32_t(b_popc(b[x]));
+        uint32_t const hx = uint32_t(H - column_top(b[x]));
+        h[x + 2] = int(hx);
+        holes += hx - n;
+        maxh = hx > maxh ? hx : maxh;
+        pairs += n * (45u - n);
+        hb[x >> 2] |= hx << (8 * (x & 3));
+        hmb[x >> 2] |= ((0u - n) & 0xFFu) << (8 * (x & 3));          // holes - height = -cells
+    }
+    // cells per row as nibbles; the row indices of all cells (board_ints)
+    uint32_t pl[4], cnt[3], rows = 0;
+    row_planes(b, pl);
+    auto spread = [](uint32_t v) {              // 8 bits -> bit 4t of a word
+        v = (v | (v << 12)) & 0x000F000Fu;
+        v = (v | (v << 6)) & 0x03030303u;
+        v = (v | (v << 3)) & 0x11111111u;
+        return v;
+    };
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        cnt[q] = 0;
+#pragma unroll
+        for (int t = 3; t >= 0; --t) cnt[q] = 2 * cnt[q] + spread((pl[t] >> (8 * q)) & 0xFFu);
+        rows = dot4_u8(cnt[q] & 0x0F0F0F0Fu, 0x06040200u + 0x08080808u * uint32_t(q), rows);
+        rows = dot4_u8((cnt[q] >> 4) & 0x0F0F0F0Fu, 0x07050301u + 0x08080808u * uint32_t(q), rows);
+    }
+    store4(rec + R_TOT, holes | (maxh << 8) | ((pairs / 2 - rows) << 16), ROWS_EMPTY - cnt[0], ROWS_EMPTY - cnt[1],
+           ROWS_EMPTY - cnt[2]);
+    store4(rec + R_TOT + 4, ROWS_EMPTY, 0u, hb[0], hmb[0]);
+    store4(rec + R_TOT + 8, hb[1], hmb[1], hb[2], hmb[2]);
+    // a combo word is the sum of a word of its window's left edge (c0) and one of its right edge
+    // (e = c0 + w): prefix sums up to the edges (pairs (x-1, x) and well flags) on the left, the
+    // totals less the prefix sums on the right
+    uint32_t pp[W + 1], left[W], right[W + 1];           // prefix: wells << 16 | surface sum << 19
+    pp[0] = 0;
+#pragma unroll
+    for (int x = 0; x < W; ++x) {
+        int const l = h[x + 1], m = h[x + 2], r = h[x + 3];
+        uint32_t const step = x > 0 ? uint32_t((m - l) * (m - l)) << 19 : 0u;
+        pp[x + 1] = pp[x] + step + (uint32_t((l < r ? l : r) >= m + 3) << 16);
+    }
+    constexpr uint32_t WELLS = 7u << 16, SURF = ~0u << 19;
+#pragma unroll
+    for (int c = 0; c < W; ++c)                          // wells among columns < c0 - 1, pairs before (c0 - 1, c0)
+        left[c] = uint32_t(h[c + 1]) | (uint32_t(c > 0 && h[c] >= h[c + 1] + 3) << 5) |
+                  (pp[c > 0 ? c - 1 : 0] & WELLS) | (pp[c > 1 ? c : 1] & SURF);
+#pragma unroll
+    for (int e = 1; e <= W; ++e)
+        right[e] = (uint32_t(h[e + 2]) << 8) | (uint32_t(e < W && h[e + 3] >= h[e + 2] + 3) << 13) |
+                   (pp[W] - pp[e + 1 < W ? e + 1 : W]);
+    store4(rec + R_TOT + 12, 0u, 0u, left[0] + right[1], left[1] + right[2]);
+    static_assert(R_COMBO + 2 == R_TOT + 16 && (NCOMBO - 2) % 4 == 0, "the first two combos share a vector");
+#pragma unroll
+    for (int id = 2; id < NCOMBO; id += 4) {
+        uint32_t v[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            int const wd = id + t < 10 ? 1 : id + t < 19 ? 2 : id + t < 27 ? 3 : 4;
+            int const c0 = id + t - (wd == 1 ? 0 : wd == 2 ? 10 : wd == 3 ? 19 : 27);
+            v[t] = left[c0] + right[c0 + wd];
+        }
+        store4(rec + R_COMBO + id, v[0], v[1], v[2], v[3]);
     }
 }
 
 // ------------------------------------------------------------ fast path ---
 // The weights the fast path needs, as pairs of hidden units (2q, 2q+1):
-// W1[o][4..9], W2[o], plus b2.
+// W1[o][4..9], W2[o], plus b2; nz = -0 (see MLP_X2FMA), a value the compiler must not know.
 struct FastW {
     float2 w4[NHID / 2], w5[NHID / 2], w6[NHID / 2], w7[NHID / 2], w8[NHID / 2], w9[NHID / 2], u[NHID / 2];
-    float b2;
+    float b2, nz;
 };
 
 template <class WF>
-TA3B_HD void load_fast_weights(WF const& w, FastW& f) {
+TA3B_HD void load_fast_weights(WF const& w, FastW& f, float nz = -0.0f) {
+    f.nz = nz;
 #pragma unroll
     for (int q = 0; q < NHID / 2; ++q) {
         int const a = 2 * q, b = 2 * q + 1;
@@ -542,10 +585,26 @@ enum FastStatus { FAST_OK = 0, FAST_DEFER = 1 };
 
 // The parent record words a fast candidate reads.
 struct RecView {
+    uint32_t const* rec;
     float P[NHID];
-    uint32_t tot, hd, rc0, rc1, rc2;
-    uint32_t h4, hm4, combo;
+    uint32_t tot, h4, hm4, combo;
 };
+
+// the parent's words for one placement (P is the caller's: the widened network has none)
+TA3B_HD void load_view(uint32_t const* rec, PlaceFast pf, RecView& r) {
+    r.rec = rec;
+    r.tot = rec[R_TOT];
+    uint32_t const* const s = rec + R_SPAN + (pf.span & 0xFFu);
+#if defined(__CUDA_ARCH__)
+    uint2 const lo = *reinterpret_cast<uint2 const*>(s), hi = *reinterpret_cast<uint2 const*>(s + 2);
+#else
+    struct { uint32_t x, y; } const lo{s[0], s[1]}, hi{s[2], s[3]};
+#endif
+    uint32_t const sh = pf.span >> 8;
+    r.h4 = fshr32(lo.x, hi.x, sh);
+    r.hm4 = fshr32(lo.y, hi.y, sh);
+    r.combo = rec[R_COMBO + pf.combo];
+}
 
 // The placement's effect on the parent, from the record alone (branch-free).
 // Returns FAST_DEFER when a piece cell may meet the stack inside the spawn rows
@@ -553,59 +612,67 @@ struct RecView {
 // MLP arithmetic: MLP_SCALAR = __fmul_rn / __fadd_rn per hidden unit;
 // MLP_PTX_X2 = pairs of hidden units per packed PTX instruction (mul/add.rn.f32x2);
 // MLP_X2 = the same pairs through the __fmul2_rn / __fadd2_rn intrinsics;
-// MLP_X2MUL = packed multiplies (__fmul2_rn), scalar adds. Each packed instruction rounds both
-// halves exactly like the scalar .rn operation, but a packed multiply feeding a packed add is
-// compiled into a fused multiply-add (one rounding): on the B200 the PTX pair equals fma.rn on
-// all of 1,048,576 probe samples. Only MLP_X2MUL keeps the reference's two roundings.
-enum MlpMode { MLP_SCALAR = 0, MLP_PTX_X2 = 1, MLP_X2 = 2, MLP_X2MUL = 3 };
+// MLP_X2MUL = packed multiplies (__fmul2_rn), scalar adds;
+// MLP_X2FMA = packed multiplies as fused multiply-adds of -0, packed adds.
+// Each packed instruction rounds both halves exactly like the scalar .rn operation, but a packed
+// multiply feeding a packed add is compiled into a fused multiply-add (one rounding): on the B200 the
+// PTX pair equals fma.rn on all of 1,048,576 probe samples. x * w + (-0) is x * w with one rounding,
+// signed zeros included, and cannot be fused with the add that follows as long as the compiler does not
+// know the -0 (a kernel parameter): MLP_X2FMA keeps the reference's two roundings with 24 packed adds in
+// place of 48 scalar ones (0 of 16,777,216 probe samples differ). A packed instruction takes two cycles
+// of the FP32 pipe, so it saves issue slots, not arithmetic.
+enum MlpMode { MLP_SCALAR = 0, MLP_PTX_X2 = 1, MLP_X2 = 2, MLP_X2MUL = 3, MLP_X2FMA = 4 };
 
 // The fast path's features of one placement (holes, hole depths, surface,
 // wells, max height) from the parent record alone; true when the candidate
-// must take the full path instead.
+// must take the full path instead. Bound by issue slots (16 warps per SM, 65 % busy): the record and
+// the placement data hold what it needs in the place where one instruction takes it (bytes, whole words,
+// top fields, sums formed when the record is built), and the columns are handled four at a time as bytes.
 struct FastFeat {
     int holes, hd, surf, wells, maxh, dr;
 };
 
+TA3B_HD int min3_s32(int a, int b, int c) {
+#if defined(__CUDA_ARCH__)
+    return __vimin3_s32(a, b, c);
+#else
+    int const m = a < b ? a : b;
+    return m < c ? m : c;
+#endif
+}
+
 TA3B_HD bool fast_features(RecView const& r, PlaceFast pf, FastFeat& f) {
-    int const width = int((pf.s >> 22) & 7u);
-    // drop = min over the piece's columns of (top - lowest piece cell - 1), top = H - height
-    int drop = 255, sumd = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int const d = int((pf.d4 >> (8 * i)) & 0xFFu) - int((r.h4 >> (8 * i)) & 0xFFu);
-        drop = d < drop ? d : drop;
-        sumd += i < width ? d : 0;
-    }
-    bool defer = drop < 0;
-    int const dr = defer ? 0 : drop;
-    // rows dr..dr+3: occupied cells + the piece's cells per row; a nibble of 10 = a full row
-    int const bit = 4 * dr;
-    uint32_t const wlo = bit < 32 ? r.rc0 : (bit < 64 ? r.rc1 : r.rc2);
-    uint32_t const whi = bit < 32 ? r.rc1 : (bit < 64 ? r.rc2 : 0u);
-    uint32_t const sh = uint32_t(bit & 31);
-    uint32_t const win = (sh ? ((wlo >> sh) | (whi << (32u - sh))) : wlo) & 0xFFFFu;
-    uint32_t const sum = (win + (pf.m & 0xFFFFu)) ^ 0xAAAAu;
-    defer = defer || (((sum - 0x1111u) & ~sum & 0x8888u) != 0u);
+    // byte i = 128 + how far piece column i can fall: 22 - lowest row - height (far above for i >= width)
+    uint32_t const d = pf.d4 - r.h4;
+    int const reach = min3_s32(int(d & 0xFFu), int((d >> 8) & 0xFFu),
+                               min3_s32(int((d >> 16) & 0xFFu), int(d >> 24), 255)) - 128;
+    bool defer = reach < 0;
+    int const dr = reach < 0 ? 0 : reach;
+    // rows dr..dr+3: a row whose empty cells are all the piece's is full (rows past the floor: 10 empty cells)
+    uint32_t const* const re = r.rec + R_RE + (dr >> 3);
+    uint32_t const left = fshr32(re[0], re[1], uint32_t(4 * dr) & 31u) - pf.rows;
+    defer = defer || (((left - 0x1111u) & ~left & 0x8888u) != 0u);
+    int const w = int(pf.tops >> 24);
     // holes gain the gaps under the piece; every new cell sits over (holes + gap) empty cells
-    int const holes = int(r.tot & 0xFFu) + sumd - width * dr;
-    int const hd = int(r.hd) + dot4_s8(pf.c4, r.hm4) + int((pf.s >> 7) & 0x7Fu) - 4 * dr;
-    int const top_max = H - dr - int((pf.m >> 25) & 3u);
-    int const maxh = int((r.tot >> 8) & 0x1Fu) > top_max ? int((r.tot >> 8) & 0x1Fu) : top_max;
-    int const n0 = H - dr - int((pf.s >> 18) & 3u);              // new height of the first / last piece column
-    int const nl = H - dr - int((pf.s >> 20) & 3u);
+    int const holes = dot4_s8(r.h4, pf.neg, int(r.tot & 0xFFu) + int(pf.adds & 0xFFu)) - w * dr;
+    int const hd = dot4_s8(pf.c4, r.hm4, int(r.tot >> 16) + int((pf.adds >> 8) & 0xFFu)) - 4 * dr;
+    // new heights of the first and last piece columns and of the piece's top
+    uint32_t const tops = pf.tops - uint32_t(dr) * 0x010101u;
+    int const n0 = int(tops & 0xFFu), nl = int((tops >> 8) & 0xFFu), top = int((tops >> 16) & 0xFFu);
+    int const maxh0 = int((r.tot >> 8) & 0xFFu);
+    int const maxh = maxh0 > top ? maxh0 : top;
     uint32_t const cb = r.combo;
-    int const hl = int((cb >> 16) & 31u), hr = int((cb >> 22) & 31u);
-    bool const lv = (pf.m >> 23) & 1u, rv = (pf.m >> 24) & 1u;
+    int const hl = int(cb & 31u), hr = int((cb >> 8) & 31u);
+    int const tl = n0 - hl, tr = nl - hr;
     // surface: the window's pairs are replaced by the piece's inner steps and the two edge pairs
-    int surf = int(r.tot >> 17) - int(cb & 0xFFFu) + int((pf.s >> 14) & 0xFu);
-    surf += lv ? (n0 - hl) * (n0 - hl) : 0;
-    surf += rv ? (hr - nl) * (hr - nl) : 0;
+    int surf = int(cb >> 19) + int((pf.adds >> 16) & 0xFFu);
+    surf += hl != int(WALL) ? tl * tl : 0;
+    surf += hr != int(WALL) ? tr * tr : 0;
     // wells: only the two neighbour columns (and a one-column piece itself) can be wells now
-    int wells = int((r.tot >> 13) & 0xFu) - int((cb >> 12) & 7u);
-    wells += int(lv && ((cb >> 15) & 1u) && n0 >= hl + 3);
-    wells += int(rv && ((cb >> 21) & 1u) && nl >= hr + 3);
-    int const hlw = lv ? hl : int(WALL), hrw = rv ? hr : int(WALL);
-    wells += int(((pf.m >> 22) & 1u) && (hlw < hrw ? hlw : hrw) >= n0 + 3);
+    int wells = int((cb >> 16) & 7u);
+    wells += int((cb & (1u << 5)) && tl >= 3);
+    wells += int((cb & (1u << 13)) && tr >= 3);
+    wells += int((pf.adds >> 24) && (tl > tr ? tl : tr) <= -3);
     f = FastFeat{holes, hd, surf, wells, maxh, dr};
     return defer;
 }
@@ -617,13 +684,13 @@ TA3B_HD int fast_eval(RecView const& r, PlaceFast pf, bool held_i, FastW const& 
     bool const defer = fast_features(r, pf, ff);
     int const holes = ff.holes, hd = ff.hd, surf = ff.surf, wells = ff.wells, maxh = ff.maxh, dr = ff.dr;
     // features (model_v11.hpp:63-91): pairs of correctly rounded quotients
-    float const sq = surf > 0 ? f_sqrt(float(surf)) : 0.0f;
+    float const s4 = surface_input(defer ? 0 : surf);            // a deferred candidate's sum may be out of range
     float2 const q56 = div2_exact(make_float2(float(holes), float(hd)), make_float2(20.0f, 200.0f),
                                   make_float2(R20, R200));
-    float2 const q94 = div2_exact(make_float2(float(wells), sq), make_float2(5.0f, 100.0f), make_float2(R5, R100));
-    float2 const x4 = make_float2(q94.y, q94.y), x5 = make_float2(q56.x, q56.x), x6 = make_float2(q56.y, q56.y);
+    float const q9 = div_exact(float(wells), 5.0f, R5);
+    float2 const x4 = make_float2(s4, s4), x5 = make_float2(q56.x, q56.x), x6 = make_float2(q56.y, q56.y);
     float const m7 = float(maxh), m8 = held_i ? 1.0f : 0.0f;
-    float2 const x7 = make_float2(m7, m7), x8 = make_float2(m8, m8), x9 = make_float2(q94.x, q94.x);
+    float2 const x7 = make_float2(m7, m7), x8 = make_float2(m8, m8), x9 = make_float2(q9, q9);
     if (dbg) {                                   // diagnostics for the self-tests
         dbg[0] = float(holes); dbg[1] = float(hd); dbg[2] = float(surf); dbg[3] = float(wells);
         dbg[4] = float(maxh); dbg[5] = x4.x; dbg[6] = x5.x; dbg[7] = x6.x; dbg[8] = x9.x; dbg[9] = float(dr);
@@ -648,6 +715,14 @@ TA3B_HD int fast_eval(RecView const& r, PlaceFast pf, bool held_i, FastW const& 
             a.y = f_add(a.y, m8.y);
             a.x = f_add(a.x, m9.x);
             a.y = f_add(a.y, m9.y);
+        } else if (MLP == MLP_X2FMA) {
+            float2 const nz = make_float2(fw.nz, fw.nz);
+            a = f2_add(a, f2_fma(x4, fw.w4[q], nz));
+            a = f2_add(a, f2_fma(x5, fw.w5[q], nz));
+            a = f2_add(a, f2_fma(x6, fw.w6[q], nz));
+            a = f2_add(a, f2_fma(x7, fw.w7[q], nz));
+            a = f2_add(a, f2_fma(x8, fw.w8[q], nz));
+            a = f2_add(a, f2_fma(x9, fw.w9[q], nz));
         } else if (MLP == MLP_X2) {
             a = f2_add(a, f2_mul(x4, fw.w4[q]));
             a = f2_add(a, f2_mul(x5, fw.w5[q]));
@@ -683,7 +758,7 @@ TA3B_HD int fast_eval(RecView const& r, PlaceFast pf, bool held_i, FastW const& 
         a.x = a.x > 0.0f ? a.x : 0.0f;                      // std::max<float>(0, v)
         a.y = a.y > 0.0f ? a.y : 0.0f;
         float2 const t = MLP == MLP_PTX_X2                  ? p2_mul(a, fw.u[q])
-                         : (MLP == MLP_X2 || MLP == MLP_X2MUL) ? f2_mul(a, fw.u[q])
+                         : (MLP == MLP_X2 || MLP == MLP_X2MUL || MLP == MLP_X2FMA) ? f2_mul(a, fw.u[q])
                                                                : make_float2(f_mul(a.x, fw.u[q].x),
                                                                              f_mul(a.y, fw.u[q].y));
         v = f_add(v, t.x);

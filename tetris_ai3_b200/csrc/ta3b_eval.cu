@@ -25,6 +25,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -78,20 +79,27 @@ constexpr DevTables make_dev_tables() {
 
 __constant__ DevTables c_tables = make_dev_tables();
 
-// Placement tables copied into shared memory per block: the incremental-path
-// data (PlaceFast) and the move itself packed as cols (16) | col0 (4) << 16 |
+// Placement tables copied into shared memory per block, indexed piece * MP + placement: the
+// incremental-path data (PlaceFast, its two vectors apart so that consecutive lanes' 16-byte
+// loads meet no bank twice) and the move itself packed as cols (16) | col0 (4) << 16 |
 // orientation (2) << 20 | (x + 2) (4) << 24.
+constexpr int NFLAT = NPIECE * MP;
+struct alignas(16) Word4 {
+    uint32_t x, y, z, w;
+};
 struct LutTables {
-    PlaceFast fast[NPIECE][MP];
-    uint32_t move[NPIECE][MP];
+    Word4 fast[2][NFLAT];
+    uint32_t move[NFLAT];
 };
 constexpr LutTables make_lut_tables() {
     LutTables t{};
     for (int p = 0; p < NPIECE; ++p)
         for (int i = 0; i < TABLES.nplace[p]; ++i) {
             Place const pl = TABLES.place[p][i];
-            t.fast[p][i] = FAST.place[p][i];
-            t.move[p][i] = uint32_t(pl.cols) | (uint32_t(pl.col0) << 16) | (uint32_t(pl.orient) << 20) |
+            PlaceFast const f = FAST.place[p][i];
+            t.fast[0][p * MP + i] = Word4{f.d4, f.c4, f.neg, f.rows};
+            t.fast[1][p * MP + i] = Word4{f.tops, f.adds, f.combo, f.span};
+            t.move[p * MP + i] = uint32_t(pl.cols) | (uint32_t(pl.col0) << 16) | (uint32_t(pl.orient) << 20) |
                            (uint32_t(pl.x + 2) << 24);
         }
     return t;
@@ -204,7 +212,7 @@ __device__ __noinline__ Applied apply_ints(uint32_t const* src, uint32_t cols, i
     uint32_t b[W], nb[W];
     load_board(src, b);
     Applied r{};
-    r.legal = apply_full(b, cols, col0, nb, r.cleared);
+    r.legal = apply_full(src, b, cols, col0, nb, r.cleared);
     if (!r.legal) return r;
     r.bi = board_ints(nb);
     if (dst)
@@ -247,7 +255,7 @@ __device__ __forceinline__ void load_board(uint32_t const* __restrict__ src, uin
 }
 
 #ifndef TA3B_MLP_MODE
-#define TA3B_MLP_MODE MLP_X2MUL     // packed multiplies, scalar adds: the reference's roundings, fewer instructions
+#define TA3B_MLP_MODE MLP_X2FMA     // packed multiplies and adds with the reference's roundings
 #endif
 
 // fast path: read the parent-record words this placement needs, then eval_core's fast_eval
@@ -259,11 +267,7 @@ __device__ __forceinline__ int fast_candidate(uint32_t const* __restrict__ rec, 
     float4 const p1 = *reinterpret_cast<float4 const*>(rec + R_P + 4);
     r.P[0] = p0.x; r.P[1] = p0.y; r.P[2] = p0.z; r.P[3] = p0.w;
     r.P[4] = p1.x; r.P[5] = p1.y; r.P[6] = p1.z; r.P[7] = p1.w;
-    uint4 const q = *reinterpret_cast<uint4 const*>(rec + R_HD);       // hd, rc0, rc1, rc2
-    r.hd = q.x; r.rc0 = q.y; r.rc1 = q.z; r.rc2 = q.w;
-    r.tot = rec[R_TOT];
-    span_of(rec, int((pf.m >> 27) & 0xFu), r.h4, r.hm4);
-    r.combo = rec[R_COMBO + ((pf.m >> 16) & 63u)];
+    load_view(rec, pf, r);
     return fast_eval<MLP>(r, pf, held_i, fw, v, dbg);
 }
 
@@ -381,11 +385,7 @@ template <int H>
 __device__ __forceinline__ int fast_candidate_wide(uint32_t const* __restrict__ rec, PlaceFast pf, bool held_i,
                                                    float const* __restrict__ w, float* hb, int lane, float& v) {
     RecView r;
-    uint4 const q = *reinterpret_cast<uint4 const*>(rec + R_HD);
-    r.hd = q.x; r.rc0 = q.y; r.rc1 = q.z; r.rc2 = q.w;
-    r.tot = rec[R_TOT];
-    span_of(rec, int((pf.m >> 27) & 0xFu), r.h4, r.hm4);
-    r.combo = rec[R_COMBO + ((pf.m >> 16) & 63u)];
+    load_view(rec, pf, r);
     WideIn in;
     bool const defer = fast_wide_inputs(r, rec[R_CLEARS], pf, held_i, in.v);
     v = wide_value<H>(in, w, hb, lane);
@@ -455,6 +455,29 @@ __device__ __forceinline__ uint64_t merge_topk(uint64_t a, uint64_t b, int kl, i
     return lane < kl ? c : 0ull;
 }
 
+// One unsorted key per lane into the warp's sorted list: a bitonic sort (k = 2 .. 32), then the two
+// descending lists merged (k = 64) into the top kl keys. A loop, not straight-line code: instruction
+// fetch bounds the kernels as much as issue.
+__device__ __noinline__ uint64_t merge_keys(uint64_t list, uint64_t v, int kl, int lane) {
+#pragma unroll 1
+    for (int k = 2; k <= 2 * WARP; k <<= 1) {
+        int j = k >> 1;
+        if (j == WARP) {
+            uint64_t const r = shfl64(v, 31 - lane);             // ascending: the larger of each pair is bitonic
+            v = list > r ? list : r;                              // and holds the 32 largest of both
+            j = WARP / 2;
+        }
+        bool const down = (lane & k) == 0;
+#pragma unroll 1
+        for (; j > 0; j >>= 1) {
+            uint64_t const o = shfl64_xor(v, j);
+            bool const keep_max = ((lane & j) == 0) == down;
+            v = (v > o) == keep_max ? v : o;
+        }
+    }
+    return lane < kl ? v : 0ull;
+}
+
 // Fold one key per lane into the warp's sorted top-K list (lane i = i-th largest, 0 = empty;
 // `thr` caches list[k-1]): the keys above thr are inserted one at a time by ballot/shuffle. The
 // threshold is refreshed once per round, not after every insertion: a key that an earlier
@@ -498,9 +521,8 @@ constexpr uint32_t TEAM_GAME_END = 0xFFFFFFFFu;
 constexpr unsigned long long kTeamWaitNs = 1000000000ull;    // 1 s
 constexpr uint32_t STATUS_TEAM = 4u;
 // a partner's stage results, in its own (otherwise unused) record area: its list (or per-lane
-// argmax) in words 0-63, its legality bits in words X_LO / X_HI; its game's evaluation count in
-// X_EVALS
-constexpr int X_LO = 64, X_HI = 65, X_EVALS = 66;
+// argmax) in words 0-63; its game's evaluation count (illegal candidates taken back) in X_EVALS
+constexpr int X_EVALS = 66;
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -511,18 +533,21 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // ---------------------------------------------------------------- kernel ---
 struct alignas(16) WarpShared {
     uint32_t rec[33][REC_WORDS];      // kept frontier records (rank -> record); [32] = committed board
-    float wfull[NPARAMS + 3];         // the v11 model's weights (full path, record partial sums)
-    float const* wglobal;              // the widened model's weights (global memory)
+    float const* wglobal;              // the model's weights (global memory)
     unsigned long long t_start;        // the launch's start on this warp (time budget)
     Engine eng;                        // the committed game
-    Stats st;
-    uint32_t seg_off[65];              // a level's candidate segments (the distinct child lists)
-    uint32_t seg_info[64];             // rec (6) | list (rank * 2 + child, 6) << 8 | piece << 16 | held-is-I << 20
-                                       // | lists it stands for << 22
-    uint32_t grp0[32], grp1[32];       // per parent: the parents whose child list 0 / 1 equals its own
+    // a level's candidate segments (the distinct child lists): x = first candidate | end << 16,
+    // y = rec (6) | list (rank * 2 + child, 6) << 8 | piece * MP << 16 | held-is-I << 24 | lists it stands for << 25
+    uint2 seg[2 * K2];
+    uint32_t grp0[K2], grp1[K2];       // per parent: the parents whose child list 0 / 1 equals its own
                                        // (grp1 = 0: list 1 equals the parent's own list 0)
     uint32_t merged;                   // parents whose list 1 equals their list 0
-    uint32_t defer[64];                // queued (segment << 8 | placement) for the full path
+    Stats st;
+    uint32_t illegal[16];              // per segment (a byte each) its placements that turned out illegal
+    uint16_t seg_of[K2];               // per parent its lists' segments, list 1's << 8
+    uint16_t defer[64];                // queued (segment << 8 | flat placement index) for the full path
+    // ---- the widened networks' warp areas end here (kWideWarpBytes)
+    alignas(16) float wfull[NPARAMS + 3];   // the v11 model's weights (full path, record partial sums)
     alignas(8) uint64_t kbuf[WARP];    // a level's keys above the top-K threshold, not yet merged
     // team kernels (TEAM warps per game; the game lives in the leader's area)
     alignas(8) unsigned long long team_bar;   // game area: the team's barrier (an mbarrier of TEAM arrivals)
@@ -532,6 +557,8 @@ struct alignas(16) WarpShared {
     uint32_t team_broken;              // this warp: a team wait ran out
     uint32_t pad_team_[2];
 };
+constexpr size_t kWideWarpBytes = offsetof(WarpShared, wfull);
+static_assert(kWideWarpBytes % 16 == 0, "warp blocks must keep 16-byte alignment");
 static_assert(sizeof(WarpShared) % 16 == 0, "warp blocks must keep 16-byte alignment");
 
 // The team barrier (pr[0] the leader's area, pr[r] warp r's): an mbarrier in the game area that
@@ -597,6 +624,7 @@ struct Params {
     uint32_t ckpt_cap;
     uint32_t handoff_at;               // hand-off flavour: hand the games over when at most this many play
     uint32_t resume;                   // paired kernel: play the checkpointed games instead of the sims
+    float neg_zero;                    // -0: a value the compiler does not know (eval_core.h, MLP_X2FMA)
     uint32_t test_flags;               // tests only: bit 0 = team partners leave at launch start, so
                                        // the leaders' first team wait runs out (status bit 4)
 };
@@ -620,7 +648,6 @@ struct LevelAcc {
     uint64_t list;                     // top-K list (STAGE_TOPK)
     uint64_t best;                     // argmax of leaf keys and fallbacks (STAGE_LEAF)
     uint64_t best2;                    // the second-largest leaf key (tracing flavour only)
-    uint32_t lo, hi;                   // bit (rank * 2 + child): that child list has a legal placement
 };
 
 // keep the two largest keys (keys are unique per move, 0 = none)
@@ -647,38 +674,54 @@ __device__ __forceinline__ void warp_top2(uint64_t& b1, uint64_t& b2) {
 
 __device__ __forceinline__ uint64_t candidate_key(bool leaf, float v, uint32_t info, uint32_t i) {
     uint32_t const pos = ((info >> 8) & 63u) * MP + i;                     // beam.hpp:296,360,423
-    uint32_t const low = leaf ? uint32_t(ORDER_SPAN) - pos : 0xFFFFFFFFu - pos;   // beam.hpp:217-219
+    uint32_t const low = (leaf ? uint32_t(ORDER_SPAN) : 0xFFFFFFFFu) - pos;       // beam.hpp:217-219
     return (uint64_t(ordered_bits(v)) << 32) | uint64_t(low);
+}
+__device__ __forceinline__ uint32_t seg_flat(uint32_t info) { return (info >> 16) & 0xFFu; }   // piece * MP
+__device__ __forceinline__ bool seg_held(uint32_t info) { return (info >> 24) & 1u; }
+__device__ __forceinline__ uint32_t seg_lists(uint32_t info) { return info >> 25; }
+__device__ __forceinline__ uint32_t make_seg_info(uint32_t rec, uint32_t list, uint32_t piece, uint32_t held, uint32_t lists) {
+    return rec | (list << 8) | ((piece * uint32_t(MP)) << 16) | (held << 24) | (lists << 25);
 }
 
 struct Luts {
-    PlaceFast const (*fast)[MP];
-    uint32_t const (*move)[MP];
+    Word4 const* fast0;
+    Word4 const* fast1;
+    uint32_t const* move;
 };
+__device__ __forceinline__ PlaceFast load_place(Luts const& lut, uint32_t flat) {
+    uint4 const a = *reinterpret_cast<uint4 const*>(lut.fast0 + flat), b = *reinterpret_cast<uint4 const*>(lut.fast1 + flat);
+    return PlaceFast{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+}
 
-// Full path for one queued candidate (segment << 8 | placement): its key, or 0 if illegal.
+// An illegal candidate (only the full path meets one): counted in its segment, and its evaluations,
+// which the level's total included, taken back.
+__device__ __forceinline__ void count_illegal(WarpShared* ws, uint32_t seg, uint32_t info, uint32_t& evals) {
+    atomicAdd(&ws->illegal[seg >> 2], 1u << (8u * (seg & 3u)));
+    evals -= seg_lists(info);
+}
+
+// Full path for one queued candidate (segment << 8 | flat placement index): its key, or 0 if illegal.
 // A legal candidate's key is never 0 (its low word is a positive position).
 __device__ __noinline__ uint64_t full_key(WarpShared* ws, Luts lut, bool leaf, uint32_t entry) {
-    uint32_t const seg = entry >> 8, i = entry & 0xFFu;
-    uint32_t const info = ws->seg_info[seg];
+    uint32_t const info = ws->seg[entry >> 8].y, flat = entry & 0xFFu;
     uint32_t const* rec = ws->rec[info & 63u];
-    uint32_t const mv = lut.move[(info >> 16) & 7u][i];
+    uint32_t const mv = lut.move[flat];
     Applied const a = apply_ints(rec + R_BOARD, mv & 0xFFFFu, int((mv >> 16) & 0xFu), nullptr);
     if (!a.legal) return 0;
-    float const v = value_full(rec[R_CLEARS] + clear_bump(a.cleared), a.bi, (info >> 20) & 1u, SmemW{ws->wfull});
-    return candidate_key(leaf, v, info, i);
+    float const v = value_full(rec[R_CLEARS] + clear_bump(a.cleared), a.bi, seg_held(info), SmemW{ws->wfull});
+    return candidate_key(leaf, v, info, flat - seg_flat(info));
 }
 
 // The widened network's full path, first half: is the queued candidate legal,
 // and its inputs (all zero when it is not).
 __device__ __noinline__ bool full_inputs_wide(WarpShared* ws, Luts lut, uint32_t entry, WideIn& in) {
-    uint32_t const seg = entry >> 8, i = entry & 0xFFu;
-    uint32_t const info = ws->seg_info[seg];
+    uint32_t const info = ws->seg[entry >> 8].y, flat = entry & 0xFFu;
     uint32_t const* rec = ws->rec[info & 63u];
-    uint32_t const mv = lut.move[(info >> 16) & 7u][i];
+    uint32_t const mv = lut.move[flat];
     Applied const a = apply_ints(rec + R_BOARD, mv & 0xFFFFu, int((mv >> 16) & 0xFu), nullptr);
     if (!a.legal) return false;
-    wide_inputs(rec[R_CLEARS] + clear_bump(a.cleared), a.bi, (info >> 20) & 1u, in.v);
+    wide_inputs(rec[R_CLEARS] + clear_bump(a.cleared), a.bi, seg_held(info), in.v);
     return true;
 }
 
@@ -691,32 +734,27 @@ __device__ __noinline__ bool full_inputs_wide(WarpShared* ws, Luts lut, uint32_t
 //
 // The top-kl list (lane i = i-th largest, 0 = empty; thr = list[kl-1]): keys are unique per level
 // (the low word encodes the slot), so the kept set equals beam.hpp:244-265's "max score, lowest
-// slot on ties" whatever the order keys arrive in. The single-warp kernels insert each key above
-// thr at once (topk_fold). The team kernels keep the list lazily: keys above thr go to the
-// warp's key buffer, and when a round's keys would overflow it (or the level ends) the buffer is
-// sorted across the lanes and merged into the list, which raises thr; a key at or below a stale
-// thr is below the final list[kl-1] too. The lazy merge shortens a warp's critical path (15 %
-// per move for a warp alone on its scheduler) but executes more instructions, which costs 3-5 %
-// at 16 warps per SM, where the single-warp kernels run.
+// slot on ties" whatever the order keys arrive in. The v11 kernels keep the list lazily: keys above thr
+// go to the warp's key buffer, and when a round's keys would overflow it (or the level ends) the buffer is
+// sorted across the lanes and merged into the list, which raises thr; a key at or below a stale thr is
+// below the final list[kl-1] too. Team kernels sort in straight-line code (a warp alone on its scheduler
+// waits for every shuffle: 15.4 ms for 30 champion games, 16.9 ms with the loop), the single-warp kernels
+// in a loop (merge_keys: a generation takes 233 ms with it, 238 ms inserting each key at once). The
+// widened kernels insert each key at once (topk_fold; their warp areas have no buffer).
+// Measured with this loop, its records and placement data, start -> now: generation 341.6 -> 233.5 ms,
+// default generation 52.4 -> 36.0 ms, 30 champion games 17.9 -> 15.3 ms; 36,800 warp instructions a move of a
+// champion's game at 16 warps per SM (ncu).
 template <int NET, bool KEYS, int TEAM = 1>
 __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, Luts lut, FastW const& fw, float* hb,
                                                bool leaf, uint32_t total, int kl, int lane, uint32_t& evals,
                                                uint32_t first = 0) {
     constexpr bool WIDE = NET != 0;
     constexpr int HW = WIDE ? NET : 64;     // the widened network's width (unused for v11)
-    uint32_t* const dq = own.defer;
+    uint16_t* const dq = own.defer;
     uint64_t* const kb = own.kbuf;
     constexpr bool TEAMED = TEAM > 1;
-    constexpr bool LAZY = TEAMED;
-    LevelAcc acc{0, 0, 0, 0, 0, 0};
-    auto consume = [&](uint64_t key, uint32_t info) {
-        if (key) {
-            evals += info >> 22;
-            uint32_t const bit = (info >> 8) & 63u;
-            if (bit < 32) acc.lo |= 1u << bit;
-            else acc.hi |= 1u << (bit - 32);
-        }
-    };
+    constexpr bool LAZY = !WIDE;
+    LevelAcc acc{0, 0, 0, 0};
     // Each iteration is one round of 32 fast-path candidates (one per lane) or, once 32 are
     // queued (or the level is done), one batch of up to 32 deferred candidates through the full
     // path; either way its keys are folded at one place. Keys are unique within a level, so the
@@ -725,7 +763,8 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
     // per lane in straight-line code measured slower (681 ms vs 486 ms per full generation).
     uint32_t queued = 0;          // < 32 at the start of every fast round: the queue holds 64
     uint32_t kcnt = 0;            // keys in the key buffer (non-leaf levels)
-    int seg = 0;
+    int seg = -1;
+    uint2 sg = make_uint2(0u, 0u);         // this lane's segment (none yet)
     uint32_t c0 = TEAMED ? first : 0u;
     for (;;) {
         bool const more = c0 < total;
@@ -750,22 +789,22 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
                 }
                 __syncwarp();
                 float const v = wide_value<HW>(in, ws.wglobal, hb, lane);
-                if (legal) {
-                    uint32_t const info = ws.seg_info[entry >> 8];
-                    key = candidate_key(leaf, v, info, entry & 0xFFu);
-                    consume(key, info);
+                if (uint32_t(lane) < n) {
+                    uint32_t const info = ws.seg[entry >> 8].y;
+                    if (legal) key = candidate_key(leaf, v, info, (entry & 0xFFu) - seg_flat(info));
+                    else count_illegal(&ws, entry >> 8, info, evals);
                 }
             } else if (uint32_t(lane) < n) {
                 uint32_t const entry = dq[lane];
                 key = full_key(&ws, lut, leaf, entry);
-                consume(key, ws.seg_info[entry >> 8]);
+                if (!key) count_illegal(&ws, entry >> 8, ws.seg[entry >> 8].y, evals);
             }
             uint32_t const rem = queued - n;
             uint32_t t = 0;
             __syncwarp();
             if (uint32_t(lane) < rem) t = dq[n + lane];
             __syncwarp();
-            if (uint32_t(lane) < rem) dq[lane] = t;
+            if (uint32_t(lane) < rem) dq[lane] = uint16_t(t);
             __syncwarp();
             queued = rem;
         } else {
@@ -773,25 +812,22 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
             uint32_t const c = c0 + uint32_t(lane);
             bool const valid = c < total;
             uint32_t const cc = valid ? c : total - 1u;          // out of range: the last candidate, discarded
-            while (ws.seg_off[seg + 1] <= cc) ++seg;
-            uint32_t const sg = uint32_t(seg);
-            uint32_t const info = ws.seg_info[seg];
-            uint32_t const idx = cc - ws.seg_off[seg];
+            while ((sg.x >> 16) <= cc) sg = ws.seg[++seg];
+            uint32_t const info = sg.y;
+            uint32_t const idx = cc - (sg.x & 0xFFFFu), flat = seg_flat(info) + idx;
             float v;
             int st;
             if constexpr (WIDE)
-                st = fast_candidate_wide<HW>(ws.rec[info & 63u], lut.fast[(info >> 16) & 7u][idx], (info >> 20) & 1u,
-                                             ws.wglobal, hb, lane, v);
+                st = fast_candidate_wide<HW>(ws.rec[info & 63u], load_place(lut, flat), seg_held(info), ws.wglobal, hb, lane, v);
             else
-                st = fast_candidate(ws.rec[info & 63u], lut.fast[(info >> 16) & 7u][idx], (info >> 20) & 1u, fw, v);
+                st = fast_candidate(ws.rec[info & 63u], load_place(lut, flat), seg_held(info), fw, v);
             bool const def = valid && st != FAST_OK;
-            if (valid && st == FAST_OK) {
-                key = candidate_key(leaf, v, info, idx);
-                consume(key, info);
-            }
+            if (valid && st == FAST_OK) key = candidate_key(leaf, v, info, idx);
             uint32_t const dm = __ballot_sync(FULL_MASK, def);
-            if (def) dq[queued + __popc(dm & ((1u << lane) - 1u))] = (sg << 8) | idx;
-            queued += __popc(dm);
+            if (dm) {
+                if (def) dq[queued + __popc(dm & ((1u << lane) - 1u))] = uint16_t((uint32_t(seg) << 8) | flat);
+                queued += __popc(dm);
+            }
             c0 += uint32_t(TEAM * WARP);
         }
         if (leaf) {
@@ -804,8 +840,8 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
             uint32_t n = __popc(m);
             if (fin || kcnt + n > uint32_t(WARP)) {          // merge the buffer into the list
                 __syncwarp();
-                uint64_t const b = warp_sort_desc(uint32_t(lane) < kcnt ? kb[lane] : 0ull, lane);
-                acc.list = merge_topk(acc.list, b, kl, lane);
+                uint64_t const b = uint32_t(lane) < kcnt ? kb[lane] : 0ull;
+                acc.list = TEAMED ? merge_topk(acc.list, warp_sort_desc(b, lane), kl, lane) : merge_keys(acc.list, b, kl, lane);
                 acc.thr = shfl64(acc.list, kl - 1);
                 kcnt = 0;
                 m = __ballot_sync(FULL_MASK, key > acc.thr);
@@ -825,7 +861,7 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
 // Two kept nodes often hold the same board and clear histogram: the same placements reached in another
 // order through the hold slot. Their child lists with the same piece and held-is-I flag then hold the
 // same candidates with the same values, so one of them (the lowest list, the representative) is evaluated
-// and stands for all: its evaluations count once per list (seg_info), its legality holds for each
+// and stands for all: its evaluations count once per list, its legality holds for each
 // (list_legal), its leaf keys beat the copies' (lower position), and in the other levels the copies of the
 // kept keys enter the top-K afterwards (expand_copies). Equality is exact: nodes are grouped by a hash of
 // the record's board words and compared word by word with their group's first node. On the generation
@@ -835,7 +871,7 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
 // dedup = false: every list stands for itself (the key-tracing flavour, whose second-best key may be a copy;
 // level 1 unless both root groups place the same piece, the only way to the same board there but for clears).
 __device__ __forceinline__ uint32_t build_segments(WarpShared& ws, uint32_t const* slot_piece, int tree, int level,
-                                                   uint32_t fnode, int kept, bool dedup, int lane) {
+                                                   uint32_t fnode, int kept, bool dedup, int lane, uint32_t& evals) {
     bool const active = lane < kept;
     uint32_t piece[2], held[2];
 #pragma unroll
@@ -885,34 +921,38 @@ __device__ __forceinline__ uint32_t build_segments(WarpShared& ws, uint32_t cons
         if (lane >= o) incl += n;
     }
     uint32_t off = (incl - own) & 0xFFFFu, s = (incl - own) >> 16;
-    uint32_t const list = uint32_t(lane) | (uint32_t(2 * lane) << 8);
+    uint32_t const list = uint32_t(2 * lane), first_seg = s;
     if (cnt0) {
-        ws.seg_off[s] = off;
-        ws.seg_info[s++] = list | (piece[0] << 16) | (held[0] << 20) | (uint32_t(__popc(m0) + __popc(m0 & merged)) << 22);
+        uint32_t const lists = uint32_t(__popc(m0) + __popc(m0 & merged));
+        ws.seg[s++] = make_uint2(off | ((off + cnt0) << 16), make_seg_info(uint32_t(lane), list, piece[0], held[0], lists));
         off += cnt0;
+        evals += cnt0 * lists;
     }
     if (cnt1) {
-        ws.seg_off[s] = off;
-        ws.seg_info[s] = list | (1u << 8) | (piece[1] << 16) | (held[1] << 20) | (uint32_t(__popc(m1)) << 22);
+        uint32_t const lists = uint32_t(__popc(m1));
+        ws.seg[s] = make_uint2(off | ((off + cnt1) << 16), make_seg_info(uint32_t(lane), list + 1u, piece[1], held[1], lists));
+        evals += cnt1 * lists;
     }
     ws.grp0[lane] = m0;
     ws.grp1[lane] = m1;
-    uint32_t const all = __shfl_sync(FULL_MASK, incl, 31);
-    if (lane == 0) {
-        ws.merged = merged;
-        ws.seg_off[all >> 16] = all & 0xFFFFu;
-    }
+    ws.seg_of[lane] = uint16_t(first_seg | (s << 8));
+    if (lane < 16) ws.illegal[lane] = 0;
+    if (lane == 0) ws.merged = merged;
     __syncwarp();
-    return all & 0xFFFFu;
+    return __shfl_sync(FULL_MASK, incl, 31) & 0xFFFFu;
 }
 
-// Bit c: parent `lane`'s child list c has a legal placement (lo, hi: the warp's bits of the lists evaluated).
-__device__ __forceinline__ uint32_t list_legal(WarpShared const& ws, uint32_t lo, uint32_t hi, int lane) {
+// Bit c: parent `lane`'s child list c has a legal placement (not every one of its segment's is illegal).
+__device__ __forceinline__ uint32_t list_legal(WarpShared const& ws, int lane) {
+    if (!__any_sync(FULL_MASK, lane < 16 && ws.illegal[lane & 15] != 0u)) return 3u;
+    auto legal = [&](uint32_t seg) {
+        uint32_t const x = ws.seg[seg].x;
+        return ((ws.illegal[seg >> 2] >> (8u * (seg & 3u))) & 0xFFu) < (x >> 16) - (x & 0xFFFFu);
+    };
     uint32_t const g0 = ws.grp0[lane], g1 = ws.grp1[lane];
-    uint64_t const bits = (uint64_t(hi) << 32) | lo;
-    uint32_t const l0 = uint32_t(bits >> (2 * (__ffs(int(g0)) - 1))) & 1u;
-    uint32_t const l1 = g1 ? uint32_t(bits >> (2 * (__ffs(int(g1)) - 1) + 1)) & 1u : l0;
-    return l0 | (l1 << 1);
+    bool const l0 = legal(ws.seg_of[__ffs(int(g0)) - 1] & 0xFFu);
+    bool const l1 = g1 ? legal(uint32_t(ws.seg_of[__ffs(int(g1)) - 1]) >> 8) : l0;
+    return uint32_t(l0) | (uint32_t(l1) << 1);
 }
 
 // A level's kept keys of the evaluated lists -> the kept keys of all its lists: each key's copies (the same
@@ -963,9 +1003,9 @@ __device__ __noinline__ void materialize(WarpShared* ws, Luts lut, bool active, 
         uint32_t const* pr = ws->rec[prec];
         uint32_t b[W];
         load_board(pr + R_BOARD, b);
-        uint32_t const mv = lut.move[piece][i];
+        uint32_t const mv = lut.move[piece * uint32_t(MP) + i];
         int cl = 0;
-        apply_full(b, mv & 0xFFFFu, int((mv >> 16) & 0xFu), nb, cl);
+        apply_full(pr + R_BOARD, b, mv & 0xFFFFu, int((mv >> 16) & 0xFu), nb, cl);
         ncl = pr[R_CLEARS] + clear_bump(cl);
     }
     __syncwarp();
@@ -1030,18 +1070,18 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             break;
         } else if (stage == 0) {               // two root groups over the committed board (beam.hpp:283-301)
             root_record<WIDE>(&ws, lut, lane);
+            uint32_t const n0 = c_tables.nplace[p0];
+            total = n0 + c_tables.nplace[p1];
             if (lane < 2) {
                 uint32_t const nd = lane ? r1 : r0;
                 uint32_t const held_slot = (nd >> 4) & 0xFu;
                 uint32_t const held_i = held_slot != HELD_NONE && slot_piece[held_slot] == 0u;
-                ws.seg_info[lane] = 32u | (uint32_t(lane) << 8) | ((lane ? p1 : p0) << 16) | (held_i << 20) | (1u << 22);
+                ws.seg[lane] = make_uint2(lane ? n0 | (total << 16) : n0 << 16,
+                                          make_seg_info(32u, uint32_t(lane), lane ? p1 : p0, held_i, 1u));
             }
-            total = c_tables.nplace[p0] + c_tables.nplace[p1];
             if (lane == 0) {
-                ws.seg_off[0] = 0;
-                ws.seg_off[1] = c_tables.nplace[p0];
-                ws.seg_off[2] = total;
-                ws.seg_off[3] = total;
+                ws.illegal[0] = 0;
+                evals += total;
             }
             __syncwarp();
         } else {
@@ -1049,7 +1089,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             // against the 5 us that the copies' rounds take there: 18.3 against 17.9 ms for 30 champion
             // games), so they evaluate every list
             dedup = !KEYS && TEAM < 4 && (stage > 1 || p0 == p1);
-            total = build_segments(ws, slot_piece, tree, stage, fnode, kept, dedup, lane);
+            total = build_segments(ws, slot_piece, tree, stage, fnode, kept, dedup, lane, evals);
         }
         if (TEAMED && !partner) {                // post the stage
             if (lane == 0) {
@@ -1064,7 +1104,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
         // team kernels reload the fast-path weights for each pass (from L1), so that they hold no
         // registers across the team barriers
         FastW fwl;
-        if (TEAMED) load_fast_weights(GlobalW{ws.wglobal}, fwl);
+        if (TEAMED) load_fast_weights(GlobalW{ws.wglobal}, fwl, fw.nz);
         LevelAcc a = level_pass<NET, KEYS, TEAM>(ws, pr[rank], lut, TEAMED ? fwl : fw, hb, leaf, total, kl, lane, evals,
                                                  uint32_t(rank * WARP));
         if (TEAMED) {
@@ -1072,11 +1112,6 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             if (partner) {
                 uint32_t* const x = pr[rank].rec[0];
                 reinterpret_cast<uint64_t*>(x)[lane] = leaf ? a.best : a.list;
-                uint32_t const lo = __reduce_or_sync(FULL_MASK, a.lo), hi = __reduce_or_sync(FULL_MASK, a.hi);
-                if (lane == 0) {
-                    x[X_LO] = lo;
-                    x[X_HI] = hi;
-                }
                 if (!team_sync(pr, rank, status, lane)) return mv;
                 continue;
             }
@@ -1087,8 +1122,6 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
                 uint64_t const b = reinterpret_cast<uint64_t const*>(x)[lane];
                 if (leaf) a.best = b > a.best ? b : a.best;
                 else a.list = merge_topk(a.list, b, kl, lane);
-                a.lo |= x[X_LO];
-                a.hi |= x[X_HI];
             }
         }
         if (stage == 0) {
@@ -1101,7 +1134,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             fnode = g;
             materialize<WIDE>(&ws, lut, lane < kept, 32u, g ? p1 : p0, root_slot % MP, lane);
         } else if (!leaf) {
-            uint32_t const legal = list_legal(ws, __reduce_or_sync(FULL_MASK, a.lo), __reduce_or_sync(FULL_MASK, a.hi), lane);
+            uint32_t const legal = list_legal(ws, lane);
             if (dedup) a.list = expand_copies<TEAMED>(&ws, a.list, kl, lane);
             // kept nodes with no legal continuation become leaves at this depth (beam.hpp:549-551)
             if (lane < kept && !legal) {
@@ -1125,7 +1158,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             kept = next;
         } else {
             // ---- leaf stage (beam.hpp:407-443): a list whose piece never fit scores the frontier board
-            uint32_t const legal = list_legal(ws, __reduce_or_sync(FULL_MASK, a.lo), __reduce_or_sync(FULL_MASK, a.hi), lane);
+            uint32_t const legal = list_legal(ws, lane);
             if (KEYS) {
                 top2_insert(best, best2, a.best);
                 top2_insert(best, best2, a.best2);
@@ -1159,7 +1192,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
     uint32_t const root_rank = order >= uint32_t(LEAF_ORDERS) ? order - LEAF_ORDERS : leaf_rank;
     uint32_t const rs = __shfl_sync(FULL_MASK, root_slot, int(root_rank & 31u));
     uint32_t const g = rs / MP;
-    uint32_t const pa = lut.move[g ? p1 : p0][rs % MP];
+    uint32_t const pa = lut.move[(g ? p1 : p0) * uint32_t(MP) + rs % MP];
     mv.orient = int((pa >> 20) & 3u);
     mv.x = int((pa >> 24) & 0xFu) - 2;
     mv.hold = int((c_tables.node[tree][0][g] >> 8) & 1u);
@@ -1225,15 +1258,17 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) eval_kernel(Params p) {
     static_assert(!HANDOFF || (!WIDE && !BUDGET && !KEYS && !TEAMED), "hand-off: the single-warp v11 kernel");
     extern __shared__ __align__(16) unsigned char dyn_smem[];    // WARPS x WarpShared
     __shared__ LutTables s_lut;
-    for (int t = int(threadIdx.x); t < NPIECE * MP; t += WARPS * 32) {
-        s_lut.fast[t / MP][t % MP] = g_lut.fast[t / MP][t % MP];
-        s_lut.move[t / MP][t % MP] = g_lut.move[t / MP][t % MP];
+    for (int t = int(threadIdx.x); t < NFLAT; t += WARPS * 32) {
+        s_lut.fast[0][t] = g_lut.fast[0][t];
+        s_lut.fast[1][t] = g_lut.fast[1][t];
+        s_lut.move[t] = g_lut.move[t];
     }
     int const lane = int(threadIdx.x & 31u);
     int const rank = TEAMED ? int((threadIdx.x >> 5) & uint32_t(TEAM - 1)) : 0;
     bool const partner = rank != 0;
     // TEAM > 1: pr[0] is the team's game (the leader's area), pr[r] warp r's area
-    WarpShared* const pr = reinterpret_cast<WarpShared*>(dyn_smem) + ((threadIdx.x >> 5) & ~uint32_t(TEAM - 1));
+    constexpr size_t AREA = WIDE ? kWideWarpBytes : sizeof(WarpShared);
+    WarpShared* const pr = reinterpret_cast<WarpShared*>(dyn_smem + ((threadIdx.x >> 5) & ~uint32_t(TEAM - 1)) * AREA);
     WarpShared& ws = pr[0];
     if (TEAMED && lane == 0) {
         if (!partner) team_bar_init(pr, uint32_t(TEAM));
@@ -1242,9 +1277,9 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) eval_kernel(Params p) {
     if (HANDOFF && lane == 0) ws.eng.over = 0;                 // (read after the game loop)
     __syncthreads();
     if (TEAMED && partner && (p.test_flags & 1u)) return;      // (no later block barrier)
-    Luts const lut{s_lut.fast, s_lut.move};
+    Luts const lut{s_lut.fast[0], s_lut.fast[1], s_lut.move};
     // the widened network's per-warp hidden-unit buffers follow the WARPS warp blocks
-    float* const hb = WIDE ? reinterpret_cast<float*>(dyn_smem + WARPS * sizeof(WarpShared)) +
+    float* const hb = WIDE ? reinterpret_cast<float*>(dyn_smem + WARPS * AREA) +
                                  (threadIdx.x >> 5) * kWideHbFloats<HW>
                            : nullptr;
     // time budget, measured from this warp's start (the persistent grid starts every warp at launch);
@@ -1295,7 +1330,8 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) eval_kernel(Params p) {
         }
         FastW fw;
         uint32_t evals = 0, moves = 0;
-        if (!WIDE) load_fast_weights(GlobalW{wsrc}, fw);
+        fw.nz = p.neg_zero;
+        if (!WIDE) load_fast_weights(GlobalW{wsrc}, fw, p.neg_zero);
         if (!partner) {
             if (!WIDE)
                 for (int i = lane; i < NPARAMS; i += WARP) ws.wfull[i] = __ldg(wsrc + i);
@@ -1410,31 +1446,33 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) eval_kernel(Params p) {
 // candidate, fast path and full path on caller-built records. cand[t] =
 // piece | placement << 8 | held-is-I << 16 | record index << 17.
 __global__ void core_selftest_kernel(uint32_t const* recs, uint32_t const* cand, uint32_t n, float const* w,
-                                     float* fast_v, int* fast_st, float* full_v, int* full_legal, float* dbg) {
+                                     float* fast_v, int* fast_st, float* full_v, int* full_legal, float* dbg, float nz) {
     uint32_t const t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     uint32_t const c = cand[t];
     uint32_t const piece = c & 0xFFu, i = (c >> 8) & 0xFFu, held = (c >> 16) & 1u;
     uint32_t const* rec = recs + size_t(c >> 17) * REC_WORDS;
     FastW fw;
-    load_fast_weights(GlobalW{w}, fw);
+    load_fast_weights(GlobalW{w}, fw, nz);
     float v = 0.0f;
     // the kernel's own arithmetic mode, then (diagnostics) every MLP mode: scalar, packed
     // intrinsics, packed PTX
-    fast_st[t] = fast_candidate(rec, g_lut.fast[piece][i], held, fw, v, dbg ? dbg + size_t(t) * 32 : nullptr);
+    Luts const lut{g_lut.fast[0], g_lut.fast[1], g_lut.move};
+    PlaceFast const pf = load_place(lut, piece * uint32_t(MP) + i);
+    fast_st[t] = fast_candidate(rec, pf, held, fw, v, dbg ? dbg + size_t(t) * 32 : nullptr);
     if (dbg) {
         float v2 = 0.0f, v3 = 0.0f, v4 = 0.0f, v5 = 0.0f;
-        fast_candidate<MLP_PTX_X2>(rec, g_lut.fast[piece][i], held, fw, v2, nullptr);
-        fast_candidate<MLP_X2>(rec, g_lut.fast[piece][i], held, fw, v3, nullptr);
-        fast_candidate<MLP_SCALAR>(rec, g_lut.fast[piece][i], held, fw, v4, nullptr);
-        fast_candidate<MLP_X2MUL>(rec, g_lut.fast[piece][i], held, fw, v5, nullptr);
+        fast_candidate<MLP_PTX_X2>(rec, pf, held, fw, v2, nullptr);
+        fast_candidate<MLP_X2>(rec, pf, held, fw, v3, nullptr);
+        fast_candidate<MLP_SCALAR>(rec, pf, held, fw, v4, nullptr);
+        fast_candidate<MLP_X2MUL>(rec, pf, held, fw, v5, nullptr);
         dbg[size_t(t) * 32 + 28] = v5;
         dbg[size_t(t) * 32 + 29] = v4;
         dbg[size_t(t) * 32 + 30] = v3;
         dbg[size_t(t) * 32 + 31] = v2;
     }
     fast_v[t] = v;
-    uint32_t const mv = g_lut.move[piece][i];
+    uint32_t const mv = g_lut.move[piece * uint32_t(MP) + i];
     uint32_t b[W], nb[W];
     for (int x = 0; x < W; ++x) b[x] = rec[R_BOARD + x];
     int cl = 0;
@@ -1494,7 +1532,9 @@ constexpr int kNumVariants = int(sizeof(kVariants) / sizeof(kVariants[0]));
 enum NetKind { NET_V11 = 0, NET_W64 = 1, NET_W32 = 2, NUM_NETS = 3 };
 constexpr int net_width(int ni) { return ni == NET_W64 ? 64 : ni == NET_W32 ? 32 : 0; }
 // dynamic shared memory per warp: its WarpShared block, plus the widened network's hidden-unit buffer
-constexpr size_t warp_bytes(int ni) { return sizeof(WarpShared) + size_t(net_width(ni)) * WARP * sizeof(float); }
+constexpr size_t warp_bytes(int ni) {
+    return ni == NET_V11 ? sizeof(WarpShared) : kWideWarpBytes + size_t(net_width(ni)) * WARP * sizeof(float);
+}
 // the widened networks' launch shapes (more registers per lane than v11): width 64 at 2 blocks
 // of 4 warps per SM (255 registers), width 32 at 3
 Variant const kWideNet[NUM_NETS] = {{nullptr, 0, 0}, {eval_kernel<4, 2, 64>, 4, 2}, {eval_kernel<4, 3, 32>, 4, 3}};
@@ -1638,7 +1678,9 @@ int set_min_carveout(ta3b_ctx* ctx, Variant const& v, size_t dyn) {
     cudaFuncAttributes fa{};
     TA3B_CUDA(ctx, cudaFuncGetAttributes(&fa, v.fn), "kernel attributes");
     size_t const need = size_t(v.min_blocks) * (dyn + fa.sharedSizeBytes + size_t(reserved));
-    int const pct = per_sm > 0 ? int((need * 100 + size_t(per_sm) - 1) / size_t(per_sm)) : 100;
+    // rounded down: the driver takes the smallest split that holds this share, and the caller checks that
+    // the blocks fit (rounded up, 166,384 bytes ask for 72 % = 168,100 and get 196 KB in place of 164 KB)
+    int const pct = per_sm > 0 ? int(need * 100 / size_t(per_sm)) : 100;
     TA3B_CUDA(ctx, cudaFuncSetAttribute(v.fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct < 100 ? pct : 100),
               "smem carveout");
     return TA3B_OK;
@@ -1708,6 +1750,7 @@ int launch(ta3b_ctx* ctx, Params const& prm, cudaStream_t st, int ni = NET_V11) 
     uint32_t const grid = spread ? (sims < ctx->sms ? (sims ? sims : 1u) : ctx->sms)
                                  : (need_blocks < max_grid ? need_blocks : max_grid);
     Params p2 = prm;
+    p2.neg_zero = -0.0f;
     p2.warps_active = spread ? (sims + grid - 1) / grid * (warps / games) : 0u;
     p2.budget_ns = ctx->budget_ns;
     p2.test_flags = ctx->test_flags;
@@ -2048,7 +2091,7 @@ int ta3b_core_selftest(uint32_t const* recs, uint32_t num_recs, uint32_t const* 
                                                         static_cast<float*>(d[2]), static_cast<float*>(d[3]),
                                                         static_cast<int*>(d[4]), static_cast<float*>(d[5]),
                                                         static_cast<int*>(d[6]),
-                                                        dbg32 ? static_cast<float*>(d[7]) : nullptr);
+                                                        dbg32 ? static_cast<float*>(d[7]) : nullptr, -0.0f);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(fast_v, d[3], sz[3], cudaMemcpyDeviceToHost);
@@ -2221,6 +2264,7 @@ extern "C" int ta3b_eval_device_noalloc(float const* d_weights, uint32_t num_isl
     prm.lines = d_lines;
     prm.evals = d_evals;
     prm.scratch = d.scratch;
+    prm.neg_zero = -0.0f;
     prm.num_games = num_games;
     prm.models_per_island = models_per_island;
     prm.max_moves = max_moves;

@@ -174,19 +174,22 @@ constexpr Tables make_tables() {
 
 constexpr Tables TABLES = make_tables();
 
-// Per-placement data for the incremental candidate path (16 bytes):
-//   d4  byte i = 22 - lowest cell row of piece column i (i < width), 127 beyond
-//   c4  byte i = cells in piece column i (i < width), 0 beyond
-//   m   cells per local row r (nibble r, 16 bits) | combo id (6) << 16 | width==1 << 22
-//       | has left neighbour column << 23 | has right neighbour column << 24
-//       | min over columns of the highest cell row (2) << 25 | window origin c0 (4) << 27
-//   s   sum_{i<w} (22 - low_i) (7) | sum_i cells_i * (22 - low_i) (7) << 7
-//       | sum of squared top-row steps inside the piece (4) << 14 | top row of column 0 (2) << 18
-//       | top row of the last column (2) << 20 | width (3) << 22
-// A combo is one (window origin c0, width w) pair; the 34 combos index the
-// per-parent table of old surface / well terms.
+// Per-placement data for the incremental candidate path, two 16-byte vectors whose
+// fields sit where one instruction takes them out (a byte, a whole word, a top field):
+//   d4    byte i = 128 + (22 - lowest cell row of piece column i) (i < width), 255 beyond
+//   c4    byte i = cells in piece column i (i < width), 0 beyond
+//   neg   byte i = -1 (i < width), 0 beyond
+//   rows  cells per local row r (nibble r, 16 bits)
+//   tops  H - top row of the first column | of the last column << 8 | of the highest cell << 16
+//         | width << 24
+//   adds  sum_{i<w} (22 - low_i) | sum_i cells_i * (22 - low_i) << 8
+//         | sum of squared top-row steps inside the piece << 16 | (width == 1) << 24
+//   combo combo id; a combo is one (window origin c0, width w) pair, and the 34 combos index the
+//         per-parent table of old surface / well terms
+//   span  word offset of the window's byte pair, 2 * (c0 / 4) | bit shift 8 * (c0 % 4) << 8
 struct PlaceFast {
-    uint32_t d4, c4, m, s;
+    uint32_t d4, c4, neg, rows;
+    uint32_t tops, adds, combo, span;
 };
 
 constexpr int combo_id(int c0, int w) {
@@ -213,11 +216,11 @@ constexpr PlaceFast make_place_fast(Place p) {
         first[i] = fi;
         cnt[i] = n;
     }
-    uint32_t d4 = 0, c4 = 0, a1 = 0, a2 = 0, sint = 0, minfirst = 3;
+    uint32_t d4 = 0, c4 = 0, neg = 0, a1 = 0, a2 = 0, sint = 0, minfirst = 3;
     for (uint32_t i = 0; i < 4; ++i) {
-        uint32_t const d = i < width ? 22u - low[i] : 127u;
-        d4 |= d << (8 * i);
+        d4 |= (i < width ? 128u + 22u - low[i] : 255u) << (8 * i);
         c4 |= (i < width ? cnt[i] : 0u) << (8 * i);
+        neg |= (i < width ? 255u : 0u) << (8 * i);
         if (i < width) {
             a1 += 22u - low[i];
             a2 += cnt[i] * (22u - low[i]);
@@ -228,12 +231,11 @@ constexpr PlaceFast make_place_fast(Place p) {
             }
         }
     }
-    int const c0 = p.col0;
-    uint32_t const m = pr | (uint32_t(combo_id(c0, int(width))) << 16) | (uint32_t(width == 1) << 22) |
-                       (uint32_t(c0 > 0) << 23) | (uint32_t(c0 + int(width) < W) << 24) | (minfirst << 25) |
-                       (uint32_t(c0) << 27);
-    uint32_t const s = a1 | (a2 << 7) | (sint << 14) | (first[0] << 18) | (first[width - 1] << 20) | (width << 22);
-    return PlaceFast{d4, c4, m, s};
+    uint32_t const c0 = uint32_t(p.col0), h = uint32_t(H);
+    uint32_t const tops = (h - first[0]) | ((h - first[width - 1]) << 8) | ((h - minfirst) << 16) | (width << 24);
+    uint32_t const adds = a1 | (a2 << 8) | (sint << 16) | (uint32_t(width == 1) << 24);
+    return PlaceFast{d4, c4, neg, pr, tops, adds, uint32_t(combo_id(p.col0, int(width))),
+                     2u * (c0 / 4u) | ((8u * (c0 % 4u)) << 8)};
 }
 
 struct FastTables {
@@ -255,7 +257,7 @@ constexpr bool span_has_no_wells() {
     for (int p = 0; p < NPIECE; ++p)
         for (int i = 0; i < TABLES.nplace[p]; ++i) {
             PlaceFast const f = FAST.place[p][i];
-            uint32_t const w = (f.s >> 22) & 7u;
+            uint32_t const w = f.tops >> 24;
             for (uint32_t c = 0; c + 1 < w; ++c) {
                 uint32_t const nib0 = (uint32_t(TABLES.place[p][i].cols) >> (4 * c)) & 0xFu;
                 uint32_t const nib1 = (uint32_t(TABLES.place[p][i].cols) >> (4 * (c + 1))) & 0xFu;
