@@ -51,10 +51,10 @@ int ta3s_predict(ta3s_model* m, const float* x, uint32_t n, float* mean_out, flo
 
 /* ---- the same scheme for any parameter-vector size (ta3w_*) ----
  * MLP in -> H -> H -> 2 for the widened evaluator's 4,929-parameter vectors
- * (H = 256) or any other size: in_dim >= 1, H a multiple of 128. Each matrix
- * product is one launch of a tcgen05 BF16 GEMM kernel (FP32 accumulation in
- * tensor memory, split-K for the first layer); bias, ReLU, output layer, loss and
- * bias gradients in FP32 on the CUDA cores. Rounding points (BF16, nearest
+ * (H = 256) or any other size: in_dim >= 1, H a multiple of 128. The matrix
+ * products run on tcgen05 BF16 GEMM tiles (FP32 accumulation in tensor memory,
+ * split-K for the first layer), a training step in six launches; bias, ReLU,
+ * output layer, loss, bias gradients and AdamW in FP32 on the CUDA cores. Rounding points (BF16, nearest
  * even): standardised inputs, W1, W2, relu(H1), dH2, dH1; everything else FP32.
  * Parameter vector (ta3w_num_params(in_dim, H) values), INP = in_dim rounded up
  * to a multiple of 128:

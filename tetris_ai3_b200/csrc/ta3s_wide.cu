@@ -4,21 +4,26 @@
 // reference; the C ABI is the ta3w_* part of include/ta3b_surrogate.h.
 //
 // Layer by layer instead of one fused kernel (the first layer's weights alone are
-// H x in = 1.3 M values): every matrix product is one launch of gemm_kernel, a
-// tcgen05.mma (kind::f16, BF16 operands staged in shared memory, FP32
-// accumulators in tensor memory) GEMM on 128 x 128 output tiles with K in
-// stages of 64 and optional split-K; the bias, ReLU, output layer, loss and
-// bias gradients run in small CUDA-core kernels between them. Every reduction
-// runs in a fixed order, so two identical calls give identical bits.
+// H x in = 1.3 M values): every matrix product is a tcgen05.mma (kind::f16, BF16
+// operands staged in shared memory, FP32 accumulators in tensor memory) GEMM on
+// 128 x 64 output tiles with K in stages of 64 and optional split-K. A training
+// step is six launches: F1 = X W1^T (split-K), act1 (sum, bias, ReLU), F2 = H1 W2^T,
+// head (output layer, loss, dH2), dW2 and dH1 side by side (the ReLU mask of layer 1
+// in the epilogue), dW1 with AdamW in its epilogue beside the bias and output-layer
+// gradients and W2's update. Each launch starts while the previous one drains
+// (programmatic dependent launch). Every reduction runs in a fixed order, so two
+// identical calls give identical bits. A step of 256 rows at 4,929 -> 256 takes
+// 45 us (eleven launches and square 128 x 128 tiles loaded by one warpgroup: 440 us),
+// of which six launches' latencies are 24 us and AdamW over 1.3 M parameters 9 us.
 //
-// Operand tiles (128 rows of M or N by 64 of K, BF16, no swizzle) are built from
-// 8 x 8 core matrices of 128 contiguous bytes. An operand whose global rows run
-// along K (K-major) stores element (r, k) at (r/8)*1024 + (k/8)*128 + (r%8)*16 +
-// (k%8)*2 and is described with LBO 128 (next 8 K) and SBO 1024 (next 8 rows);
-// an operand whose global rows run along M/N (MN-major: the weight-gradient
-// products, where K is the batch) stores element (k, r) at (k/8)*2048 +
-// (r/8)*128 + (k%8)*16 + (r%8)*2 with LBO 2048 (next 8 K) and SBO 128 (next 8
-// of M/N). Either way one 16-byte global load fills one core-matrix row.
+// Operand tiles (128 of M or 64 of N by 64 of K, BF16) are stored in rows of 128 bytes (64 elements) with
+// the 128-byte swizzle (the row's eight 16-byte chunks XORed with the row number mod 8), eight rows an
+// atom of 1,024 bytes. An operand whose global rows run along K (K-major) has a row per m or n: SBO 1,024
+// (next 8 rows), 32 bytes on per 16 of K. One whose global rows run along M/N (MN-major: the
+// weight-gradient products, where K is the batch) has a row per k, in blocks of 64 of M/N: SBO 1,024 (next
+// 8 of K), LBO 8,192 (next 64 of M/N), 2,048 bytes on per 16 of K. Either way eight threads copy a
+// contiguous 128-byte line into eight different bank groups (with unswizzled core matrices the same
+// copies took 30 cycles a warp instruction: 4,200 cycles for three stages against 900 now).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -31,27 +36,34 @@
 #include <vector>
 
 #include "../../include/ta3b_surrogate.h"
+#include "column_stats.cuh"
 
 namespace ta3w {
 
-constexpr int TILE = 128;                       // M and N per output tile
+constexpr int TILE = 128;                       // M per output tile, and the padding of rows and inputs
+constexpr int TN = 64;                          // N per output tile: twice the CTAs of a square tile, and two fit an SM
 constexpr int KS = 64;                          // K per shared-memory stage
-constexpr int THREADS = 128;
-constexpr uint32_t OP_BYTES = TILE * KS * 2;    // one operand stage: 16 KB
-constexpr uint32_t S_BAR = 4 * OP_BYTES;        // two stages of A and B, then two mbarriers
-constexpr uint32_t S_TMEM = S_BAR + 16;
-constexpr uint32_t SMEM_BYTES = S_TMEM + 16 + 1024;   // + alignment slack
+constexpr int STAGES = 4;                       // stages in flight: the whole K of a 256-row minibatch
+constexpr int THREADS = 512;                    // 32 warps an SM for the AdamW epilogue (two CTAs)
+constexpr uint32_t A_BYTES = TILE * KS * 2, B_BYTES = TN * KS * 2, STAGE_BYTES = A_BYTES + B_BYTES;   // 16 + 8 KB
+constexpr uint32_t S_BAR = STAGES * STAGE_BYTES;   // the stages, then an mbarrier each
+constexpr uint32_t S_TMEM = S_BAR + 8 * STAGES;
+constexpr uint32_t S_ROWS = S_TMEM + 16;        // operand row maps: 128 of A's M, or up to 1,024 of B's K
+constexpr int MAP_ROWS = 1024;
+constexpr uint32_t SMEM_BYTES = S_ROWS + 4 * MAP_ROWS + 1024;   // + alignment slack
+constexpr int LDT = TN + 4;                     // row stride of an output tile in shared memory (16-byte rows, 4 banks apart)
+static_assert(TILE * LDT * 4 <= int(S_BAR), "the output tile reuses the stages");
 constexpr long long WAIT_LIMIT_CYCLES = 4000000000LL;  // ~2 s at 1.9 GHz
 
-// tcgen05 shared-memory matrix descriptor: start, LBO, SBO (all >> 4), version 1, no swizzle
+// tcgen05 shared-memory matrix descriptor: start, LBO, SBO (all >> 4), version 1, 128-byte swizzle
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
     return uint64_t((saddr >> 4) & 0x3FFF) | (uint64_t((lbo >> 4) & 0x3FFF) << 16) |
-           (uint64_t((sbo >> 4) & 0x3FFF) << 32) | (uint64_t(1) << 46);
+           (uint64_t((sbo >> 4) & 0x3FFF) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61);
 }
-// instruction descriptor: D F32, A/B BF16, majors (0 = K, 1 = MN), N = 128, M = 128
+// instruction descriptor: D F32, A/B BF16, majors (0 = K, 1 = MN), N = 64, M = 128
 __host__ __device__ constexpr uint32_t instr_desc(int a_mn, int b_mn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(a_mn) << 15) | (uint32_t(b_mn) << 16) |
-           (uint32_t(TILE >> 3) << 17) | (uint32_t(TILE >> 4) << 24);
+           (uint32_t(TN >> 3) << 17) | (uint32_t(TILE >> 4) << 24);
 }
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     asm volatile(
@@ -98,135 +110,252 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     }
 }
 
+// The previous launch's results are visible after pdl_wait; pdl_go lets the next launch start (it
+// waits for this one to complete in its own pdl_wait, so nothing of it overlaps but its set-up).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Which source row a pass's row r is: r < valid ? (idx ? idx[r] : r) : none (-1, a zero row).
+struct RowMap {
+    int32_t const* idx;
+    int valid;
+    __device__ __forceinline__ int at(int r) const { return r < valid ? (idx ? __ldg(idx + r) : r) : -1; }
+};
+
+// AdamW's constants and the arrays it updates at flat parameter index i
+struct Adam {
+    float* param;
+    float* m;
+    float* v;
+    float lr, b1, b2, eps, c1, c2, wd;
+    __device__ __forceinline__ float step(float g, float& mi, float& vi, float w) const {
+        mi = b1 * mi + (1.f - b1) * g;
+        vi = b2 * vi + (1.f - b2) * g * g;
+        return w - lr * (mi / c1) / (sqrtf(vi / c2) + eps) - lr * wd * w;
+    }
+    __device__ __forceinline__ float update(int64_t i, float g) const {       // the new parameter
+        float mi = m[i], vi = v[i];
+        float const w = step(g, mi, vi, param[i]);
+        m[i] = mi;
+        v[i] = vi;
+        param[i] = w;
+        return w;
+    }
+};
+
 // C[split][M][N] (FP32) = sum over this split's K of A(m, k) B(n, k), where
-//   A(m, k) = A_MN ? a[k' * lda + m] : a[m' * lda + k]   (BF16; ' = through a_idx when given,
-//   B(n, k) = B_MN ? b[k' * ldb + n] : b[n' * ldb + k]    a negative index reads zeros)
-// M, N multiples of 128; K and k_split multiples of 64. Grid (M/128, N/128, splits).
+//   A(m, k) = A_MN ? a[k * lda + m] : a[m' * lda + k]   (BF16; ' = through the row map when
+//   B(n, k) = B_MN ? b[k' * ldb + n] : b[n * ldb + k]    MAPPED)
+// M a multiple of 128, N and K of 64, k_split of 64.
+enum Epilogue { EPI_STORE = 0, EPI_MASK = 1, EPI_ADAM = 2 };
 struct GemmArgs {
     __nv_bfloat16 const* a;
     int64_t lda;
-    int32_t const* a_idx;
     __nv_bfloat16 const* b;
     int64_t ldb;
-    int32_t const* b_idx;
+    RowMap map;
     float* c;
     int64_t ldc;
     int64_t c_split;       // floats between consecutive splits' outputs
     int m, n, k, k_split;
     uint32_t* status;      // bit 0: a tensor-core wait timed out
+    __nv_bfloat16 const* mask;   // EPI_MASK: out16 = BF16(mask > 0 ? C : 0), both [M][ldc]
+    __nv_bfloat16* out16;        // EPI_MASK; EPI_ADAM: the BF16 copy of the updated weights [M][ldc]
+    int mapped;                  // the row map applies (to A's rows, or to B's with B_MN)
 };
 
-// one operand stage (128 rows of M/N x 64 of K) from global memory into its core-matrix layout
-template <int MN>
-__device__ __forceinline__ void stage_operand(uint8_t* dst, __nv_bfloat16 const* src, int64_t ld,
-                                              int32_t const* idx, int r0, int k0, int tid) {
+__device__ __forceinline__ void cp_async16(uint32_t dst, void const* src, bool valid) {   // zeros when not valid
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// one operand stage (EXT of M/N x 64 of K) from global memory into its swizzled rows, 16 bytes a copy
+template <int MN, int EXT>
+__device__ __forceinline__ void stage_operand(uint32_t dst, __nv_bfloat16 const* src, int64_t ld, int32_t const* rows,
+                                              RowMap const& map, bool mapped, int r0, int k0, int kbase, int tid) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        int const c = tid + THREADS * q;               // 1,024 16-byte chunks
-        int outer, inner;
+    for (int q = 0; q < EXT * 8 / THREADS; ++q) {
+        int const c = tid + THREADS * q, j = c & 7;    // EXT * 8 chunks, eight to a row
+        int outer, inner, row;
         uint32_t off;
-        if (MN) {                                      // global rows = K, 16 chunks of 8 along M/N
-            int const kr = c >> 4, j = c & 15;
-            outer = k0 + kr;
-            inner = r0 + 8 * j;
-            off = uint32_t((kr >> 3) * 2048 + j * 128 + (kr & 7) * 16);
-        } else {                                       // global rows = M/N, 8 chunks of 8 along K
-            int const r = c >> 3, j = c & 7;
-            outer = r0 + r;
+        if (MN) {                                      // global rows = K, EXT / 64 tile rows each
+            int const blk = EXT == 64 ? 0 : (c >> 3) & 1;
+            row = EXT == 64 ? c >> 3 : c >> 4;
+            outer = k0 + row;
+            if (mapped) outer = outer - kbase < MAP_ROWS ? rows[outer - kbase] : map.at(outer);
+            inner = r0 + 64 * blk + 8 * j;
+            off = uint32_t(blk * 8192);
+        } else {                                       // global rows = M/N, one tile row each
+            row = c >> 3;
+            outer = mapped ? rows[row] : r0 + row;
             inner = k0 + 8 * j;
-            off = uint32_t((r >> 3) * 1024 + j * 128 + (r & 7) * 16);
+            off = 0;
         }
-        if (idx) outer = idx[outer];
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (outer >= 0) v = __ldg(reinterpret_cast<uint4 const*>(src + outer * ld + inner));
-        *reinterpret_cast<uint4*>(dst + off) = v;
+        cp_async16(dst + off + uint32_t(row * 128 + ((j ^ (row & 7)) * 16)), src + (outer >= 0 ? outer : 0) * ld + inner,
+                   outer >= 0);
     }
 }
 
-template <int A_MN, int B_MN>
-__global__ void __launch_bounds__(THREADS, 1) gemm_kernel(GemmArgs g) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+// one 128 x 64 output tile, for all threads of a CTA. What bounds it at these sizes (K of 256 to 320 per
+// tile) is latency: every stage of a minibatch's K is in flight at once, one thread issues the MMAs as the
+// stages land. A 128 x 64 x 256 tile takes 5,000 cycles from its first copy to its last store (15,000 with
+// unswizzled operands and each thread storing its own row).
+template <int A_MN, int B_MN, int EPI>
+__device__ __forceinline__ void gemm_tile(GemmArgs const& g, Adam const& ad, int tile_m, int tile_n, int split,
+                                          uint8_t* sm, int tid) {
     uint32_t const sbase = uint32_t(__cvta_generic_to_shared(sm));
-    int const tid = threadIdx.x, warp = tid >> 5;
-    int const m0 = blockIdx.x * TILE, n0 = blockIdx.y * TILE;
-    int const kb = blockIdx.z * g.k_split;
+    int const warp = tid >> 5, lane = tid & 31;
+    int const m0 = tile_m * TILE, n0 = tile_n * TN;
+    int const kb = split * g.k_split;
     int const ke = min(g.k, kb + g.k_split);
     int const nk = (ke - kb) / KS;
     uint32_t const bar0 = sbase + S_BAR;                // stage b's barrier: bar0 + 8 b
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + S_TMEM);
     volatile uint32_t* abort_s = reinterpret_cast<volatile uint32_t*>(sm + S_TMEM + 4);
+    int32_t* const rows = reinterpret_cast<int32_t*>(sm + S_ROWS);
     if (tid == 0) {
-        mbar_init(bar0);
-        mbar_init(bar0 + 8);
+        for (int b = 0; b < STAGES; ++b) mbar_init(bar0 + 8 * b);
         *abort_s = 0u;
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + S_TMEM),
-                     "r"(uint32_t(TILE)) : "memory");
+                     "r"(uint32_t(TN)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    pdl_wait();
+    pdl_go();
+    if (g.mapped) {                                     // A's 128 rows, or (B_MN) the first MAP_ROWS of this split's K
+        int const first = B_MN ? kb : m0, count = B_MN ? min(ke - kb, MAP_ROWS) : TILE;
+        for (int r = tid; r < count; r += THREADS) rows[r] = g.map.at(first + r);
     }
     fence_before();
     __syncthreads();
     fence_after();
     uint32_t const tmem = *tmem_slot;
     uint32_t const idesc = instr_desc(A_MN, B_MN);
+    auto load = [&](int it) {
+        uint32_t const as = sbase + uint32_t(it % STAGES) * STAGE_BYTES;
+        int const k0 = kb + it * KS;
+        stage_operand<A_MN, TILE>(as, g.a, g.lda, rows, g.map, g.mapped && !B_MN, m0, k0, kb, tid);
+        stage_operand<B_MN, TN>(as + A_BYTES, g.b, g.ldb, rows, g.map, g.mapped && B_MN, n0, k0, kb, tid);
+    };
+    for (int it = 0; it < STAGES - 1; ++it) {
+        if (it < nk) load(it);
+        cp_async_commit();
+    }
     for (int it = 0; it < nk; ++it) {
-        int const buf = it & 1;
-        // the stage's buffers are free once the MMAs of two iterations ago completed
-        if (tid == 0 && it >= 2 && !mbar_wait(bar0 + 8 * buf, uint32_t((it - 2) >> 1) & 1u)) {
+        // the buffer loaded below is free once the MMAs of the iteration before completed
+        if (tid == 0 && it >= 1 && it + STAGES - 1 < nk &&
+            !mbar_wait(bar0 + 8 * ((it - 1) % STAGES), uint32_t((it - 1) / STAGES) & 1u)) {
             *abort_s = 1u;
             atomicOr(g.status, 1u);
         }
+        cp_async_wait<STAGES - 2>();                    // this thread's share of stage `it` has landed
+        fence_async_smem();
         __syncthreads();
         if (*abort_s) break;
-        uint8_t* const as = sm + buf * 2 * OP_BYTES;
-        uint8_t* const bs = as + OP_BYTES;
-        int const k0 = kb + it * KS;
-        stage_operand<A_MN>(as, g.a, g.lda, g.a_idx, m0, k0, tid);
-        stage_operand<B_MN>(bs, g.b, g.ldb, g.b_idx, n0, k0, tid);
-        fence_async_smem();
-        fence_before();
-        __syncthreads();
-        fence_after();
         if (tid == 0) {
-            uint32_t const a_s = sbase + buf * 2 * OP_BYTES, b_s = a_s + OP_BYTES;
+            fence_after();
+            uint32_t const a_s = sbase + uint32_t(it % STAGES) * STAGE_BYTES, b_s = a_s + A_BYTES;
 #pragma unroll
             for (int kk = 0; kk < KS / 16; ++kk) {
-                uint64_t const ad = A_MN ? smem_desc(a_s + kk * 4096, 2048, 128) : smem_desc(a_s + kk * 256, 128, 1024);
-                uint64_t const bd = B_MN ? smem_desc(b_s + kk * 4096, 2048, 128) : smem_desc(b_s + kk * 256, 128, 1024);
-                mma_bf16(tmem, ad, bd, idesc, (it > 0 || kk > 0) ? 1u : 0u);
+                uint64_t const da = smem_desc(a_s + kk * (A_MN ? 2048 : 32), A_MN ? 8192 : 16, 1024);
+                uint64_t const db = smem_desc(b_s + kk * (B_MN ? 2048 : 32), B_MN ? 8192 : 16, 1024);
+                mma_bf16(tmem, da, db, idesc, (it > 0 || kk > 0) ? 1u : 0u);
             }
-            mma_commit(bar0 + 8 * buf);
+            mma_commit(bar0 + 8 * (it % STAGES));
         }
+        if (it + STAGES - 1 < nk) load(it + STAGES - 1);
+        cp_async_commit();
     }
+    cp_async_wait<0>();
     // the last commit completes after every MMA of this CTA
-    if (tid == 0 && !*abort_s && nk > 0 && !mbar_wait(bar0 + 8 * ((nk - 1) & 1), uint32_t((nk - 1) >> 1) & 1u)) {
+    if (tid == 0 && !*abort_s && nk > 0 && !mbar_wait(bar0 + 8 * ((nk - 1) % STAGES), uint32_t((nk - 1) / STAGES) & 1u)) {
         *abort_s = 1u;
         atomicOr(g.status, 1u);
     }
     __syncthreads();
     fence_after();
     if (!*abort_s) {
-        // TMEM lane t = output row m0 + t
-        float* const crow = g.c + int64_t(blockIdx.z) * g.c_split + int64_t(m0 + tid) * g.ldc + n0;
-        uint32_t const lane_base = tmem + (uint32_t(warp * 32) << 16);
-        for (int cc = 0; cc < TILE / 16; ++cc) {
-            float v[16];
-            if (nk > 0) tmem_ld16(lane_base + cc * 16, v);
-            else
+        // TMEM lane = output row; each group of four warps takes 16 of the tile's columns
+        static_assert(TN == 16 * (THREADS / 128), "four warps per 16 columns");
+        int const r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 16;
+        uint32_t const lane_base = tmem + (uint32_t((warp & 3) * 32) << 16);
+        float v[16];
+        if (nk > 0) {
+            tmem_ld16(lane_base + c0, v);
+        } else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = 0.f;
+            for (int j = 0; j < 16; ++j) v[j] = 0.f;
+        }
+        // through shared memory (the stages are free), so that 16 threads move a row's 256 contiguous bytes
+        float* const t = reinterpret_cast<float*>(sm);
 #pragma unroll
-            for (int j = 0; j < 16; j += 4)
-                *reinterpret_cast<float4*>(crow + cc * 16 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        for (int j = 0; j < 16; j += 4)
+            *reinterpret_cast<float4*>(t + r * LDT + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        __syncthreads();
+        int const cc = (tid & 15) * 4;
+        float* const crow = EPI == EPI_STORE ? g.c + int64_t(split) * g.c_split : nullptr;
+#pragma unroll 2
+        for (int rr = tid >> 4; rr < TILE; rr += THREADS / 16) {
+            int64_t const at = int64_t(m0 + rr) * g.ldc + n0 + cc;
+            float4 x = *reinterpret_cast<float4 const*>(t + rr * LDT + cc);
+            if (EPI == EPI_STORE) {
+                *reinterpret_cast<float4*>(crow + at) = x;
+            } else {
+                if (EPI == EPI_MASK) {
+                    uint2 const h = *reinterpret_cast<uint2 const*>(g.mask + at);
+                    x.x = __uint_as_float(h.x << 16) > 0.f ? x.x : 0.f;
+                    x.y = __uint_as_float(h.x & 0xFFFF0000u) > 0.f ? x.y : 0.f;
+                    x.z = __uint_as_float(h.y << 16) > 0.f ? x.z : 0.f;
+                    x.w = __uint_as_float(h.y & 0xFFFF0000u) > 0.f ? x.w : 0.f;
+                } else {                                          // AdamW with the gradient x
+                    float4 mi = *reinterpret_cast<float4 const*>(ad.m + at), vi = *reinterpret_cast<float4 const*>(ad.v + at);
+                    float4 const w = *reinterpret_cast<float4 const*>(ad.param + at);
+                    x.x = ad.step(x.x, mi.x, vi.x, w.x);
+                    x.y = ad.step(x.y, mi.y, vi.y, w.y);
+                    x.z = ad.step(x.z, mi.z, vi.z, w.z);
+                    x.w = ad.step(x.w, mi.w, vi.w, w.w);
+                    *reinterpret_cast<float4*>(ad.m + at) = mi;
+                    *reinterpret_cast<float4*>(ad.v + at) = vi;
+                    *reinterpret_cast<float4*>(ad.param + at) = x;
+                }
+                __nv_bfloat162 const lo = __floats2bfloat162_rn(x.x, x.y), hi = __floats2bfloat162_rn(x.z, x.w);
+                *reinterpret_cast<uint2*>(g.out16 + at) = make_uint2(*reinterpret_cast<uint32_t const*>(&lo),
+                                                                     *reinterpret_cast<uint32_t const*>(&hi));
+            }
         }
     }
     fence_before();
     __syncthreads();
     fence_after();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(TILE)) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(TN)) : "memory");
+}
+
+__device__ __forceinline__ uint8_t* aligned_smem() {
+    extern __shared__ uint8_t smem_raw[];
+    return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+}
+
+// one product: grid (M/128, N/64, splits)
+template <int A_MN, int B_MN>
+__global__ void __launch_bounds__(THREADS, 2) gemm_kernel(GemmArgs g) {
+    gemm_tile<A_MN, B_MN, EPI_STORE>(g, Adam{}, blockIdx.x, blockIdx.y, blockIdx.z, aligned_smem(), threadIdx.x);
+}
+
+// two independent products of the backward pass in one launch (neither fills the chip): dW2 = dH2^T H1 on
+// the first tiles, dH1 = BF16((H1 > 0) * dH2 W2) on the others
+__global__ void __launch_bounds__(THREADS, 2) backward_kernel(GemmArgs dw2, GemmArgs dh1) {
+    int const tiles2 = (dw2.m / TILE) * (dw2.n / TN);
+    int const b = int(blockIdx.x);
+    if (b < tiles2)
+        gemm_tile<1, 1, EPI_STORE>(dw2, Adam{}, b % (dw2.m / TILE), b / (dw2.m / TILE), 0, aligned_smem(), threadIdx.x);
+    else
+        gemm_tile<0, 1, EPI_MASK>(dh1, Adam{}, (b - tiles2) % (dh1.m / TILE), (b - tiles2) / (dh1.m / TILE), 0,
+                                  aligned_smem(), threadIdx.x);
 }
 
 using GemmFn = void (*)(GemmArgs);
@@ -254,136 +383,251 @@ inline Dims make_dims(int in, int h) {
     return d;
 }
 
-// the pass's row map: out[r] = idx[r] (or r without idx) for r < valid, -1 (a zero row) after
-__global__ void rowmap_kernel(int32_t const* __restrict__ idx, int valid, int rows, int32_t* __restrict__ out) {
-    int const r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < rows) out[r] = r < valid ? (idx ? idx[r] : r) : -1;
-}
-
-// standardised FP32 rows [rows][in] -> BF16 [rows][inp] (padding columns zero)
-__global__ void pack_kernel(float const* __restrict__ x, int rows, int in, int inp, float const* __restrict__ mean,
+// standardised FP32 rows [rows][in] -> BF16 [rows][inp] (padding columns zero), 4 columns per thread;
+// grid (inp / 4 / 128 rounded up, rows)
+__global__ void pack_kernel(float const* __restrict__ x, int in, int inp, float const* __restrict__ mean,
                             float const* __restrict__ inv_std, __nv_bfloat16* __restrict__ xb) {
-    int64_t const i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= int64_t(rows) * inp) return;
-    int64_t const r = i / inp;
-    int const c = int(i % inp);
-    float const v = c < in ? (x[r * in + c] - mean[c]) * inv_std[c] : 0.f;
-    xb[i] = __float2bfloat16_rn(v);
+    int const c0 = 4 * int(blockIdx.x * blockDim.x + threadIdx.x);
+    if (c0 >= inp) return;
+    int64_t const r = blockIdx.y + int64_t(blockIdx.z) * gridDim.y;
+    __nv_bfloat16 o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        int const c = c0 + j;
+        o[j] = __float2bfloat16_rn(c < in ? (x[r * in + c] - mean[c]) * inv_std[c] : 0.f);
+    }
+    *reinterpret_cast<uint2*>(xb + r * inp + c0) = *reinterpret_cast<uint2 const*>(o);
 }
 
-// H1 = BF16(relu(sum of the split partials + b1)), [rows][h]
-__global__ void act1_kernel(float const* __restrict__ part, int splits, int64_t split_stride, int rows, int h,
-                            float const* __restrict__ b1, __nv_bfloat16* __restrict__ h1b) {
-    int64_t const i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= int64_t(rows) * h) return;
-    float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += part[k * split_stride + i];
-    s += b1[i % h];
-    h1b[i] = __float2bfloat16_rn(s > 0.f ? s : 0.f);
+// H1 = BF16(relu(sum of the split partials + b1)), [rows][h], 4 values per thread (h a multiple of 128);
+// the partials' loads are independent, their sum runs in split order
+// (no __restrict__ on what the launches before wrote: non-coherent loads do not wait for them)
+__global__ void act1_kernel(float const* part, int splits, int64_t split_stride, int64_t n, int h, float const* b1,
+                            __nv_bfloat16* h1b) {
+    int64_t const i = 4 * (int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
+    pdl_wait();
+    pdl_go();
+    if (i >= n) return;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int k = 0; k < splits; ++k) {
+        float4 const p = __ldcg(reinterpret_cast<float4 const*>(part + k * split_stride + i));
+        s.x += p.x;
+        s.y += p.y;
+        s.z += p.z;
+        s.w += p.w;
+    }
+    float4 const b = *reinterpret_cast<float4 const*>(b1 + i % h);
+    s.x += b.x;
+    s.y += b.y;
+    s.z += b.z;
+    s.w += b.w;
+    __nv_bfloat162 const lo = __floats2bfloat162_rn(s.x > 0.f ? s.x : 0.f, s.y > 0.f ? s.y : 0.f),
+                         hi = __floats2bfloat162_rn(s.z > 0.f ? s.z : 0.f, s.w > 0.f ? s.w : 0.f);
+    *reinterpret_cast<uint2*>(h1b + i) = make_uint2(*reinterpret_cast<uint32_t const*>(&lo),
+                                                    *reinterpret_cast<uint32_t const*>(&hi));
 }
 
-// Output layer, loss and the first backward step, one thread per row:
+// Output layer, loss and the first backward step, 32 rows per block:
 //   z2 = F2 + b2, h2 = relu(z2), (mu, s) = W3 h2 + b3 (FP32, ascending);
 //   training rows (y given, row valid): NLL 0.5 (s' + (y - mu)^2 e^-s'), s' = clamp(s, +-12),
 //   dmu, ds of the batch mean, dH2 = BF16((z2 > 0) (dmu W3[0] + ds W3[1])).
-__global__ void head_kernel(float const* __restrict__ f2, int rows, int valid_rows, int h,
-                            float const* __restrict__ p, int64_t off_w3, int64_t off_b2, int64_t off_b3,
-                            float const* __restrict__ y, int32_t const* __restrict__ idx, float inv_n,
-                            float* __restrict__ out, float* __restrict__ h2f, float* __restrict__ gcols,
-                            float* __restrict__ row_loss, __nv_bfloat16* __restrict__ dh2b) {
-    int const r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    float const* z = f2 + int64_t(r) * h;
-    float const* w3 = p + off_w3;
-    float const* b2 = p + off_b2;
-    float o0 = p[off_b3], o1 = p[off_b3 + 1];
-    for (int o = 0; o < h; ++o) {
-        float const v = z[o] + b2[o];
-        float const hv = v > 0.f ? v : 0.f;
-        o0 = fmaf(hv, w3[o], o0);
-        o1 = fmaf(hv, w3[h + o], o1);
-        if (h2f) h2f[int64_t(r) * h + o] = hv;
+// The two sums are one chain of h multiply-adds per row, so a lane owns a row (warp 0 the mean, warp 1 the
+// log-variance) and reads it from shared memory; all threads move the rows in and out in whole lines. With
+// one thread per row straight from global memory the kernel took 118 us for any number of rows.
+constexpr int HEAD_ROWS = 32, HEAD_THREADS = 256;
+inline size_t head_smem(int h) { return size_t(HEAD_ROWS * (h + 1) + 2 * h + 4 * HEAD_ROWS) * 4; }
+__global__ void __launch_bounds__(HEAD_THREADS)
+    head_kernel(float const* f2, int h, float const* p, int64_t off_w3, int64_t off_b2, int64_t off_b3,
+                float const* y, RowMap map, float inv_n, float* out, float* h2f, float* gcols, float* row_loss,
+                __nv_bfloat16* dh2b) {
+    extern __shared__ uint8_t smem_raw[];
+    float* const z = reinterpret_cast<float*>(smem_raw);       // [32][h + 1]
+    float* const w3 = z + HEAD_ROWS * (h + 1);                 // [2][h]
+    float* const o = w3 + 2 * h;                               // [2][32] outputs
+    float* const gd = o + 2 * HEAD_ROWS;                       // [2][32] dmu, ds
+    int const tid = threadIdx.x, r0 = int(blockIdx.x) * HEAD_ROWS;
+    pdl_wait();
+    pdl_go();
+    for (int i = tid; i < h; i += HEAD_THREADS) {
+        w3[i] = p[off_w3 + i];
+        w3[h + i] = p[off_w3 + h + i];
     }
-    if (out) {
-        out[2 * r] = o0;
-        out[2 * r + 1] = o1;
+    // a warp moves whole rows (rows is a multiple of 128, h of 128): 16 bytes a lane, four rows in flight
+    int const warp = tid >> 5, lane = tid & 31;
+    for (int c = 4 * lane; c < h; c += 128) {
+        float const* const bp = p + off_b2 + c;                 // (the offset is even only)
+        float const b[4] = {bp[0], bp[1], bp[2], bp[3]};
+        float4 q[HEAD_ROWS / 8];
+#pragma unroll
+        for (int k = 0; k < HEAD_ROWS / 8; ++k)
+            q[k] = __ldcg(reinterpret_cast<float4 const*>(f2 + int64_t(r0 + warp + 8 * k) * h + c));
+#pragma unroll
+        for (int k = 0; k < HEAD_ROWS / 8; ++k) {
+            int const r = warp + 8 * k;
+            float const v[4] = {q[k].x + b[0], q[k].y + b[1], q[k].z + b[2], q[k].w + b[3]};
+            float* const zr = z + r * (h + 1) + c;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) zr[j] = v[j];
+            if (h2f)
+                *reinterpret_cast<float4*>(h2f + int64_t(r0 + r) * h + c) =
+                    make_float4(v[0] > 0.f ? v[0] : 0.f, v[1] > 0.f ? v[1] : 0.f, v[2] > 0.f ? v[2] : 0.f, v[3] > 0.f ? v[3] : 0.f);
+        }
+    }
+    __syncthreads();
+    if (tid < 2 * HEAD_ROWS) {
+        int const r = tid & (HEAD_ROWS - 1), which = tid / HEAD_ROWS;
+        float const* const w = w3 + which * h;
+        float const* const zr = z + r * (h + 1);
+        float acc = p[off_b3 + which];
+#pragma unroll 8
+        for (int c = 0; c < h; ++c) acc = fmaf(zr[c] > 0.f ? zr[c] : 0.f, w[c], acc);
+        o[which * HEAD_ROWS + r] = acc;
+    }
+    __syncthreads();
+    if (tid < HEAD_ROWS) {
+        int const r = r0 + tid;
+        float const o0 = o[tid], o1 = o[HEAD_ROWS + tid];
+        if (out) {
+            out[2 * r] = o0;
+            out[2 * r + 1] = o1;
+        }
+        if (y) {
+            int const src = map.at(r);
+            float dmu = 0.f, ds = 0.f, loss = 0.f;
+            if (src >= 0) {
+                float const s = fminf(fmaxf(o1, -12.f), 12.f);
+                float const e = expf(-s);
+                float const d = y[src] - o0;
+                loss = 0.5f * (s + d * d * e);
+                dmu = -d * e * inv_n;
+                ds = (o1 > -12.f && o1 < 12.f) ? 0.5f * (1.f - d * d * e) * inv_n : 0.f;
+            }
+            gcols[2 * r] = dmu;
+            gcols[2 * r + 1] = ds;
+            row_loss[r] = loss;
+            gd[tid] = dmu;
+            gd[HEAD_ROWS + tid] = ds;
+        }
     }
     if (!y) return;
-    int const src = r < valid_rows ? (idx ? idx[r] : r) : -1;
-    float dmu = 0.f, ds = 0.f, loss = 0.f;
-    if (src >= 0) {
-        float const s = fminf(fmaxf(o1, -12.f), 12.f);
-        float const e = expf(-s);
-        float const d = y[src] - o0;
-        loss = 0.5f * (s + d * d * e);
-        dmu = -d * e * inv_n;
-        ds = (o1 > -12.f && o1 < 12.f) ? 0.5f * (1.f - d * d * e) * inv_n : 0.f;
-    }
-    gcols[2 * r] = dmu;
-    gcols[2 * r + 1] = ds;
-    row_loss[r] = loss;
-    for (int o = 0; o < h; ++o) {
-        float const v = z[o] + b2[o];
-        dh2b[int64_t(r) * h + o] = __float2bfloat16_rn(v > 0.f ? fmaf(dmu, w3[o], ds * w3[h + o]) : 0.f);
-    }
-}
-
-// dH1 = BF16((H1 > 0) * F3), [rows][h]
-__global__ void mask1_kernel(float const* __restrict__ f3, __nv_bfloat16 const* __restrict__ h1b, int64_t n,
-                             __nv_bfloat16* __restrict__ dh1b) {
-    int64_t const i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    dh1b[i] = __float2bfloat16_rn(__bfloat162float(h1b[i]) > 0.f ? f3[i] : 0.f);
-}
-
-// Column sums over the batch rows in order: db1, db2 (of the BF16 dH1, dH2),
-// dW3 = sum h2 [dmu, ds], db3, and the summed loss. One thread per hidden unit.
-__global__ void small_grads_kernel(int rows, int h, __nv_bfloat16 const* __restrict__ dh1b,
-                                   __nv_bfloat16 const* __restrict__ dh2b, float const* __restrict__ h2f,
-                                   float const* __restrict__ gcols, float const* __restrict__ row_loss,
-                                   float* __restrict__ grad, int64_t off_w3, int64_t off_b1, int64_t off_b2,
-                                   int64_t off_b3, float* __restrict__ loss_out) {
-    int const o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o < h) {
-        float s1 = 0.f, s2 = 0.f, w0 = 0.f, w1 = 0.f;
-        for (int r = 0; r < rows; ++r) {
-            int64_t const i = int64_t(r) * h + o;
-            s1 += __bfloat162float(dh1b[i]);
-            s2 += __bfloat162float(dh2b[i]);
-            w0 = fmaf(h2f[i], gcols[2 * r], w0);
-            w1 = fmaf(h2f[i], gcols[2 * r + 1], w1);
+    __syncthreads();
+    for (int c = 2 * lane; c < h; c += 64) {
+        float const wa = w3[c], wb = w3[c + 1], va = w3[h + c], vb = w3[h + c + 1];
+#pragma unroll
+        for (int k = 0; k < HEAD_ROWS / 8; ++k) {
+            int const r = warp + 8 * k;
+            float const dmu = gd[r], ds = gd[HEAD_ROWS + r];
+            float const* const zr = z + r * (h + 1) + c;
+            __nv_bfloat162 const v = __floats2bfloat162_rn(zr[0] > 0.f ? fmaf(dmu, wa, ds * va) : 0.f,
+                                                           zr[1] > 0.f ? fmaf(dmu, wb, ds * vb) : 0.f);
+            *reinterpret_cast<__nv_bfloat162*>(dh2b + int64_t(r0 + r) * h + c) = v;
         }
-        grad[off_b1 + o] = s1;
-        grad[off_b2 + o] = s2;
-        grad[off_w3 + o] = w0;
-        grad[off_w3 + h + o] = w1;
-    } else if (o < h + 3) {
-        int const c = o - h;        // 0, 1: db3; 2: loss
-        float s = 0.f;
-        for (int r = 0; r < rows; ++r) s += c < 2 ? gcols[2 * r + c] : row_loss[r];
-        if (c < 2) grad[off_b3 + c] = s;
-        else if (loss_out) *loss_out = s;
     }
 }
 
-// AdamW over the flat parameter vector (padding columns of W1 stay zero), then
-// the BF16 copies of W1 and W2 the GEMMs read.
-__global__ void adam_kernel(float* __restrict__ param, float* __restrict__ m, float* __restrict__ v,
-                            float const* __restrict__ grad, int64_t n, int64_t off_w2, int64_t off_w3, int in,
-                            int inp, float lr, float b1, float b2, float eps, float c1, float c2, float wd,
-                            __nv_bfloat16* __restrict__ w1b, __nv_bfloat16* __restrict__ w2b) {
-    int64_t const i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (i < off_w2 && int(i % inp) >= in) return;
-    float const g = grad[i];
-    float const mi = b1 * m[i] + (1.f - b1) * g;
-    float const vi = b2 * v[i] + (1.f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    float const w = param[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps) - lr * wd * param[i];
-    param[i] = w;
-    if (i < off_w2) w1b[i] = __float2bfloat16_rn(w);
-    else if (i < off_w3) w2b[i - off_w2] = __float2bfloat16_rn(w);
+// The column sums of the backward pass, over the batch rows in order: db1, db2 (of the BF16 dH1, dH2),
+// dW3 = sum h2 [dmu, ds], db3, and the summed loss.
+struct SmallGrads {
+    int rows, h;
+    __nv_bfloat16 const* dh1b;
+    __nv_bfloat16 const* dh2b;
+    float const* h2f;
+    float const* gcols;
+    float const* row_loss;
+    float* grad;
+    int64_t w3, b1, b2, b3;     // parameter offsets
+    float* loss;
+};
+
+// Columns [32 cb, 32 cb + 32) of the hidden units (cb = h / 32: db3 and the loss): four warps, one sum of
+// every column each; each sum is a chain over the rows, so the loads run ahead of it.
+constexpr int SG_DEEP = 16;
+template <class Load>
+__device__ __forceinline__ float ordered_sum(int rows, Load load, bool fma_form) {
+    float s = 0.f, a[SG_DEEP], b[SG_DEEP];
+#pragma unroll
+    for (int i = 0; i < SG_DEEP; ++i) load(i, a[i], b[i]);
+    for (int r0 = 0; r0 < rows; r0 += SG_DEEP) {        // rows: a multiple of 128
+        float na[SG_DEEP], nb[SG_DEEP];
+        bool const more = r0 + SG_DEEP < rows;
+#pragma unroll
+        for (int i = 0; i < SG_DEEP; ++i) {
+            na[i] = nb[i] = 0.f;
+            if (more) load(r0 + SG_DEEP + i, na[i], nb[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < SG_DEEP; ++i) s = fma_form ? fmaf(a[i], b[i], s) : s + a[i];
+#pragma unroll
+        for (int i = 0; i < SG_DEEP; ++i) {
+            a[i] = na[i];
+            b[i] = nb[i];
+        }
+    }
+    return s;
+}
+
+// the launch's other work beside the dW1 tiles (update: AdamW on what it computes, else into g.grad)
+__device__ __forceinline__ void small_grads(SmallGrads const& g, Adam const& ad, bool update, int cb, int tid) {
+    int const warp = tid >> 5, lane = tid & 31;
+    if (warp >= 4) return;
+    int64_t at = -1;
+    float s = 0.f;
+    if (cb < g.h / 32) {
+        int const o = cb * 32 + lane;
+        int64_t const h = g.h;
+        if (warp < 2) {
+            __nv_bfloat16 const* const src = warp == 0 ? g.dh1b : g.dh2b;
+            at = (warp == 0 ? g.b1 : g.b2) + o;
+            s = ordered_sum(g.rows, [&](int r, float& a, float&) { a = __bfloat162float(src[r * h + o]); }, false);
+        } else {
+            int const c = warp - 2;
+            at = g.w3 + c * h + o;
+            s = ordered_sum(g.rows, [&](int r, float& a, float& b) {
+                a = g.h2f[r * h + o];
+                b = g.gcols[2 * r + c];
+            }, true);
+        }
+    } else if (warp == 0 && lane < 3) {
+        if (lane < 2) at = g.b3 + lane;
+        s = ordered_sum(g.rows, [&](int r, float& a, float&) { a = lane < 2 ? g.gcols[2 * r + lane] : g.row_loss[r]; }, false);
+        if (lane == 2) *g.loss = s;
+    }
+    if (at < 0) return;
+    if (update) ad.update(at, s);
+    else g.grad[at] = s;
+}
+
+// AdamW on W2 (its gradient complete since the launch before) and W2's BF16 copy
+constexpr int W2_PER_BLOCK = 4 * THREADS;
+__device__ __forceinline__ void update_w2(Adam const& ad, float const* grad, int64_t off, int64_t n, __nv_bfloat16* w2b,
+                                          int block, int tid) {
+#pragma unroll
+    for (int q = 0; q < W2_PER_BLOCK / THREADS; ++q) {
+        int64_t const i = int64_t(block) * W2_PER_BLOCK + q * THREADS + tid;
+        if (i < n) w2b[i] = __float2bfloat16_rn(ad.update(off + i, grad[off + i]));
+    }
+}
+
+// The last launch of a step: the small gradients first (their chains are the longest), then W2's update,
+// then dW1 = dH1^T X (M = h, N = inp, K = rows) tile by tile. UPDATE: each tile's AdamW runs in its
+// epilogue, so W1's gradient is never written (and the separate pass over 1.3 M parameters is gone);
+// otherwise the gradients are stored.
+template <bool UPDATE>
+__global__ void __launch_bounds__(THREADS, 2) last_kernel(GemmArgs dw1, SmallGrads sg, Adam ad, int64_t off_w2, __nv_bfloat16* w2b) {
+    int const b = int(blockIdx.x), nsmall = sg.h / 32 + 1;
+    int64_t const n2 = int64_t(sg.h) * sg.h;
+    int const nw2 = UPDATE ? int((n2 + W2_PER_BLOCK - 1) / W2_PER_BLOCK) : 0;
+    if (b < nsmall + nw2) {
+        pdl_wait();
+        pdl_go();
+        if (b < nsmall) small_grads(sg, ad, UPDATE, b, threadIdx.x);
+        else update_w2(ad, sg.grad, off_w2, n2, w2b, b - nsmall, threadIdx.x);
+        return;
+    }
+    int const t = b - nsmall - nw2;
+    gemm_tile<1, 1, UPDATE ? EPI_ADAM : EPI_STORE>(dw1, ad, t % (dw1.m / TILE), t / (dw1.m / TILE), 0, aligned_smem(),
+                                                   threadIdx.x);
 }
 
 __global__ void refresh_kernel(float const* __restrict__ param, int64_t off_w2, int64_t off_w3,
@@ -412,7 +656,6 @@ struct ta3w_model {
     uint32_t* d_status = nullptr;
     float* d_loss = nullptr;
     float* d_stats = nullptr;          // mean [inp], inv_std [inp]
-    std::vector<float> x_mean, x_inv_std;
     float y_mean = 0.f, y_std = 1.f;
     // data
     uint32_t rows = 0;
@@ -427,14 +670,13 @@ struct ta3w_model {
     int max_splits = 1;
     float* d_f1 = nullptr;             // [splits][rows][h]
     __nv_bfloat16* d_h1b = nullptr;
-    float* d_f2 = nullptr;             // F2, then F3
+    float* d_f2 = nullptr;
     float* d_h2f = nullptr;
     float* d_gcols = nullptr;
     float* d_rowloss = nullptr;
     __nv_bfloat16* d_dh2b = nullptr;
     __nv_bfloat16* d_dh1b = nullptr;
     float* d_out = nullptr;
-    int32_t* d_rowidx = nullptr;       // identity / padded row map of a full pass
     uint64_t adam_t = 0;
 };
 
@@ -479,31 +721,36 @@ int ensure_act(ta3w_model* m, size_t rows) {
     int const h = m->d.h;
     int const splits = m->max_splits;
     for (void* p : {(void*)m->d_f1, (void*)m->d_h1b, (void*)m->d_f2, (void*)m->d_h2f, (void*)m->d_gcols,
-                    (void*)m->d_rowloss, (void*)m->d_dh2b, (void*)m->d_dh1b, (void*)m->d_out, (void*)m->d_rowidx})
+                    (void*)m->d_rowloss, (void*)m->d_dh2b, (void*)m->d_dh1b, (void*)m->d_out})
         if (p) cudaFree(p);
     m->d_f1 = m->d_f2 = m->d_h2f = m->d_gcols = m->d_rowloss = m->d_out = nullptr;
     m->d_h1b = m->d_dh2b = m->d_dh1b = nullptr;
-    m->d_rowidx = nullptr;
     m->cap_act = 0;
     if (walloc(m, m->d_f1, size_t(splits) * rows * h, "alloc F1") || walloc(m, m->d_h1b, rows * h, "alloc H1") ||
         walloc(m, m->d_f2, rows * h, "alloc F2") || walloc(m, m->d_h2f, rows * h, "alloc H2") ||
         walloc(m, m->d_gcols, rows * 2, "alloc G") || walloc(m, m->d_rowloss, rows, "alloc loss rows") ||
         walloc(m, m->d_dh2b, rows * h, "alloc dH2") || walloc(m, m->d_dh1b, rows * h, "alloc dH1") ||
-        walloc(m, m->d_out, rows * 2, "alloc outputs") || walloc(m, m->d_rowidx, rows, "alloc row map"))
+        walloc(m, m->d_out, rows * 2, "alloc outputs"))
         return 1;
     m->cap_act = rows;
     return 0;
 }
 
-int gemm(ta3w_model* m, int a_mn, int b_mn, __nv_bfloat16 const* a, int64_t lda, int32_t const* a_idx,
-         __nv_bfloat16 const* b, int64_t ldb, int32_t const* b_idx, float* c, int64_t ldc, int64_t c_split, int M,
-         int N, int K, int splits) {
-    int const kst = K / KS;
-    int const per = (kst + splits - 1) / splits;
-    splits = (kst + per - 1) / per;
-    GemmArgs g{a, lda, a_idx, b, ldb, b_idx, c, ldc, c_split, M, N, K, per * KS, m->d_status};
-    gemm_fn(a_mn, b_mn)<<<dim3(M / TILE, N / TILE, splits), THREADS, SMEM_BYTES, m->stream>>>(g);
-    TA3W_CUDA(m, cudaGetLastError(), "gemm launch");
+// a launch that may start while the one before it on the stream drains (each kernel waits with pdl_wait
+// before it touches what another launch wrote)
+template <class... Args>
+int launch(ta3w_model* m, char const* what, void (*fn)(Args...), dim3 grid, int threads, size_t smem, Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = m->stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    TA3W_CUDA(m, cudaLaunchKernelEx(&cfg, fn, args...), what);
     return 0;
 }
 
@@ -513,46 +760,66 @@ int splits_for(ta3w_model* m, int M, int N, int K) {
     return std::min({want, K / KS, m->max_splits});
 }
 
-// forward (and with y, the backward pass into d_grad) over `rows` rows of d_x
-// selected by idx (device, `rows` entries, -1 = none; rows padded to 128 here)
-int pass(ta3w_model* m, int32_t const* idx, int valid_rows, bool train) {
+// forward (and with train the backward pass) over `valid_rows` rows of x [..][inp] BF16, selected by idx
+// (device, -1 = none; null: rows 0 .. valid_rows - 1), padded to a multiple of 128 here. ad: the step's
+// AdamW, applied as the gradients come; without it they go to d_grad.
+int pass(ta3w_model* m, __nv_bfloat16 const* x, int32_t const* idx, int valid_rows, bool train, Adam const* ad = nullptr) {
     Dims const& d = m->d;
     int const R = round128(valid_rows);
     if (ensure_act(m, size_t(R))) return 1;
     int const h = d.h;
-    rowmap_kernel<<<unsigned((R + 255) / 256), 256, 0, m->stream>>>(idx, valid_rows, R, m->d_rowidx);
-    TA3W_CUDA(m, cudaGetLastError(), "row map");
-    int32_t const* rows = m->d_rowidx;
+    RowMap const rows{idx, valid_rows};
     // layer 1: F1 = X W1^T (M = rows, N = h, K = inp), split over K
     int const s1 = splits_for(m, R, h, d.inp);
-    int64_t const f1_stride = int64_t(R) * h;
-    if (gemm(m, 0, 0, m->d_x, d.inp, rows, m->d_w1b, d.inp, nullptr, m->d_f1, h, f1_stride, R, h, d.inp, s1)) return 1;
     int const per = (d.inp / KS + s1 - 1) / s1;
     int const s1_used = (d.inp / KS + per - 1) / per;
     int64_t const n_act = int64_t(R) * h;
-    act1_kernel<<<unsigned((n_act + 255) / 256), 256, 0, m->stream>>>(m->d_f1, s1_used, f1_stride, R, h,
-                                                                      m->d_param + d.b1, m->d_h1b);
-    TA3W_CUDA(m, cudaGetLastError(), "act1");
+    GemmArgs f1{};
+    f1.a = x, f1.lda = d.inp, f1.map = rows, f1.mapped = 1;
+    f1.b = m->d_w1b, f1.ldb = d.inp;
+    f1.c = m->d_f1, f1.ldc = h, f1.c_split = n_act;
+    f1.m = R, f1.n = h, f1.k = d.inp, f1.k_split = per * KS, f1.status = m->d_status;
+    if (launch(m, "layer 1", gemm_kernel<0, 0>, dim3(unsigned(R / TILE), unsigned(h / TN), unsigned(s1_used)), THREADS,
+               SMEM_BYTES, f1))
+        return 1;
+    if (launch(m, "act1", act1_kernel, dim3(unsigned((n_act / 4 + 127) / 128)), 128, 0, (float const*)m->d_f1, s1_used,
+               n_act, n_act, h, (float const*)(m->d_param + d.b1), m->d_h1b))
+        return 1;
     // layer 2: F2 = H1 W2^T
-    if (gemm(m, 0, 0, m->d_h1b, h, nullptr, m->d_w2b, h, nullptr, m->d_f2, h, 0, R, h, h, 1)) return 1;
-    head_kernel<<<unsigned((R + 127) / 128), 128, 0, m->stream>>>(
-        m->d_f2, R, valid_rows, h, m->d_param, d.w3, d.b2, d.b3, train ? m->d_y : nullptr, rows,
-        1.0f / float(valid_rows), m->d_out, train ? m->d_h2f : nullptr, m->d_gcols, m->d_rowloss, m->d_dh2b);
-    TA3W_CUDA(m, cudaGetLastError(), "head");
+    GemmArgs f2{};
+    f2.a = m->d_h1b, f2.lda = h, f2.b = m->d_w2b, f2.ldb = h;
+    f2.c = m->d_f2, f2.ldc = h, f2.m = R, f2.n = h, f2.k = h, f2.k_split = h, f2.status = m->d_status;
+    if (launch(m, "layer 2", gemm_kernel<0, 0>, dim3(unsigned(R / TILE), unsigned(h / TN), 1), THREADS, SMEM_BYTES, f2))
+        return 1;
+    if (launch(m, "head", head_kernel, dim3(unsigned(R / HEAD_ROWS)), HEAD_THREADS, head_smem(h),
+               (float const*)m->d_f2, h, (float const*)m->d_param, d.w3, d.b2, d.b3,
+               (float const*)(train ? m->d_y : nullptr), rows, 1.0f / float(valid_rows), m->d_out,
+               train ? m->d_h2f : (float*)nullptr, m->d_gcols, m->d_rowloss, m->d_dh2b))
+        return 1;
     if (!train) return 0;
-    // dW2 = dH2^T H1 (M = h out, N = h in, K = rows), straight into the gradient vector
-    if (gemm(m, 1, 1, m->d_dh2b, h, nullptr, m->d_h1b, h, nullptr, m->d_grad + d.w2, h, 0, h, h, R, 1)) return 1;
-    // F3 = dH2 W2 (M = rows, N = h in, K = h out), then the ReLU mask of layer 1
-    if (gemm(m, 0, 1, m->d_dh2b, h, nullptr, m->d_w2b, h, nullptr, m->d_f2, h, 0, R, h, h, 1)) return 1;
-    mask1_kernel<<<unsigned((n_act + 255) / 256), 256, 0, m->stream>>>(m->d_f2, m->d_h1b, n_act, m->d_dh1b);
-    TA3W_CUDA(m, cudaGetLastError(), "mask1");
-    // dW1 = dH1^T X (M = h, N = inp, K = rows)
-    if (gemm(m, 1, 1, m->d_dh1b, h, nullptr, m->d_x, d.inp, rows, m->d_grad + d.w1, d.inp, 0, h, d.inp, R, 1)) return 1;
-    small_grads_kernel<<<unsigned((h + 3 + 127) / 128), 128, 0, m->stream>>>(
-        R, h, m->d_dh1b, m->d_dh2b, m->d_h2f, m->d_gcols, m->d_rowloss, m->d_grad, d.w3, d.b1, d.b2, d.b3,
-        m->d_loss);
-    TA3W_CUDA(m, cudaGetLastError(), "small grads");
-    return 0;
+    // dW2 = dH2^T H1 (M = h out, N = h in, K = rows) and dH1 = mask(dH2 W2) (M = rows, N = h in, K = h out)
+    GemmArgs dw2{}, dh1{};
+    dw2.a = m->d_dh2b, dw2.lda = h, dw2.b = m->d_h1b, dw2.ldb = h;
+    dw2.c = m->d_grad + d.w2, dw2.ldc = h, dw2.m = h, dw2.n = h, dw2.k = R, dw2.k_split = R, dw2.status = m->d_status;
+    dh1.a = m->d_dh2b, dh1.lda = h, dh1.b = m->d_w2b, dh1.ldb = h;
+    dh1.ldc = h, dh1.m = R, dh1.n = h, dh1.k = h, dh1.k_split = h, dh1.status = m->d_status;
+    dh1.mask = m->d_h1b, dh1.out16 = m->d_dh1b;
+    if (launch(m, "backward 2", backward_kernel, dim3(unsigned((h / TILE) * (h / TN) + (R / TILE) * (h / TN))), THREADS,
+               SMEM_BYTES, dw2, dh1))
+        return 1;
+    GemmArgs dw1{};
+    dw1.a = m->d_dh1b, dw1.lda = h, dw1.b = x, dw1.ldb = d.inp, dw1.map = rows, dw1.mapped = 1;
+    dw1.c = m->d_grad + d.w1, dw1.ldc = d.inp, dw1.m = h, dw1.n = d.inp, dw1.k = R, dw1.k_split = R;
+    dw1.status = m->d_status, dw1.out16 = m->d_w1b;
+    SmallGrads const sg{R, h, m->d_dh1b, m->d_dh2b, m->d_h2f, m->d_gcols, m->d_rowloss, m->d_grad,
+                        d.w3, d.b1, d.b2, d.b3, m->d_loss};
+    int const tiles = (h / TILE) * (d.inp / TN), small = h / 32 + 1;
+    int const w2_blocks = int((int64_t(h) * h + W2_PER_BLOCK - 1) / W2_PER_BLOCK);
+    if (ad)
+        return launch(m, "backward 1 and update", last_kernel<true>, dim3(unsigned(small + w2_blocks + tiles)), THREADS,
+                      SMEM_BYTES, dw1, sg, *ad, d.w2, m->d_w2b);
+    return launch(m, "backward 1", last_kernel<false>, dim3(unsigned(small + tiles)), THREADS, SMEM_BYTES, dw1, sg, Adam{},
+                  d.w2, m->d_w2b);
 }
 
 int check_status(ta3w_model* m) {
@@ -563,7 +830,9 @@ int check_status(ta3w_model* m) {
     return 0;
 }
 
-int upload_rows(ta3w_model* m, float const* x, uint32_t n) {
+// the rows on the device, standardised in BF16 (with `standardize` by their own statistics, which stay for
+// later predictions)
+int upload_rows(ta3w_model* m, float const* x, uint32_t n, bool standardize) {
     Dims const& d = m->d;
     if (n > m->cap_rows) {
         size_t c1 = 0, c2 = 0, c3 = 0;
@@ -580,10 +849,17 @@ int upload_rows(ta3w_model* m, float const* x, uint32_t n) {
         m->cap_rows = n;
     }
     TA3W_CUDA(m, cudaMemcpyAsync(m->d_xraw, x, size_t(n) * d.in * 4, cudaMemcpyHostToDevice, m->stream), "copy rows");
-    int64_t const total = int64_t(n) * d.inp;
-    pack_kernel<<<unsigned((total + 255) / 256), 256, 0, m->stream>>>(m->d_xraw, int(n), d.in, d.inp, m->d_stats,
-                                                                      m->d_stats + d.inp, m->d_x);
-    TA3W_CUDA(m, cudaGetLastError(), "pack");
+    if (standardize)
+        TA3W_CUDA(m, ta3_stats::column_stats(m->d_xraw, int(n), d.in, d.in, m->d_stats, m->d_stats + d.inp, m->stream),
+                  "column statistics");
+    uint32_t const fold = 32768, cols = unsigned((d.inp / 4 + 127) / 128);      // grid y and z hold at most 65,535
+    for (uint32_t r0 = 0; r0 < n;) {
+        uint32_t const left = n - r0, ny = std::min(left, fold), nz = std::min(left / ny, 32768u);
+        pack_kernel<<<dim3(cols, ny, nz), 128, 0, m->stream>>>(m->d_xraw + size_t(r0) * d.in, d.in, d.inp, m->d_stats,
+                                                               m->d_stats + d.inp, m->d_x + size_t(r0) * d.inp);
+        TA3W_CUDA(m, cudaGetLastError(), "pack");
+        r0 += ny * nz;
+    }
     return 0;
 }
 
@@ -615,11 +891,15 @@ ta3w_model* ta3w_create(int device, uint32_t in_dim, uint32_t hidden, uint32_t s
     if (prop.major != 10) return bad("needs an sm_100 (B200) device");
     m->sms = prop.multiProcessorCount;
     m->max_splits = 16;
+    auto smem = [](auto* fn, size_t bytes) {
+        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) == cudaSuccess;
+    };
     for (int a = 0; a < 2; ++a)
         for (int b = 0; b < 2; ++b)
-            if (cudaFuncSetAttribute(gemm_fn(a, b), cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES)) !=
-                cudaSuccess)
-                return bad("smem attribute");
+            if (!smem(gemm_fn(a, b), SMEM_BYTES)) return bad("smem attribute");
+    if (!smem(backward_kernel, SMEM_BYTES) || !smem(last_kernel<true>, SMEM_BYTES) || !smem(last_kernel<false>, SMEM_BYTES) ||
+        !smem(head_kernel, head_smem(1024)))
+        return bad("smem attribute");
     if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess) return bad("stream");
     Dims const& d = m->d;
     size_t const np = size_t(d.n);
@@ -639,8 +919,6 @@ ta3w_model* ta3w_create(int device, uint32_t in_dim, uint32_t hidden, uint32_t s
     if (ta3w_set_params(m, w.data())) return bad(m->err);
     std::vector<float> stats(2 * size_t(d.inp), 0.f);
     std::fill(stats.begin() + d.inp, stats.end(), 1.f);
-    m->x_mean.assign(size_t(d.in), 0.f);
-    m->x_inv_std.assign(size_t(d.in), 1.f);
     // on the model's stream: its kernels run on a non-blocking stream, which does not wait for the
     // legacy default stream (a pageable cudaMemcpy can even return before its DMA has landed)
     if (cudaMemcpyAsync(m->d_stats, stats.data(), stats.size() * 4, cudaMemcpyHostToDevice, m->stream) != cudaSuccess ||
@@ -657,7 +935,7 @@ void ta3w_destroy(ta3w_model* m) {
                     (void*)m->d_w2b, (void*)m->d_status, (void*)m->d_loss, (void*)m->d_stats, (void*)m->d_xraw,
                     (void*)m->d_x, (void*)m->d_y, (void*)m->d_idx, (void*)m->d_f1, (void*)m->d_h1b, (void*)m->d_f2,
                     (void*)m->d_h2f, (void*)m->d_gcols, (void*)m->d_rowloss, (void*)m->d_dh2b, (void*)m->d_dh1b,
-                    (void*)m->d_out, (void*)m->d_rowidx})
+                    (void*)m->d_out})
         if (p) cudaFree(p);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
@@ -701,33 +979,16 @@ static int set_data_impl(ta3w_model* m, const float* x, const float* y, uint32_t
     m->y_mean = 0.f;
     m->y_std = 1.f;
     if (standardize) {
-        for (int c = 0; c < d.in; ++c) {
-            double s = 0, s2 = 0;
-            for (uint32_t r = 0; r < n; ++r) s += x[size_t(r) * d.in + c];
-            double const mu = s / n;
-            for (uint32_t r = 0; r < n; ++r) {
-                double const dv = x[size_t(r) * d.in + c] - mu;
-                s2 += dv * dv;
-            }
-            double const sd = std::sqrt(s2 / n);
-            m->x_mean[c] = float(mu);
-            m->x_inv_std[c] = sd > 1e-12 ? float(1.0 / sd) : 1.f;
-            stats[c] = m->x_mean[c];
-            stats[d.inp + c] = m->x_inv_std[c];
-        }
         double s = 0, s2 = 0;
         for (uint32_t r = 0; r < n; ++r) s += y[r];
         double const mu = s / n;
         for (uint32_t r = 0; r < n; ++r) s2 += (y[r] - mu) * (y[r] - mu);
         m->y_mean = float(mu);
         m->y_std = s2 > 0 ? float(std::sqrt(s2 / n)) : 1.f;
-    } else {
-        std::fill(m->x_mean.begin(), m->x_mean.end(), 0.f);
-        std::fill(m->x_inv_std.begin(), m->x_inv_std.end(), 1.f);
     }
     TA3W_CUDA(m, cudaMemcpyAsync(m->d_stats, stats.data(), stats.size() * 4, cudaMemcpyHostToDevice, m->stream),
               "stats");
-    if (upload_rows(m, x, n)) return 1;
+    if (upload_rows(m, x, n, standardize)) return 1;
     std::vector<float> ys(n);
     for (uint32_t r = 0; r < n; ++r) ys[r] = (y[r] - m->y_mean) / m->y_std;
     TA3W_CUDA(m, cudaMemcpyAsync(m->d_y, ys.data(), size_t(n) * 4, cudaMemcpyHostToDevice, m->stream), "targets");
@@ -753,7 +1014,7 @@ int ta3w_gradients(ta3w_model* m, float* grad_out, float* loss_sum_out) {
     TA3W_CUDA(m, cudaSetDevice(m->device), "set device");
     TA3W_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
     TA3W_CUDA(m, cudaMemsetAsync(m->d_grad, 0, size_t(m->d.n) * 4, m->stream), "grad");
-    if (pass(m, nullptr, int(m->rows), true)) return 1;
+    if (pass(m, m->d_x, nullptr, int(m->rows), true)) return 1;
     if (check_status(m)) return 1;
     TA3W_CUDA(m, cudaMemcpy(grad_out, m->d_grad, size_t(m->d.n) * 4, cudaMemcpyDeviceToHost), "grad");
     if (loss_sum_out) TA3W_CUDA(m, cudaMemcpy(loss_sum_out, m->d_loss, 4, cudaMemcpyDeviceToHost), "loss");
@@ -765,7 +1026,6 @@ int ta3w_train(ta3w_model* m, uint32_t epochs, uint32_t batch, float lr, float w
     if (!m || batch == 0 || batch > kMaxPassRows) return wfail(m, "ta3w_train: batch must be 1 .. 65,536");
     if (m->rows == 0) return wfail(m, "ta3w_train: no data");
     TA3W_CUDA(m, cudaSetDevice(m->device), "set device");
-    Dims const& d = m->d;
     uint32_t const n = m->rows;
     uint32_t const steps = (n + batch - 1) / batch;
     size_t const total = size_t(epochs) * steps * batch;
@@ -790,13 +1050,10 @@ int ta3w_train(ta3w_model* m, uint32_t epochs, uint32_t batch, float lr, float w
     for (uint32_t e = 0; e < epochs; ++e)
         for (uint32_t s = 0; s < steps; ++s) {
             uint32_t const rows_here = std::min(batch, n - s * batch);
-            if (pass(m, m->d_idx + (size_t(e) * steps + s) * batch, int(rows_here), true)) return 1;
             ++m->adam_t;
             float const c1 = 1.f - std::pow(b1, float(m->adam_t)), c2 = 1.f - std::pow(b2, float(m->adam_t));
-            adam_kernel<<<unsigned((d.n + 255) / 256), 256, 0, m->stream>>>(
-                m->d_param, m->d_m, m->d_v, m->d_grad, d.n, d.w2, d.w3, d.in, d.inp, lr, b1, b2, eps, c1, c2,
-                weight_decay, m->d_w1b, m->d_w2b);
-            TA3W_CUDA(m, cudaGetLastError(), "adam");
+            Adam const ad{m->d_param, m->d_m, m->d_v, lr, b1, b2, eps, c1, c2, weight_decay};
+            if (pass(m, m->d_x, m->d_idx + (size_t(e) * steps + s) * batch, int(rows_here), true, &ad)) return 1;
             last_rows = rows_here;
         }
     if (check_status(m)) return 1;
@@ -811,22 +1068,15 @@ int ta3w_predict(ta3w_model* m, const float* x, uint32_t n, float* mean_out, flo
     if (!m || !x || !mean_out) return wfail(m, "ta3w_predict: null argument");
     if (n == 0) return 0;
     TA3W_CUDA(m, cudaSetDevice(m->device), "set device");
-    if (upload_rows(m, x, n)) return 1;
+    if (upload_rows(m, x, n, false)) return 1;
     TA3W_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
     uint32_t const chunk = 4096;
     std::vector<float> out(size_t(n) * 2);
     for (uint32_t r0 = 0; r0 < n; r0 += chunk) {
         uint32_t const k = std::min(chunk, n - r0);
-        std::vector<int32_t> map(k);
-        std::iota(map.begin(), map.end(), int32_t(r0));
-        size_t cap = m->cap_idx;
-        if (wgrow(m, m->d_idx, cap, std::max<size_t>(m->cap_idx, k), "alloc indices")) return 1;
-        m->cap_idx = cap;
-        TA3W_CUDA(m, cudaMemcpyAsync(m->d_idx, map.data(), size_t(k) * 4, cudaMemcpyHostToDevice, m->stream), "rows");
-        if (pass(m, m->d_idx, int(k), false)) return 1;
+        if (pass(m, m->d_x + size_t(r0) * m->d.inp, nullptr, int(k), false)) return 1;
         TA3W_CUDA(m, cudaMemcpyAsync(out.data() + size_t(r0) * 2, m->d_out, size_t(k) * 8, cudaMemcpyDeviceToHost,
                                      m->stream), "outputs");
-        TA3W_CUDA(m, cudaStreamSynchronize(m->stream), "predict");
     }
     if (check_status(m)) return 1;
     for (uint32_t r = 0; r < n; ++r) {
@@ -869,8 +1119,10 @@ int ta3w_gemm_test(int device, int a_mn, int b_mn, int m, int n, int k, int spli
         cudaMemcpy(da, a, size_t(m) * k * 2, cudaMemcpyHostToDevice);
         cudaMemcpy(db, b, size_t(n) * k * 2, cudaMemcpyHostToDevice);
         cudaMemset(ds, 0, 4);
-        GemmArgs g{da, a_mn ? m : k, nullptr, db, b_mn ? n : k, nullptr, dc, n, int64_t(m) * n, m, n, k, per * KS, ds};
-        gemm_fn(a_mn, b_mn)<<<dim3(m / TILE, n / TILE, used), THREADS, SMEM_BYTES>>>(g);
+        GemmArgs g{};
+        g.a = da, g.lda = a_mn ? m : k, g.b = db, g.ldb = b_mn ? n : k;
+        g.c = dc, g.ldc = n, g.c_split = int64_t(m) * n, g.m = m, g.n = n, g.k = k, g.k_split = per * KS, g.status = ds;
+        gemm_fn(a_mn, b_mn)<<<dim3(m / TILE, n / TN, used), THREADS, SMEM_BYTES>>>(g);
         cudaError_t e = cudaDeviceSynchronize();
         uint32_t st = 0;
         if (e == cudaSuccess) e = cudaMemcpy(&st, ds, 4, cudaMemcpyDeviceToHost);
