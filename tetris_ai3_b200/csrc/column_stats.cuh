@@ -15,7 +15,7 @@ constexpr int DEEP = 16;      // rows in flight per thread
 // One thread per column; a warp reads 128 contiguous bytes of a row. The adds are one chain per column,
 // so the loads run DEEP rows ahead. 2 passes over x (the second mostly from L2). The host loop it
 // replaces walked the columns with a stride of a row: 43 ms of a 71 ms retrain on 4,000 x 4,929.
-__global__ void __launch_bounds__(COLS) column_stats_kernel(float const* __restrict__ x, int rows, int cols, int64_t ld,
+static __global__ void __launch_bounds__(COLS) column_stats_kernel(float const* __restrict__ x, int rows, int cols, int64_t ld,
                                                             float* __restrict__ mean, float* __restrict__ inv_std) {
     int const c = int(blockIdx.x) * COLS + int(threadIdx.x);
     if (c >= cols) return;
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(COLS) column_stats_kernel(float const* __restr
     inv_std[c] = sd > 1e-12 ? float(__ddiv_rn(1.0, sd)) : 1.f;
 }
 
-inline cudaError_t column_stats(float const* x, int rows, int cols, int64_t ld, float* mean, float* inv_std,
+static inline cudaError_t column_stats(float const* x, int rows, int cols, int64_t ld, float* mean, float* inv_std,
                                 cudaStream_t st) {
     column_stats_kernel<<<unsigned((cols + COLS - 1) / COLS), COLS, 0, st>>>(x, rows, cols, ld, mean, inv_std);
     return cudaGetLastError();

@@ -7,9 +7,18 @@
 // pass is a tcgen05.mma (kind::f16, BF16 operands from shared memory, FP32
 // accumulators in tensor memory) issued by one thread; the 2-wide output layer,
 // the loss and the elementwise parts run on the CUDA cores from TMEM values.
-// One CTA (4 warps, 128 threads, ~200 KB shared memory, all 512 TMEM columns)
-// per SM; thread t owns batch row t of a 128-row tile for the elementwise work
-// and TMEM lane t (= output row t of every MMA).
+// One CTA (16 warps, ~200 KB shared memory, all 512 TMEM columns) per SM; four
+// threads own batch row t of a 128-row tile for the elementwise work (32 columns
+// each) and TMEM lane t (= output row t of every MMA).
+//
+// Training runs whole: one launch of a cluster of eight CTAs loops over the steps.
+// Up to eight of them compute a tile of the minibatch each and write their gradient
+// partials; after a cluster barrier all eight update their share of the parameters,
+// whose FP32 values and Adam moments stay in registers from step to step, and write the
+// new weights straight into the tile CTAs' shared memory; another barrier starts the
+// next step. A step of 256 rows is bound by the latency of its chain of small products
+// and barriers: 20 us (of it the update 3, the gradients' way out 3), where a launch of the tile kernel and one of the Adam kernel
+// took 41 us. (Minibatches of more than eight tiles still take those two launches.)
 //
 // Shared-memory operand layout (no swizzle): a 128 x 128 BF16 tile stores
 // element (r, c) at byte (r/8)*2048 + (c/8)*128 + (r%8)*16 + (c%8)*2, i.e. 8x8
@@ -36,6 +45,7 @@
 #include <vector>
 
 #include "../../include/ta3b_surrogate.h"
+#include "column_stats.cuh"
 
 namespace ta3s {
 
@@ -43,7 +53,8 @@ constexpr int IN = 97;          // v11 parameter count
 constexpr int IN_K = 112;       // first-layer K, padded to a multiple of 16
 constexpr int HID = 128;
 constexpr int ROWS = 128;       // batch rows per tile = MMA M
-constexpr int THREADS = 128;
+constexpr int THREADS = 512;    // four per row of the tile
+constexpr int CLUSTER = 8;      // CTAs of a training launch
 
 // flat FP32 parameter vector (also the gradient layout)
 constexpr int OFF_W1 = 0;                       // [128][112] (o, i); i >= 97 stays zero
@@ -60,9 +71,14 @@ constexpr uint32_t TILE_BYTES = 128 * 128 * 2;
 constexpr uint32_t S_X = 0, S_W1 = S_X + TILE_BYTES, S_W2 = S_W1 + TILE_BYTES, S_H1 = S_W2 + TILE_BYTES,
                    S_H2 = S_H1 + TILE_BYTES, S_D1 = S_H2 + TILE_BYTES, S_G = S_D1 + TILE_BYTES;   // S_G: [128][16]
 constexpr uint32_t S_F32 = S_G + 128 * 16 * 2;  // W3 [2][128], b1, b2 [128], b3 [2]
-constexpr uint32_t S_BAR = S_F32 + (4 * HID + 4) * 4;
+constexpr uint32_t S_ROW = S_F32 + (4 * HID + 4) * 4;   // per row: source row, mean, log-variance, dmu, ds
+constexpr uint32_t S_BAR = S_ROW + 5 * ROWS * 4;
 constexpr uint32_t S_TMEM = S_BAR + 8;
 constexpr uint32_t SMEM_BYTES = S_TMEM + 8 + 1024;   // + alignment slack
+constexpr int COLS = 32;                        // a thread's columns of its row
+constexpr uint32_t S_OUT = S_H1;                // the gradient tiles on their way out: [128][132] FP32 over H1, H2, D1
+constexpr int LDT = 132;
+static_assert(ROWS * LDT * 4 <= 3 * int(TILE_BYTES) && S_BAR % 8 == 0 && SMEM_BYTES <= 232448, "shared memory");
 
 // TMEM columns
 constexpr uint32_t T_F1 = 0, T_F2 = 128, T_DW2 = 256, T_DW1 = 384, T_SMALL = 496;
@@ -104,7 +120,7 @@ __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::aft
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// 16 consecutive FP32 columns of this thread's TMEM lane
+// consecutive FP32 columns of this thread's TMEM lane; the values are there after tmem_wait
 __device__ __forceinline__ void tmem_ld16(uint32_t addr, float* v) {
     uint32_t r[16];
     asm volatile(
@@ -115,6 +131,38 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, float* v) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+// 32 columns at once (one wait for twice the columns)
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, float* v) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, void const* src, bool valid) {   // zeros when not valid
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// this CTA's shared-memory address, as CTA `rank` of the cluster has it
+__device__ __forceinline__ uint32_t map_rank(uint32_t saddr, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar) {
@@ -147,15 +195,17 @@ __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w 
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
 // 8 FP32 values -> one 16-byte BF16 chunk of a tile
-__device__ __forceinline__ void st_chunk(uint8_t* smem, uint32_t off, float const* v) {
+__device__ __forceinline__ uint4 st_chunk(uint8_t* smem, uint32_t off, float const* v) {
     uint4 q;
     q.x = pack_bf16(v[0], v[1]);
     q.y = pack_bf16(v[2], v[3]);
     q.z = pack_bf16(v[4], v[5]);
     q.w = pack_bf16(v[6], v[7]);
     *reinterpret_cast<uint4*>(smem + off) = q;
+    return q;
 }
 
+// What a tile reads and writes.
 struct Params {
     __nv_bfloat16 const* x;     // [rows][128] standardised inputs (columns >= 97 zero)
     float const* y;             // [rows] standardised targets (training)
@@ -171,89 +221,127 @@ struct Params {
     int train;
 };
 
-__global__ void __launch_bounds__(THREADS, 1) mlp_kernel(Params p) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint32_t const sbase = uint32_t(__cvta_generic_to_shared(sm));
-    int const tid = threadIdx.x, warp = tid >> 5;
-    float* w3s = reinterpret_cast<float*>(sm + S_F32);
-    float* b1s = w3s + 2 * HID;
-    float* b2s = b1s + HID;
-    float* b3s = b2s + HID;
-    uint32_t const bar = sbase + S_BAR;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + S_TMEM);
-    volatile uint32_t* abort_s = reinterpret_cast<volatile uint32_t*>(sm + S_TMEM + 4);   // block-uniform stop
+// One CTA's shared memory, tensor memory and running sums.
+struct Block {
+    uint8_t* sm;
+    uint32_t sbase, tmem, bar, lane_base;
+    int tid, warp, row, part;               // this thread's tile row, and which 32 of the 128 columns it takes
+    float *w3s, *b1s, *b2s, *b3s;           // W3 [2][128], b1, b2 [128], b3 [2]
+    int32_t* src;                           // per row: its source row, -1 = none
+    float *o0s, *o1s, *dmus, *dss;          // per row
+    volatile uint32_t* abort_s;             // block-uniform stop
+    uint32_t phase;
+    bool ok;
+    uint32_t* status;
+    float acc_w3a, acc_w3b, acc_b1, acc_b2;             // threads 0..127: lane = feature
+    float acc_b3a, acc_b3b, acc_loss, acc_rows;         // threads 384..511: row owner
+    bool first;                                          // no tile accumulated yet
 
-    // weights into shared memory: thread o owns rows o of W1 and W2
-    for (int c = 0; c < 16; ++c) {
-        *reinterpret_cast<uint4*>(sm + S_W1 + tile_off(tid, c * 8)) =
-            __ldg(reinterpret_cast<uint4 const*>(p.w1 + tid * 128 + c * 8));
-        *reinterpret_cast<uint4*>(sm + S_W2 + tile_off(tid, c * 8)) =
-            __ldg(reinterpret_cast<uint4 const*>(p.w2 + tid * 128 + c * 8));
+    __device__ void open(uint8_t* smem_raw, uint32_t* status_word) {
+        sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+        sbase = uint32_t(__cvta_generic_to_shared(sm));
+        tid = int(threadIdx.x);
+        warp = tid >> 5;
+        row = tid & (ROWS - 1);
+        part = tid >> 7;
+        w3s = reinterpret_cast<float*>(sm + S_F32);
+        b1s = w3s + 2 * HID;
+        b2s = b1s + HID;
+        b3s = b2s + HID;
+        src = reinterpret_cast<int32_t*>(sm + S_ROW);
+        o0s = reinterpret_cast<float*>(src + ROWS);
+        o1s = o0s + ROWS;
+        dmus = o1s + ROWS;
+        dss = dmus + ROWS;
+        bar = sbase + S_BAR;
+        abort_s = reinterpret_cast<volatile uint32_t*>(sm + S_TMEM + 4);
+        status = status_word;
+        phase = 0;
+        ok = true;
+        if (tid == 0) {
+            mbar_init(bar);
+            *abort_s = 0u;
+        }
+        if (warp == 0) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + S_TMEM),
+                         "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+        fence_before();
+        __syncthreads();
+        fence_after();
+        tmem = *reinterpret_cast<uint32_t volatile*>(sm + S_TMEM);
+        lane_base = tmem + (uint32_t((warp & 3) * 32) << 16);
+        start();
     }
-    w3s[tid] = p.p32[OFF_W3 + tid];
-    w3s[HID + tid] = p.p32[OFF_W3 + HID + tid];
-    b1s[tid] = p.p32[OFF_B1 + tid];
-    b2s[tid] = p.p32[OFF_B2 + tid];
-    if (tid < 2) b3s[tid] = p.p32[OFF_B3 + tid];
-    if (tid == 0) {
-        mbar_init(bar);
-        *abort_s = 0u;
+    __device__ void start() {                // no tile accumulated
+        first = true;
+        acc_w3a = acc_w3b = acc_b1 = acc_b2 = acc_b3a = acc_b3b = acc_loss = acc_rows = 0.f;
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + S_TMEM),
-                     "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    __device__ void close() {
+        fence_before();
+        __syncthreads();
+        fence_after();
+        if (warp == 0)
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
-    fence_async_smem();
-    fence_before();
-    __syncthreads();
-    fence_after();
-    uint32_t const tmem = *tmem_slot;
-    uint32_t const lane_base = tmem + (uint32_t(warp * 32) << 16);   // this warp's TMEM lanes
-    uint32_t phase = 0;
-    bool ok = true;
 
-    // every thread waits for the last commit; a timeout is recorded and makes the
-    // whole block stop at the next tile boundary (all threads read the flag after a barrier)
-    auto sync_mma = [&]() {
+    // every thread waits for the last commit; a timeout is recorded and makes the whole block stop at the
+    // next tile boundary (all threads read the flag after a barrier)
+    __device__ void sync_mma() {
         if (ok && !mbar_wait(bar, phase)) {
             ok = false;
             *abort_s = 1u;
-            atomicOr(p.status, 1u);
+            atomicOr(status, 1u);
         }
         phase ^= 1u;
         fence_after();
-    };
-    auto publish = [&]() {           // smem writes + TMEM reads done -> MMA may run
+    }
+    __device__ void publish() {              // smem writes + TMEM reads done -> MMA may run
         fence_async_smem();
         fence_before();
         __syncthreads();
         fence_after();
-    };
+    }
 
-    uint32_t const x_s = sbase + S_X, w1_s = sbase + S_W1, w2_s = sbase + S_W2, h1_s = sbase + S_H1,
-                   h2_s = sbase + S_H2, d1_s = sbase + S_D1, g_s = sbase + S_G;
-    uint32_t const id128_kk = instr_desc(128, 0, 0), id128_mm = instr_desc(128, 1, 1),
-                   id128_km = instr_desc(128, 0, 1), id112_mm = instr_desc(IN_K, 1, 1),
-                   id16_mm = instr_desc(16, 1, 1);
-
-    float acc_w3a = 0.f, acc_w3b = 0.f, acc_b1 = 0.f, acc_b2 = 0.f;   // lane = feature
-    float acc_b3a = 0.f, acc_b3b = 0.f, acc_loss = 0.f, acc_rows = 0.f;   // row owner
-    int const ntiles = (p.batch + ROWS - 1) / ROWS;
-    bool first = true;
-
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        int const r = tile * ROWS + tid;
-        bool const valid = r < p.batch;
-        int const row = valid ? (p.idx ? p.idx[r] : r) : 0;
-        // ---- X tile
-        for (int c = 0; c < 16; ++c) {
-            uint4 q = make_uint4(0, 0, 0, 0);
-            if (valid) q = __ldg(reinterpret_cast<uint4 const*>(p.x + size_t(row) * 128 + c * 8));
-            *reinterpret_cast<uint4*>(sm + S_X + tile_off(tid, c * 8)) = q;
+    // a 128-row, 256-byte-wide BF16 matrix into its tile, 16 bytes a copy: two neighbouring threads take a
+    // 32-byte sector, sixteen threads 256 bytes of the tile
+    template <class RowOf>
+    __device__ void load_tile(uint32_t dst, __nv_bfloat16 const* base, RowOf row_of) {   // (row -1: zeros)
+#pragma unroll
+        for (int q = 0; q < ROWS * 16 / THREADS; ++q) {
+            int const c = tid + THREADS * q, j = 2 * ((c >> 4) & 7) + (c & 1), r = 8 * (c >> 7) + ((c >> 1) & 7);
+            int const from = row_of(r);
+            cp_async16(sbase + dst + tile_off(r, 8 * j), base + size_t(from < 0 ? 0 : from) * 128 + 8 * j, from >= 0);
         }
-        float const yv = (p.train && valid) ? p.y[row] : 0.f;
+    }
+    __device__ void load_weights(Params const& p) {
+        load_tile(S_W1, p.w1, [](int r) { return r; });
+        load_tile(S_W2, p.w2, [](int r) { return r; });
+        for (int i = tid; i < 4 * HID + 2; i += THREADS)         // W3, b1, b2, b3 in the parameter vector's order
+            w3s[i] = __ldcg(p.p32 + OFF_W3 + i);
+    }
+    __device__ void load_rows(Params const& p, int tile) {       // the X tile and its rows' sources
+        __syncthreads();                                         // (the last tile's rows are done with)
+        if (tid < ROWS) {
+            int const r = tile * ROWS + tid;
+            src[tid] = r < p.batch ? (p.idx ? __ldg(p.idx + r) : r) : -1;
+        }
+        __syncthreads();
+        load_tile(S_X, p.x, [&](int r) { return src[r]; });
+    }
+
+    // forward and backward of the tile in shared memory (weights and rows loaded or on their way)
+    __device__ void run_tile(Params const& p, int tile) {
+        uint32_t const x_s = sbase + S_X, w1_s = sbase + S_W1, w2_s = sbase + S_W2, h1_s = sbase + S_H1,
+                       h2_s = sbase + S_H2, d1_s = sbase + S_D1, g_s = sbase + S_G;
+        uint32_t const id128_kk = instr_desc(128, 0, 0), id128_mm = instr_desc(128, 1, 1),
+                       id128_km = instr_desc(128, 0, 1), id112_mm = instr_desc(IN_K, 1, 1),
+                       id16_mm = instr_desc(16, 1, 1);
+        int const c0 = COLS * part, srow = src[row];
+        bool const valid = srow >= 0, last = part == 3;
+        float const yv = p.train && last && valid ? __ldg(p.y + srow) : 0.f;
+        cp_async_wait();
         publish();
         // ---- layer 1: H1 = X W1^T (M = rows, N = 128, K = 112)
         if (tid == 0) {
@@ -263,13 +351,20 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_kernel(Params p) {
             mma_commit(bar);
         }
         sync_mma();
-        for (int cc = 0; cc < 8; ++cc) {
-            float v[16];
-            tmem_ld16(lane_base + T_F1 + cc * 16, v);
+        float h[COLS];
+        tmem_ld32(lane_base + T_F1 + c0, h);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j] + b1s[cc * 16 + j], 0.f);
-            st_chunk(sm + S_H1, tile_off(tid, cc * 16), v);
-            st_chunk(sm + S_H1, tile_off(tid, cc * 16 + 8), v + 8);
+        for (int j = 0; j < COLS; ++j) h[j] = fmaxf(h[j] + b1s[c0 + j], 0.f);
+        uint32_t m1 = 0u, m2 = 0u;           // relu masks of layers 1 (of the stored BF16 values) and 2, this thread's columns
+#pragma unroll
+        for (int j = 0; j < COLS; j += 8) {
+            uint4 const q = st_chunk(sm + S_H1, tile_off(row, c0 + j), h + j);
+            uint32_t const w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {    // (relu's results: positive unless all bits are zero)
+                m1 |= (w[i] & 0x7FFFu) ? 1u << (j + 2 * i) : 0u;
+                m1 |= (w[i] & 0x7FFF0000u) ? 2u << (j + 2 * i) : 0u;
+            }
         }
         publish();
         // ---- layer 2: H2 = relu(H1) W2^T
@@ -280,133 +375,132 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_kernel(Params p) {
             mma_commit(bar);
         }
         sync_mma();
-        // ---- output layer on the CUDA cores (FP32): mean, log-variance
-        float o0 = b3s[0], o1 = b3s[1];
-        for (int cc = 0; cc < 8; ++cc) {
-            float v[16];
-            tmem_ld16(lane_base + T_F2 + cc * 16, v);
+        // ---- output layer on the CUDA cores (FP32): mean, log-variance; one chain over the columns in
+        // order, so each of the row's threads goes on where the one before ended
+        tmem_ld32(lane_base + T_F2 + c0, h);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                float const h = fmaxf(v[j] + b2s[cc * 16 + j], 0.f);
-                v[j] = h;
-                o0 = fmaf(h, w3s[cc * 16 + j], o0);
-                o1 = fmaf(h, w3s[HID + cc * 16 + j], o1);
+        for (int j = 0; j < COLS; ++j) {
+            float const z = h[j] + b2s[c0 + j];
+            h[j] = fmaxf(z, 0.f);
+            m2 |= z > 0.f ? 1u << j : 0u;
+        }
+        if (p.train) {
+#pragma unroll
+            for (int j = 0; j < COLS; j += 8) st_chunk(sm + S_H2, tile_off(row, c0 + j), h + j);
+        }
+        float o0 = b3s[0], o1 = b3s[1];
+        for (int q = 0; q < 4; ++q) {
+            if (part == q) {
+                if (q) {
+                    o0 = o0s[row];
+                    o1 = o1s[row];
+                }
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) {
+                    o0 = fmaf(h[j], w3s[c0 + j], o0);
+                    o1 = fmaf(h[j], w3s[HID + c0 + j], o1);
+                }
+                o0s[row] = o0;
+                o1s[row] = o1;
             }
-            if (p.train) {
-                st_chunk(sm + S_H2, tile_off(tid, cc * 16), v);
-                st_chunk(sm + S_H2, tile_off(tid, cc * 16 + 8), v + 8);
+            if (q < 3) __syncthreads();
+        }
+        if (last) {
+            if (!p.train) {
+                if (valid) {
+                    size_t const r = size_t(tile) * ROWS + row;
+                    p.out[2 * r] = o0;
+                    p.out[2 * r + 1] = o1;
+                }
+            } else {
+                // ---- Gaussian NLL 0.5 * (s + (y - mu)^2 e^-s), mean over the batch
+                float dmu = 0.f, ds = 0.f;
+                if (valid) {
+                    float const s = fminf(fmaxf(o1, -12.f), 12.f);
+                    float const e = expf(-s);
+                    float const d = yv - o0;
+                    acc_loss += 0.5f * (s + d * d * e);
+                    acc_rows += 1.f;
+                    dmu = -d * e * p.inv_batch;
+                    ds = (o1 > -12.f && o1 < 12.f) ? 0.5f * (1.f - d * d * e) * p.inv_batch : 0.f;
+                }
+                acc_b3a += dmu;
+                acc_b3b += ds;
+                dmus[row] = dmu;
+                dss[row] = ds;
+                float g[16] = {valid ? 1.f : 0.f, dmu, ds, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+                st_chunk(sm + S_G, gtile_off(row, 0), g);
+                st_chunk(sm + S_G, gtile_off(row, 8), g + 8);
             }
         }
         if (!p.train) {
-            if (valid) {
-                p.out[size_t(r) * 2] = o0;
-                p.out[size_t(r) * 2 + 1] = o1;
-            }
             fence_before();
             __syncthreads();
             fence_after();
             ok = *abort_s == 0u;
-            continue;
+            return;
         }
-        // ---- Gaussian NLL 0.5 * (s + (y - mu)^2 e^-s), mean over the batch
-        float dmu = 0.f, ds = 0.f;
-        if (valid) {
-            float const s = fminf(fmaxf(o1, -12.f), 12.f);
-            float const e = expf(-s);
-            float const d = yv - o0;
-            acc_loss += 0.5f * (s + d * d * e);
-            acc_rows += 1.f;
-            dmu = -d * e * p.inv_batch;
-            ds = (o1 > -12.f && o1 < 12.f) ? 0.5f * (1.f - d * d * e) * p.inv_batch : 0.f;
-        }
-        acc_b3a += dmu;
-        acc_b3b += ds;
+        __syncthreads();
+        // ---- dH2 = (dmu W3[0] + ds W3[1]) * relu'(H2), into the D1 tile
         {
-            float g[16] = {valid ? 1.f : 0.f, dmu, ds, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-            st_chunk(sm + S_G, gtile_off(tid, 0), g);
-            st_chunk(sm + S_G, gtile_off(tid, 8), g + 8);
+            float const dmu = dmus[row], ds = dss[row];
+#pragma unroll
+            for (int j = 0; j < COLS; ++j)
+                h[j] = (m2 >> j) & 1u ? fmaf(dmu, w3s[c0 + j], ds * w3s[HID + c0 + j]) : 0.f;
+#pragma unroll
+            for (int j = 0; j < COLS; j += 8) st_chunk(sm + S_D1, tile_off(row, c0 + j), h + j);
         }
         publish();
-        // ---- dW3^T[i][c] = sum_b H2[b][i] G[b][c]   (M = feature, N = 16, K = rows)
+        // ---- dW3^T[i][c] = sum_b H2[b][i] G[b][c] (M = feature, N = 16, K = rows) and dH1 = dH2 W2, which
+        // the next step waits for; behind them db2 = column sums of dH2 (its 16 columns over F2, which has
+        // been read) and dW2 += dH2^T H1, which the last commit covers
         if (tid == 0) {
             for (int kk = 0; kk < ROWS / 16; ++kk)
                 mma_bf16(tmem + T_SMALL, smem_desc(h2_s + kk * 4096, 2048, 128), smem_desc(g_s + kk * 512, 256, 128),
                          id16_mm, kk > 0);
+            for (int kk = 0; kk < HID / 16; ++kk)
+                mma_bf16(tmem + T_F1, smem_desc(d1_s + kk * 256, 128, 2048), smem_desc(w2_s + kk * 4096, 2048, 128),
+                         id128_km, kk > 0);
             mma_commit(bar);
+            for (int kk = 0; kk < ROWS / 16; ++kk)
+                mma_bf16(tmem + T_F2, smem_desc(d1_s + kk * 4096, 2048, 128), smem_desc(g_s + kk * 512, 256, 128),
+                         id16_mm, kk > 0);
+            for (int kk = 0; kk < ROWS / 16; ++kk)
+                mma_bf16(tmem + T_DW2, smem_desc(d1_s + kk * 4096, 2048, 128), smem_desc(h1_s + kk * 4096, 2048, 128),
+                         id128_mm, (!first || kk > 0) ? 1u : 0u);
         }
         sync_mma();
-        {
+        if (part == 0) {
             float v[16];
             tmem_ld16(lane_base + T_SMALL, v);
             acc_w3a += v[1];
             acc_w3b += v[2];
         }
-        // ---- dH2 = (dmu W3[0] + ds W3[1]) * relu'(H2) (overwrites the H2 tile: its MMA has completed)
-        for (int cc = 0; cc < 8; ++cc) {
-            float v[16];
-            tmem_ld16(lane_base + T_F2 + cc * 16, v);
+        // ---- dH1 = (dH2 W2) * relu'(H1), into the H2 tile (its product has completed)
+        tmem_ld32(lane_base + T_F1 + c0, h);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                int const o = cc * 16 + j;
-                v[j] = (v[j] + b2s[o] > 0.f) ? fmaf(dmu, w3s[o], ds * w3s[HID + o]) : 0.f;
-            }
-            st_chunk(sm + S_H2, tile_off(tid, cc * 16), v);
-            st_chunk(sm + S_H2, tile_off(tid, cc * 16 + 8), v + 8);
-        }
-        publish();
-        // ---- dW2 += dH2^T H1, dH1 = dH2 W2, db2 = column sums of dH2
-        if (tid == 0) {
-            for (int kk = 0; kk < ROWS / 16; ++kk)
-                mma_bf16(tmem + T_DW2, smem_desc(h2_s + kk * 4096, 2048, 128), smem_desc(h1_s + kk * 4096, 2048, 128),
-                         id128_mm, (!first || kk > 0) ? 1u : 0u);
-            for (int kk = 0; kk < HID / 16; ++kk)
-                mma_bf16(tmem + T_F1, smem_desc(h2_s + kk * 256, 128, 2048), smem_desc(w2_s + kk * 4096, 2048, 128),
-                         id128_km, kk > 0);
-            for (int kk = 0; kk < ROWS / 16; ++kk)
-                mma_bf16(tmem + T_SMALL, smem_desc(h2_s + kk * 4096, 2048, 128), smem_desc(g_s + kk * 512, 256, 128),
-                         id16_mm, kk > 0);
-            mma_commit(bar);
-        }
-        sync_mma();
-        {
-            float v[16];
-            tmem_ld16(lane_base + T_SMALL, v);
-            acc_b2 += v[0];
-        }
-        // ---- dH1 = (dH2 W2) * relu'(H1), the mask read back from this thread's H1 row
-        for (int cc = 0; cc < 8; ++cc) {
-            float v[16];
-            tmem_ld16(lane_base + T_F1 + cc * 16, v);
+        for (int j = 0; j < COLS; ++j)
+            if (!((m1 >> j) & 1u)) h[j] = 0.f;
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint4 const h = *reinterpret_cast<uint4 const*>(sm + S_H1 + tile_off(tid, cc * 16 + half * 8));
-                uint32_t const hw[4] = {h.x, h.y, h.z, h.w};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    float* vv = v + half * 8 + q * 2;
-                    if (!(bf16_lo(hw[q]) > 0.f)) vv[0] = 0.f;
-                    if (!(bf16_hi(hw[q]) > 0.f)) vv[1] = 0.f;
-                }
-            }
-            st_chunk(sm + S_D1, tile_off(tid, cc * 16), v);
-            st_chunk(sm + S_D1, tile_off(tid, cc * 16 + 8), v + 8);
-        }
+        for (int j = 0; j < COLS; j += 8) st_chunk(sm + S_H2, tile_off(row, c0 + j), h + j);
         publish();
         // ---- dW1 += dH1^T X (N = 112), db1 = column sums of dH1
         if (tid == 0) {
             for (int kk = 0; kk < ROWS / 16; ++kk)
-                mma_bf16(tmem + T_DW1, smem_desc(d1_s + kk * 4096, 2048, 128), smem_desc(x_s + kk * 4096, 2048, 128),
-                         id112_mm, (!first || kk > 0) ? 1u : 0u);
-            for (int kk = 0; kk < ROWS / 16; ++kk)
-                mma_bf16(tmem + T_SMALL, smem_desc(d1_s + kk * 4096, 2048, 128), smem_desc(g_s + kk * 512, 256, 128),
+                mma_bf16(tmem + T_SMALL, smem_desc(h2_s + kk * 4096, 2048, 128), smem_desc(g_s + kk * 512, 256, 128),
                          id16_mm, kk > 0);
+            for (int kk = 0; kk < ROWS / 16; ++kk)
+                mma_bf16(tmem + T_DW1, smem_desc(h2_s + kk * 4096, 2048, 128), smem_desc(x_s + kk * 4096, 2048, 128),
+                         id112_mm, (!first || kk > 0) ? 1u : 0u);
             mma_commit(bar);
         }
         sync_mma();
-        {
+        if (part == 0) {
             float v[16];
             tmem_ld16(lane_base + T_SMALL, v);
             acc_b1 += v[0];
+            tmem_ld16(lane_base + T_F2, v);
+            acc_b2 += v[0];
         }
         first = false;
         fence_before();
@@ -415,79 +509,231 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_kernel(Params p) {
         ok = *abort_s == 0u;
     }
 
-    if (p.train) {
-        float* part = p.partial + size_t(blockIdx.x) * PARTIAL;
-        int const o = tid;   // TMEM lane = feature row of the weight gradients
-        if (ok && !first) {
-            for (int cc = 0; cc < 8; ++cc) {
+    // one weight gradient ([128][cols] from `off` of the parameter vector) from TMEM through shared memory, so
+    // that rows go out in whole lines
+    template <int COLUMNS>
+    __device__ void write_gradient(uint32_t t_col, bool have, float* dst) {
+        float* const t = reinterpret_cast<float*>(sm + S_OUT);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            int const c = COLS * part + 16 * u;
+            if (c < COLUMNS) {                                   // (uniform over a warp)
                 float v[16];
-                tmem_ld16(lane_base + T_DW2 + cc * 16, v);
-                for (int j = 0; j < 16; ++j) part[OFF_W2 + o * HID + cc * 16 + j] = v[j];
+                if (have) {
+                    tmem_ld16(lane_base + t_col + c, v);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = 0.f;
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (COLUMNS == IN_K && c + j >= IN) v[j] = 0.f;
+#pragma unroll
+                for (int j = 0; j < 16; j += 4)
+                    *reinterpret_cast<float4*>(t + row * LDT + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             }
-            for (int cc = 0; cc < IN_K / 16; ++cc) {
-                float v[16];
-                tmem_ld16(lane_base + T_DW1 + cc * 16, v);
-                for (int j = 0; j < 16; ++j) part[OFF_W1 + o * IN_K + cc * 16 + j] = (cc * 16 + j < IN) ? v[j] : 0.f;
-            }
-        } else {
-            for (int i = 0; i < HID; ++i) part[OFF_W2 + o * HID + i] = 0.f;
-            for (int i = 0; i < IN_K; ++i) part[OFF_W1 + o * IN_K + i] = 0.f;
         }
-        part[OFF_W3 + o] = acc_w3a;
-        part[OFF_W3 + HID + o] = acc_w3b;
-        part[OFF_B1 + o] = acc_b1;
-        part[OFF_B2 + o] = acc_b2;
-        // row-owned sums: block reduction through shared memory (the S_G tile is free now)
-        float* red = reinterpret_cast<float*>(sm + S_G);
         __syncthreads();
-        red[tid] = acc_b3a;
-        red[THREADS + tid] = acc_b3b;
-        red[2 * THREADS + tid] = acc_loss;
-        red[3 * THREADS + tid] = acc_rows;
-        __syncthreads();
-        if (tid < 4) {
-            float s = 0.f;
-            for (int k = 0; k < THREADS; ++k) s += red[tid * THREADS + k];
-            int const dst[4] = {OFF_B3, OFF_B3 + 1, NPARAM, NPARAM + 1};
-            part[dst[tid]] = s;
+        constexpr int QUADS = COLUMNS / 4;
+#pragma unroll
+        for (int q = 0; q < HID * QUADS / THREADS; ++q) {
+            int const i = tid + THREADS * q, r = i / QUADS, c = 4 * (i % QUADS);
+            *reinterpret_cast<float4*>(dst + r * COLUMNS + c) = *reinterpret_cast<float4 const*>(t + r * LDT + c);
         }
+        __syncthreads();
     }
-    fence_before();
-    __syncthreads();
-    fence_after();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    // this CTA's gradient partials
+    __device__ void write_partial(float* out) {
+        float* const red = reinterpret_cast<float*>(sm + S_G);
+        bool const have = ok && !first;
+        if (part == 3) {                                         // row-owned sums, added in row order below
+            red[row] = acc_b3a;
+            red[ROWS + row] = acc_b3b;
+            red[2 * ROWS + row] = acc_loss;
+            red[3 * ROWS + row] = acc_rows;
+        }
+        if (part == 0) {
+            out[OFF_W3 + tid] = acc_w3a;
+            out[OFF_W3 + HID + tid] = acc_w3b;
+            out[OFF_B1 + tid] = acc_b1;
+            out[OFF_B2 + tid] = acc_b2;
+        }
+        write_gradient<HID>(T_DW2, have, out + OFF_W2);
+        if (tid >= THREADS - 4) {
+            int const k = tid - (THREADS - 4);
+            float s = 0.f;
+#pragma unroll 16
+            for (int r = 0; r < ROWS; ++r) s += red[k * ROWS + r];
+            out[k < 2 ? OFF_B3 + k : NPARAM + k - 2] = s;
+        }
+        write_gradient<IN_K>(T_DW1, have, out + OFF_W1);
+    }
+};
+
+// predictions, or one pass's gradient partials: tiles dealt to the CTAs in turn
+__global__ void __launch_bounds__(THREADS, 1) mlp_kernel(Params p) {
+    extern __shared__ uint8_t smem_raw[];
+    Block b;
+    b.open(smem_raw, p.status);
+    b.load_weights(p);
+    int const ntiles = (p.batch + ROWS - 1) / ROWS;
+    for (int tile = int(blockIdx.x); tile < ntiles && b.ok; tile += int(gridDim.x)) {
+        b.load_rows(p, tile);
+        b.run_tile(p, tile);
+    }
+    if (p.train) b.write_partial(p.partial + size_t(blockIdx.x) * PARTIAL);
+    b.close();
+}
+
+// AdamW's constants; one parameter's step from its gradient
+struct AdamConst {
+    float lr, b1, b2, eps, wd;
+    __device__ __forceinline__ float step(float g, float c1, float c2, float& m, float& v, float w) const {
+        m = b1 * m + (1.f - b1) * g;
+        v = b2 * v + (1.f - b2) * g * g;
+        return w - lr * (m / c1) / (sqrtf(v / c2) + eps) - lr * wd * w;
+    }
+};
+__device__ __forceinline__ bool is_padding(int i) { return i < OFF_W2 && (i % IN_K) >= IN; }
+// the BF16 copy of parameter i (W1, W2)
+__device__ __forceinline__ void store_bf16(int i, float w, __nv_bfloat16* w1b, __nv_bfloat16* w2b) {
+    if (i < OFF_W2) w1b[(i / IN_K) * 128 + i % IN_K] = __float2bfloat16_rn(w);
+    else if (i < OFF_W3) w2b[i - OFF_W2] = __float2bfloat16_rn(w);
+}
+
+// `steps` training steps in one launch of one cluster (minibatches of at most CLUSTER tiles).
+struct TrainArgs {
+    Params p;                    // idx: the first step's rows; batch: rows of a full minibatch
+    int steps, first_step;       // steps of this launch; how many of the call came before
+    int steps_per_epoch, rows;   // the last minibatch of an epoch has what is left of the rows
+    float const* c1;             // [steps] bias corrections 1 - b1^t, 1 - b2^t
+    float const* c2;
+    float* param;
+    float* m;
+    float* v;
+    __nv_bfloat16* w1b;
+    __nv_bfloat16* w2b;
+    AdamConst adam;
+    float* loss_out;             // the last step's summed loss and rows
+};
+constexpr int OWN = 8;           // parameters per thread: eight in a row are one 16-byte chunk of a BF16 tile
+static_assert(CLUSTER * THREADS * OWN >= NPARAM && IN_K % OWN == 0 && OFF_W2 % OWN == 0 && OFF_W3 % OWN == 0 &&
+              PARTIAL % 4 == 0, "the cluster owns every parameter, in whole chunks of the weight matrices");
+
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS, 1) train_kernel(TrainArgs a) {
+    extern __shared__ uint8_t smem_raw[];
+    int const rank = int(blockIdx.x), tid = int(threadIdx.x);
+    Block b;
+    b.open(smem_raw, a.p.status);
+    // this thread's parameters; values and moments stay in registers
+    int const i0 = (rank * THREADS + tid) * OWN;
+    auto owned = [&](int k) { return i0 + k < NPARAM; };
+    float w[OWN], m[OWN], v[OWN];
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+        w[k] = owned(k) ? a.param[i0 + k] : 0.f;
+        m[k] = owned(k) ? a.m[i0 + k] : 0.f;
+        v[k] = owned(k) ? a.v[i0 + k] : 0.f;
+    }
+    // where they live in a tile CTA's shared memory: a BF16 chunk of W1 or W2, or FP32 words of W3 and the
+    // biases (in the parameter vector's order; the last chunk's words past b3 are padding)
+    uint32_t const home = b.sbase + (i0 < OFF_W2   ? S_W1 + tile_off(i0 / IN_K, i0 % IN_K)
+                                     : i0 < OFF_W3 ? S_W2 + tile_off((i0 - OFF_W2) / HID, (i0 - OFF_W2) % HID)
+                                                   : S_F32 + 4u * uint32_t(i0 - OFF_W3));
+    auto minibatch = [&](int s) {                       // step s of this launch
+        Params p = a.p;
+        int const in_epoch = (a.first_step + s) % a.steps_per_epoch;
+        p.batch = min(a.p.batch, a.rows - in_epoch * a.p.batch);
+        p.idx = a.p.idx + size_t(s) * a.p.batch;
+        p.inv_batch = 1.0f / float(p.batch);
+        return p;
+    };
+    auto tiles = [](Params const& p) { return (p.batch + ROWS - 1) / ROWS; };
+    Params p = minibatch(0);
+    int const most = tiles(a.p);                        // CTAs that ever take a tile: their weights stay in shared memory
+    if (rank < most) b.load_weights(p);
+    if (rank < tiles(p)) b.load_rows(p, rank);
+    for (int s = 0; s < a.steps; ++s) {
+        int const n = tiles(p);
+        float const c1 = __ldg(a.c1 + s), c2 = __ldg(a.c2 + s);
+        if (rank < n) {
+            b.start();
+            b.run_tile(p, rank);
+            b.write_partial(p.partial + size_t(rank) * PARTIAL);
+        }
+        Params const next = s + 1 < a.steps ? minibatch(s + 1) : p;
+        if (s + 1 < a.steps && rank < tiles(next)) b.load_rows(next, rank);     // on their way during the update
+        cluster_sync();
+        if (*reinterpret_cast<volatile uint32_t*>(a.p.status)) break;           // (set before the barrier: all see it)
+        if (i0 < NPARAM) {
+            float g[OWN];
+#pragma unroll
+            for (int k = 0; k < OWN; ++k) g[k] = 0.f;
+            for (int q = 0; q < n; ++q) {               // the partials in CTA order
+                float const* const from = p.partial + size_t(q) * PARTIAL + i0;
+                float4 const lo = __ldcg(reinterpret_cast<float4 const*>(from));
+                float4 const hi = owned(4) ? __ldcg(reinterpret_cast<float4 const*>(from + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                float const t[OWN] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                for (int k = 0; k < OWN; ++k) g[k] += t[k];
+            }
+#pragma unroll
+            for (int k = 0; k < OWN; ++k)
+                if (owned(k) && !is_padding(i0 + k)) w[k] = a.adam.step(g[k], c1, c2, m[k], v[k], w[k]);
+            for (int q = 0; q < most; ++q) {
+                uint32_t const at = map_rank(home, q);
+                if (i0 < OFF_W3) {
+                    st_cluster128(at, pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]), pack_bf16(w[4], w[5]),
+                                  pack_bf16(w[6], w[7]));
+                } else {
+                    st_cluster128(at, __float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), __float_as_uint(w[3]));
+                    if (owned(4))
+                        st_cluster128(at + 16, __float_as_uint(w[4]), __float_as_uint(w[5]), __float_as_uint(w[6]),
+                                      __float_as_uint(w[7]));
+                }
+            }
+        }
+        if (s + 1 == a.steps && rank == 0 && tid < 2) {
+            float t = 0.f;
+            for (int q = 0; q < n; ++q) t += __ldcg(p.partial + size_t(q) * PARTIAL + NPARAM + tid);
+            a.loss_out[tid] = t;
+        }
+        cluster_sync();
+        p = next;
+    }
+#pragma unroll
+    for (int k = 0; k < OWN; ++k)
+        if (owned(k)) {
+            a.param[i0 + k] = w[k];
+            a.m[i0 + k] = m[k];
+            a.v[i0 + k] = v[k];
+            if (!is_padding(i0 + k)) store_bf16(i0 + k, w[k], a.w1b, a.w2b);
+        }
+    cp_async_wait();
+    b.close();
 }
 
 // Adam over the flat parameter vector; gradients summed over the CTA partials
-// in a fixed order (deterministic). Refreshes the BF16 weight copies.
+// in a fixed order (deterministic). Refreshes the BF16 weight copies. The update
+// of minibatches that one cluster cannot hold.
 __global__ void adam_kernel(float* __restrict__ param, float* __restrict__ m, float* __restrict__ v,
-                            float const* __restrict__ partial, int nparts, float lr, float b1, float b2, float eps,
-                            float c1, float c2, float wd, __nv_bfloat16* __restrict__ w1b, __nv_bfloat16* __restrict__ w2b,
-                            float* __restrict__ loss_out) {
+                            float const* __restrict__ partial, int nparts, AdamConst ad, float c1, float c2,
+                            __nv_bfloat16* __restrict__ w1b, __nv_bfloat16* __restrict__ w2b, float* __restrict__ loss_out) {
     int const i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < PARTIAL && i >= NPARAM && loss_out) {
-        float s = 0.f;
-        for (int k = 0; k < nparts; ++k) s += partial[size_t(k) * PARTIAL + i];
-        loss_out[i - NPARAM] = s;
-    }
-    if (i >= NPARAM) return;
+    if (i >= PARTIAL) return;
     float g = 0.f;
     for (int k = 0; k < nparts; ++k) g += partial[size_t(k) * PARTIAL + i];
-    bool const pad = i < OFF_W2 && (i % IN_K) >= IN;
-    if (pad) return;
-    float const mi = b1 * m[i] + (1.f - b1) * g;
-    float const vi = b2 * v[i] + (1.f - b2) * g * g;
+    if (i >= NPARAM) {
+        loss_out[i - NPARAM] = g;
+        return;
+    }
+    if (is_padding(i)) return;
+    float mi = m[i], vi = v[i];
+    float const w = ad.step(g, c1, c2, mi, vi, param[i]);
     m[i] = mi;
     v[i] = vi;
-    float const w = param[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps) - lr * wd * param[i];   // AdamW
     param[i] = w;
-    if (i < OFF_W2) {
-        int const o = i / IN_K, c = i % IN_K;
-        w1b[o * 128 + c] = __float2bfloat16_rn(w);
-    } else if (i < OFF_W3) {
-        int const k = i - OFF_W2;
-        w2b[k] = __float2bfloat16_rn(w);
-    }
+    store_bf16(i, w, w1b, w2b);
 }
 
 // BF16 weight copies from the FP32 parameters
@@ -537,7 +783,8 @@ struct ta3s_model {
     size_t cap_idx = 0;
     float* d_out = nullptr;
     float* d_stats = nullptr;     // mean[128], inv_std[128]
-    std::vector<float> x_mean, x_inv_std;
+    float* d_corr = nullptr;      // a training call's bias corrections
+    size_t cap_corr = 0;
     float y_mean = 0.f, y_std = 1.f;
     uint32_t rows = 0;
     uint64_t adam_t = 0;
@@ -577,7 +824,9 @@ int check_status(ta3s_model* m) {
     return 0;
 }
 
-int upload_rows(ta3s_model* m, float const* x, uint32_t n) {
+// the rows on the device, standardised in BF16 (with `standardize` by their own statistics, which stay for
+// later predictions)
+int upload_rows(ta3s_model* m, float const* x, uint32_t n, bool standardize) {
     size_t cap = m->cap_rows;
     if (n > cap) {
         size_t c1 = cap, c2 = cap, c3 = cap;
@@ -589,14 +838,15 @@ int upload_rows(ta3s_model* m, float const* x, uint32_t n) {
         m->cap_rows = n;
     }
     TA3S_CUDA(m, cudaMemcpyAsync(m->d_xraw, x, size_t(n) * IN * 4, cudaMemcpyHostToDevice, m->stream), "copy rows");
+    if (standardize)
+        TA3S_CUDA(m, ta3_stats::column_stats(m->d_xraw, int(n), IN, IN, m->d_stats, m->d_stats + 128, m->stream),
+                  "column statistics");
     pack_kernel<<<(n * 128 + 255) / 256, 256, 0, m->stream>>>(m->d_xraw, int(n), m->d_stats, m->d_stats + 128, m->d_x);
     TA3S_CUDA(m, cudaGetLastError(), "pack");
     return 0;
 }
 
-int launch_mlp(ta3s_model* m, int batch, int32_t const* d_idx, int train) {
-    int const ntiles = (batch + ROWS - 1) / ROWS;
-    int const grid = std::min(ntiles, m->sms);
+Params make_params(ta3s_model* m, int batch, int32_t const* d_idx, int train) {
     Params prm{};
     prm.x = m->d_x;
     prm.y = m->d_y;
@@ -610,7 +860,13 @@ int launch_mlp(ta3s_model* m, int batch, int32_t const* d_idx, int train) {
     prm.status = m->d_status;
     prm.inv_batch = 1.0f / float(batch);
     prm.train = train;
-    mlp_kernel<<<grid, THREADS, SMEM_BYTES, m->stream>>>(prm);
+    return prm;
+}
+
+int launch_mlp(ta3s_model* m, int batch, int32_t const* d_idx, int train) {
+    int const ntiles = (batch + ROWS - 1) / ROWS;
+    int const grid = std::min(ntiles, m->sms);
+    mlp_kernel<<<grid, THREADS, SMEM_BYTES, m->stream>>>(make_params(m, batch, d_idx, train));
     TA3S_CUDA(m, cudaGetLastError(), "surrogate mlp launch");
     return 0;
 }
@@ -642,7 +898,9 @@ ta3s_model* ta3s_create(int device, uint32_t seed) {
     }
     m->sms = prop.multiProcessorCount;
     if ((e = cudaFuncSetAttribute(mlp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES))) !=
-        cudaSuccess)
+            cudaSuccess ||
+        (e = cudaFuncSetAttribute(train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES))) !=
+            cudaSuccess)
         return bad("smem attribute", e);
     if ((e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking)) != cudaSuccess) return bad("stream", e);
     size_t const part = size_t(m->sms) * PARTIAL;
@@ -666,8 +924,6 @@ ta3s_model* ta3s_create(int device, uint32_t seed) {
     }
     std::vector<float> stats(256, 0.f);
     for (int c = 0; c < 128; ++c) stats[128 + c] = 1.f;
-    m->x_mean.assign(IN, 0.f);
-    m->x_inv_std.assign(IN, 1.f);
     // every copy and fill goes on the model's stream: its kernels run on a non-blocking stream, which
     // does not wait for work on the legacy default stream (a pageable cudaMemcpy can even return
     // before its DMA has landed)
@@ -686,7 +942,7 @@ void ta3s_destroy(ta3s_model* m) {
     cudaSetDevice(m->device);
     for (void* p : {(void*)m->d_param, (void*)m->d_m, (void*)m->d_v, (void*)m->d_w1b, (void*)m->d_w2b,
                     (void*)m->d_partial, (void*)m->d_status, (void*)m->d_loss, (void*)m->d_xraw, (void*)m->d_x,
-                    (void*)m->d_y, (void*)m->d_idx, (void*)m->d_out, (void*)m->d_stats})
+                    (void*)m->d_y, (void*)m->d_idx, (void*)m->d_out, (void*)m->d_stats, (void*)m->d_corr})
         if (p) cudaFree(p);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
@@ -719,30 +975,14 @@ int ta3s_get_params(ta3s_model* m, float* params_out) {
 int ta3s_set_data(ta3s_model* m, const float* x, const float* y, uint32_t n) {
     if (!m || !x || !y || n == 0) return fail(m, "ta3s_set_data: need n > 0 rows");
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
-    // per-column standardisation of inputs and of the target (host, FP64 sums)
-    std::vector<float> stats(256, 0.f);
-    for (int c = 0; c < IN; ++c) {
-        double s = 0, s2 = 0;
-        for (uint32_t r = 0; r < n; ++r) s += x[size_t(r) * IN + c];
-        double const mu = s / n;
-        for (uint32_t r = 0; r < n; ++r) {
-            double const d = x[size_t(r) * IN + c] - mu;
-            s2 += d * d;
-        }
-        double const sd = std::sqrt(s2 / n);
-        m->x_mean[c] = float(mu);
-        m->x_inv_std[c] = sd > 1e-12 ? float(1.0 / sd) : 1.f;
-        stats[c] = m->x_mean[c];
-        stats[128 + c] = m->x_inv_std[c];
-    }
+    // per-column standardisation of the inputs (device) and of the target (host), FP64 sums
     double s = 0, s2 = 0;
     for (uint32_t r = 0; r < n; ++r) s += y[r];
     double const mu = s / n;
     for (uint32_t r = 0; r < n; ++r) s2 += (y[r] - mu) * (y[r] - mu);
     m->y_mean = float(mu);
     m->y_std = s2 > 0 ? float(std::sqrt(s2 / n)) : 1.f;
-    TA3S_CUDA(m, cudaMemcpyAsync(m->d_stats, stats.data(), 256 * 4, cudaMemcpyHostToDevice, m->stream), "stats");
-    if (upload_rows(m, x, n)) return 1;
+    if (upload_rows(m, x, n, true)) return 1;
     std::vector<float> ys(n);
     for (uint32_t r = 0; r < n; ++r) ys[r] = (y[r] - m->y_mean) / m->y_std;
     TA3S_CUDA(m, cudaMemcpyAsync(m->d_y, ys.data(), size_t(n) * 4, cudaMemcpyHostToDevice, m->stream), "targets");
@@ -756,12 +996,10 @@ int ta3s_set_data_standardized(ta3s_model* m, const float* x, const float* y, ui
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
     std::vector<float> stats(256, 0.f);
     for (int c = 0; c < 128; ++c) stats[128 + c] = 1.f;
-    std::fill(m->x_mean.begin(), m->x_mean.end(), 0.f);
-    std::fill(m->x_inv_std.begin(), m->x_inv_std.end(), 1.f);
     m->y_mean = 0.f;
     m->y_std = 1.f;
     TA3S_CUDA(m, cudaMemcpyAsync(m->d_stats, stats.data(), 256 * 4, cudaMemcpyHostToDevice, m->stream), "stats");
-    if (upload_rows(m, x, n)) return 1;
+    if (upload_rows(m, x, n, false)) return 1;
     TA3S_CUDA(m, cudaMemcpyAsync(m->d_y, y, size_t(n) * 4, cudaMemcpyHostToDevice, m->stream), "targets");
     TA3S_CUDA(m, cudaStreamSynchronize(m->stream), "set data");
     m->rows = n;
@@ -812,20 +1050,52 @@ int ta3s_train(ta3s_model* m, uint32_t epochs, uint32_t batch, float lr, float w
     if (grow(m, m->d_idx, m->cap_idx, std::max<size_t>(total, 1), "alloc indices")) return 1;
     TA3S_CUDA(m, cudaMemcpyAsync(m->d_idx, idx.data(), total * 4, cudaMemcpyHostToDevice, m->stream), "indices");
     TA3S_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
-    float const b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    for (uint32_t e = 0; e < epochs; ++e)
-        for (uint32_t s = 0; s < steps_per_epoch; ++s) {
-            uint32_t const rows_here = std::min(batch, n - s * batch);
-            if (launch_mlp(m, int(rows_here), m->d_idx + (size_t(e) * steps_per_epoch + s) * batch, 1)) return 1;
-            ++m->adam_t;
-            float const c1 = 1.f - std::pow(b1, float(m->adam_t)), c2 = 1.f - std::pow(b2, float(m->adam_t));
+    AdamConst const ad{lr, 0.9f, 0.999f, 1e-8f, weight_decay};
+    uint64_t const steps = uint64_t(epochs) * steps_per_epoch;
+    // bias corrections of every step
+    std::vector<float> corr(2 * size_t(steps));
+    for (uint64_t k = 0; k < steps; ++k) {
+        ++m->adam_t;
+        corr[k] = 1.f - std::pow(ad.b1, float(m->adam_t));
+        corr[steps + k] = 1.f - std::pow(ad.b2, float(m->adam_t));
+    }
+    if (std::min(batch, n) <= uint32_t(CLUSTER * ROWS)) {
+        // minibatches of one cluster: whole runs of steps in one launch, bounded so that a launch stays short
+        constexpr uint64_t kStepsPerLaunch = 4096;
+        if (steps && grow(m, m->d_corr, m->cap_corr, corr.size(), "alloc bias corrections")) return 1;
+        if (steps)
+            TA3S_CUDA(m, cudaMemcpyAsync(m->d_corr, corr.data(), corr.size() * 4, cudaMemcpyHostToDevice, m->stream),
+                      "bias corrections");
+        for (uint64_t k = 0; k < steps; k += kStepsPerLaunch) {
+            TrainArgs a{};
+            a.p = make_params(m, int(batch), m->d_idx + size_t(k) * batch, 1);
+            a.steps = int(std::min(kStepsPerLaunch, steps - k));
+            a.first_step = int(k % steps_per_epoch);
+            a.steps_per_epoch = int(steps_per_epoch);
+            a.rows = int(n);
+            a.c1 = m->d_corr + k;
+            a.c2 = m->d_corr + steps + k;
+            a.param = m->d_param;
+            a.m = m->d_m;
+            a.v = m->d_v;
+            a.w1b = m->d_w1b;
+            a.w2b = m->d_w2b;
+            a.adam = ad;
+            a.loss_out = m->d_loss;
+            train_kernel<<<CLUSTER, THREADS, SMEM_BYTES, m->stream>>>(a);
+            TA3S_CUDA(m, cudaGetLastError(), "train launch");
+        }
+    } else {
+        for (uint64_t k = 0; k < steps; ++k) {
+            uint32_t const rows_here = std::min(batch, n - uint32_t(k % steps_per_epoch) * batch);
+            if (launch_mlp(m, int(rows_here), m->d_idx + size_t(k) * batch, 1)) return 1;
             int const grid = std::min(int((rows_here + ROWS - 1) / ROWS), m->sms);
-            adam_kernel<<<(PARTIAL + 255) / 256, 256, 0, m->stream>>>(m->d_param, m->d_m, m->d_v, m->d_partial, grid,
-                                                                      lr, b1, b2, eps, c1, c2, weight_decay,
-                                                                      m->d_w1b, m->d_w2b,
+            adam_kernel<<<(PARTIAL + 255) / 256, 256, 0, m->stream>>>(m->d_param, m->d_m, m->d_v, m->d_partial, grid, ad,
+                                                                      corr[k], corr[steps + k], m->d_w1b, m->d_w2b,
                                                                       m->d_loss);
             TA3S_CUDA(m, cudaGetLastError(), "adam launch");
         }
+    }
     if (check_status(m)) return 1;
     if (final_loss) {
         float l[2];
@@ -839,7 +1109,7 @@ int ta3s_predict(ta3s_model* m, const float* x, uint32_t n, float* mean_out, flo
     if (!m || !x || !mean_out) return fail(m, "ta3s_predict: null argument");
     if (n == 0) return 0;
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
-    if (upload_rows(m, x, n)) return 1;
+    if (upload_rows(m, x, n, false)) return 1;
     TA3S_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
     if (launch_mlp(m, int(n), nullptr, 0)) return 1;
     std::vector<float> out(size_t(n) * 2);
