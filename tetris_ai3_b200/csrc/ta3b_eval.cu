@@ -428,16 +428,23 @@ __device__ __forceinline__ uint64_t shfl64_xor(uint64_t v, int m) {
     return (uint64_t(__shfl_xor_sync(FULL_MASK, uint32_t(v >> 32), m)) << 32) | __shfl_xor_sync(FULL_MASK, uint32_t(v), m);
 }
 
-// Bitonic sort of one key per lane into descending order (lane i = i-th largest).
+// One compare-exchange: lanes whose bit j is clear keep the larger key of the pair, the others the smaller.
+__device__ __forceinline__ uint64_t keep_larger_low(uint64_t v, int j, int lane) {
+    uint64_t const o = shfl64_xor(v, j);
+    return (v > o) != ((lane & j) != 0) ? v : o;
+}
+
+// Bitonic sort of one key per lane into descending order (lane i = i-th largest). Runs that have to ascend
+// hold their keys complemented, so every exchange is the same.
 __device__ __forceinline__ uint64_t warp_sort_desc(uint64_t v, int lane) {
+    uint32_t flipped = 0;
 #pragma unroll
     for (int k = 2; k <= WARP; k <<= 1) {
+        uint32_t const flip = (lane & k) ? 0xFFFFFFFFu : 0u, change = flip ^ flipped;
+        v ^= (uint64_t(change) << 32) | change;
+        flipped = flip;
 #pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            uint64_t const o = shfl64_xor(v, j);
-            bool const keep_max = ((lane & j) == 0) == ((lane & k) == 0);   // descending runs where lane & k == 0
-            v = keep_max ? (v > o ? v : o) : (v < o ? v : o);
-        }
+        for (int j = k >> 1; j > 0; j >>= 1) v = keep_larger_low(v, j, lane);
     }
     return v;
 }
@@ -447,12 +454,15 @@ __device__ __forceinline__ uint64_t merge_topk(uint64_t a, uint64_t b, int kl, i
     uint64_t const rb = shfl64(b, 31 - lane);                    // ascending
     uint64_t c = a > rb ? a : rb;                                // bitonic, holds the 32 largest of both
 #pragma unroll
-    for (int j = 16; j > 0; j >>= 1) {
-        uint64_t const o = shfl64_xor(c, j);
-        bool const lower = (lane & j) == 0;
-        c = lower ? (c > o ? c : o) : (c < o ? c : o);
-    }
+    for (int j = 16; j > 0; j >>= 1) c = keep_larger_low(c, j, lane);
     return lane < kl ? c : 0ull;
+}
+
+// One unsorted key per lane into the warp's sorted list, in straight-line code (team kernels). Not inlined:
+// the level pass and expand_copies share one copy (a team's move at 4 games per SM takes 75 us with it, 85 us
+// with a copy at each: instruction fetch).
+__device__ __noinline__ uint64_t merge_keys_fast(uint64_t list, uint64_t v, int kl, int lane) {
+    return merge_topk(list, warp_sort_desc(v, lane), kl, lane);
 }
 
 // One unsorted key per lane into the warp's sorted list: a bitonic sort (k = 2 .. 32), then the two
@@ -841,7 +851,7 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
             if (fin || kcnt + n > uint32_t(WARP)) {          // merge the buffer into the list
                 __syncwarp();
                 uint64_t const b = uint32_t(lane) < kcnt ? kb[lane] : 0ull;
-                acc.list = TEAMED ? merge_topk(acc.list, warp_sort_desc(b, lane), kl, lane) : merge_keys(acc.list, b, kl, lane);
+                acc.list = TEAMED ? merge_keys_fast(acc.list, b, kl, lane) : merge_keys(acc.list, b, kl, lane);
                 acc.thr = shfl64(acc.list, kl - 1);
                 kcnt = 0;
                 m = __ballot_sync(FULL_MASK, key > acc.thr);
@@ -984,7 +994,7 @@ __device__ __noinline__ uint64_t expand_copies(WarpShared const* ws, uint64_t li
             else c1 &= c1 - 1u;
             copy = (key & 0xFFFFFFFF00000000ull) | uint64_t(0xFFFFFFFFu - pos);
         }
-        if (SORTED) list = merge_topk(list, warp_sort_desc(copy, lane), kl, lane);
+        if (SORTED) list = merge_keys_fast(list, copy, kl, lane);
         else topk_fold(list, thr, copy, kl, lane);
     }
     return list;
@@ -1085,10 +1095,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             }
             __syncwarp();
         } else {
-            // teams of four share a pass's rounds, but not the serial grouping and copying (5 us a move
-            // against the 5 us that the copies' rounds take there: 18.3 against 17.9 ms for 30 champion
-            // games), so they evaluate every list
-            dedup = !KEYS && TEAM < 4 && (stage > 1 || p0 == p1);
+            dedup = !KEYS && (stage > 1 || p0 == p1);
             total = build_segments(ws, slot_piece, tree, stage, fnode, kept, dedup, lane, evals);
         }
         if (TEAMED && !partner) {                // post the stage
