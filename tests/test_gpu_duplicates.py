@@ -67,3 +67,19 @@ def test_tied_widened_models_match_the_oracle(oracle, hidden):
     seeds = np.arange(7, 9, dtype=np.uint64)
     with ModelEvaluator(device=0) as ev:
         assert _device(ev, w, seeds) == _oracle(oracle, w, (hidden, hidden), seeds)
+
+
+def test_large_widened_batch_plays_the_small_ones_games():
+    """Width 32 has a launch shape of its own for large batches (at least four games per slot of 12 warps
+    an SM): the same games as batches below that, bit for bit."""
+    from tetris_ai3_b200 import ModelEvaluator, workload
+    b = workload.wide_batch(islands=1, pop=80, games=90, max_moves=6, hidden=32)
+    with ModelEvaluator(device=0) as ev:
+        assert b.sims >= 4 * 12 * ev.launch_info()["sms"]
+        many = ev.eval_full(b.weights, b.models, b.seeds, b.max_moves)
+        assert ev.launch_info()["warps_per_block"] == 12
+        for m in (0, 41, 79):
+            few = ev.eval_full(b.weights[m:m + 1], 1, b.seeds, b.max_moves)
+            assert ev.launch_info()["warps_per_block"] == 4
+            for x, y in zip(many, few):
+                assert x[m * 90:(m + 1) * 90].tobytes() == y.tobytes()

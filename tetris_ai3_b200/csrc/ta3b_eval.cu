@@ -272,124 +272,128 @@ __device__ __forceinline__ int fast_candidate(uint32_t const* __restrict__ rec, 
 }
 
 // ------------------------------------------------ widened network (device) ---
-// One lane = one candidate; the warp's lanes run the network together so that a
-// term can be left out when its input is exactly zero in every lane. That is
+// A lane takes two candidates, and the warp's lanes run the network together: every 16-byte load of weights
+// serves 64 candidates (a load that all lanes share still takes four cycles of the L1 data path, as much as
+// four packed operations of the FP32 pipes; with one candidate a lane that path was 54 % busy and the FP32
+// pipes 33 %), and a term can be left out when its input is exactly zero in all of them. That is
 // exact: x + (±0 * w) == x for finite w and every x but -0, and a sum that starts
 // from a bias other than -0 is never -0 (under round-to-nearest a sum is -0 only
 // for (-0) + (-0)). repack_wide_kernel sets WIDE_SKIP for models whose weights
 // are all finite and whose biases are not -0; every other model runs every term.
 // Each unit's sum keeps the reference order (utility.hpp:30-46: bias, then the
-// inputs ascending), only without the zero terms. Lanes without a candidate pass
-// zero inputs. hb: this warp's hidden-unit buffer, [unit][lane] floats (no bank conflicts).
-struct WideIn {
-    float v[NIN];
-};
+// inputs ascending), only without the zero terms. Candidates that are not there pass
+// zero inputs. hb: this warp's buffer, [input or hidden unit][lane] pairs of floats, a pair per lane's two
+// candidates: the inputs, then over them the hidden units (no lane reads another's).
 template <int H>
-constexpr int kWideHbFloats = H * WARP;                // per warp: H units x 32 lanes (8 KB for 64)
+constexpr int kWideHbFloats = H * 2 * WARP;            // per warp: H units x 64 candidates (16 KB for 64)
 
-// four units' sums += x * q: the products as two packed multiplies (each half rounded like the
-// scalar multiply), the additions scalar, so that no multiply is fused into an add
-__device__ __forceinline__ void wide_fold4(float* a, float2 x, float4 q) {
-    float2 const p01 = f2_mul(x, make_float2(q.x, q.y));
-    float2 const p23 = f2_mul(x, make_float2(q.z, q.w));
-    a[0] = f_add(a[0], p01.x);
-    a[1] = f_add(a[1], p01.y);
-    a[2] = f_add(a[2], p23.x);
-    a[3] = f_add(a[3], p23.y);
+// four units' sums (two pairs) of one candidate += x * q: packed multiplies as fused multiply-adds of -0 and
+// packed adds, each half rounded like the scalar operations (eval_core.h, MLP_X2FMA)
+__device__ __forceinline__ void wide_fold4(float2* a, float2 x, float4 q, float2 nz) {
+    a[0] = f2_add(a[0], f2_fma(x, make_float2(q.x, q.y), nz));
+    a[1] = f2_add(a[1], f2_fma(x, make_float2(q.z, q.w), nz));
 }
 
+// Measured (start -> two candidates a lane with the weights fetched ahead): 2,000 games of width 64 at cap 200
+// 405 -> 233 ms, of width 32 at cap 300 248 -> 147 ms (335 and 194 with one candidate a lane and distinct lists);
+// FP32 pipes 33 -> 48 % busy. The rest is 6 warps an SM in the level's other phases.
 template <int H>
-__device__ __noinline__ float wide_value(WideIn in, float const* __restrict__ w, float* __restrict__ hb, int lane) {
-    static_assert(H >= 4 && H <= 64 && H % 4 == 0, "the hidden-unit masks hold 64 units");
+__device__ __noinline__ float2 wide_value(float const* __restrict__ w, float2* __restrict__ hb, int lane, float neg_zero) {
+    static_assert(H == 32 || H == 64, "a row of weights is one or two floats a lane");
     using D = WideNet<H>;
+    float2 const nz = make_float2(neg_zero, neg_zero);
     uint32_t const skip = __ldg(reinterpret_cast<uint32_t const*>(w) + D::SKIP);
-    float a[H];
-#pragma unroll
-    for (int o = 0; o < H; o += 4) {
-        float4 const b = __ldg(reinterpret_cast<float4 const*>(w + D::B1 + o));
-        a[o] = b.x; a[o + 1] = b.y; a[o + 2] = b.z; a[o + 3] = b.w;
-    }
-    // layer 1, one input at a time over all 64 units (inputs that are zero in every lane skipped)
+    float2* const own = hb + lane;
     uint32_t inz = 0;
 #pragma unroll
-    for (int i = 0; i < NIN; ++i) inz |= in.v[i] != 0.0f ? 1u << i : 0u;
-    inz = skip ? __reduce_or_sync(FULL_MASK, inz) : (1u << NIN) - 1u;
-#pragma unroll
     for (int i = 0; i < NIN; ++i) {
-        if (!((inz >> i) & 1u)) continue;
-        float4 const* wr = reinterpret_cast<float4 const*>(w + D::W1T + i * H);
-        float2 const x = make_float2(in.v[i], in.v[i]);
+        float2 const x = own[i * WARP];
+        inz |= x.x != 0.0f || x.y != 0.0f ? 1u << i : 0u;
+    }
+    uint64_t m = skip ? __reduce_or_sync(FULL_MASK, inz) : (1u << NIN) - 1u;
+    float2 a[H / 2], b[H / 2];                    // the two candidates' units (2k, 2k + 1)
+    // layers 1 and 2 through one body: one input (then hidden unit) at a time over all H units
+#pragma unroll 1
+    for (int layer = 0;; ++layer) {
+        float const* const bias = w + (layer ? D::B2 : D::B1);
+        float const* const wt = w + (layer ? D::W2T : D::W1T);
 #pragma unroll
         for (int o = 0; o < H; o += 4) {
-            float4 const q = __ldg(wr + o / 4);
-            wide_fold4(a + o, x, q);
+            float4 const q = __ldg(reinterpret_cast<float4 const*>(bias + o));
+            a[o / 2] = b[o / 2] = make_float2(q.x, q.y);
+            a[o / 2 + 1] = b[o / 2 + 1] = make_float2(q.z, q.w);
         }
-    }
-    // ReLU into the buffer; nz = the units that are non-zero in some lane
-    uint32_t nz[2] = {0u, 0u};
+        // An input's row of weights (H floats) waits in the buffer: the lanes fetch it two inputs ahead, a share
+        // each, and store it over the row of the input before it, which every lane has read by then. (The
+        // first row is read from global memory.)
+        auto next = [&]() {                       // the next input, or the last one again
+            int const n = m ? __ffsll(static_cast<long long>(m)) - 1 : -1;
+            m &= m - 1;
+            return n;
+        };
+        auto fetch = [&](int i) {
+            if constexpr (H == 64) return __ldg(reinterpret_cast<float2 const*>(wt + i * H) + lane);
+            else return make_float2(__ldg(wt + i * H + lane), 0.0f);
+        };
+        int i = next(), i1 = next();
+        float4 const* row = reinterpret_cast<float4 const*>(wt + i * H);
+        float2 ahead = fetch(i1 < 0 ? 0 : i1);
+#pragma unroll 1
+        while (i >= 0) {
+            float2 const x = own[i * WARP], xa = make_float2(x.x, x.x), xb = make_float2(x.y, x.y);
+            int const i2 = next();
+            float2* const home = hb + i * WARP;
+            __syncwarp();                         // every lane has its x; the row of this input's weights is complete
+            if constexpr (H == 64) home[lane] = ahead;
+            else reinterpret_cast<float*>(home)[lane] = ahead.x;
+            ahead = fetch(i2 < 0 ? 0 : i2);
 #pragma unroll
-    for (int o = 0; o < H; o += 4) {
-        float4 const h = make_float4(relu(a[o]), relu(a[o + 1]), relu(a[o + 2]), relu(a[o + 3]));
-        float* const hq = hb + lane;
-        hq[(o + 0) * WARP] = h.x;
-        hq[(o + 1) * WARP] = h.y;
-        hq[(o + 2) * WARP] = h.z;
-        hq[(o + 3) * WARP] = h.w;
-        uint32_t const bits = (h.x != 0.0f ? 1u : 0u) | (h.y != 0.0f ? 2u : 0u) | (h.z != 0.0f ? 4u : 0u) |
-                              (h.w != 0.0f ? 8u : 0u);
-        nz[o >> 5] |= bits << (o & 31);
-    }
-    if (skip) {
-        nz[0] = __reduce_or_sync(FULL_MASK, nz[0]);
-        nz[1] = __reduce_or_sync(FULL_MASK, nz[1]);
-    } else {
-        nz[0] = nz[1] = ~0u;
-    }
-    // layer 2, one hidden unit at a time over all 64 outputs
-#pragma unroll
-    for (int o = 0; o < H; o += 4) {
-        float4 const b = __ldg(reinterpret_cast<float4 const*>(w + D::B2 + o));
-        a[o] = b.x; a[o + 1] = b.y; a[o + 2] = b.z; a[o + 3] = b.w;
-    }
-    float const* hs = hb + lane;
-    uint64_t m = (uint64_t(nz[1]) << 32) | nz[0];
-    if (H < 64) m &= (uint64_t(1) << (H & 63)) - 1u;         // only the H units that exist
-    while (m) {
-        int const i = __ffsll(static_cast<long long>(m)) - 1;
-        m &= m - 1;
-        float2 const x = make_float2(hs[i * WARP], hs[i * WARP]);
-        float4 const* wr = reinterpret_cast<float4 const*>(w + D::W2T + i * H);
-#pragma unroll
-        for (int o = 0; o < H; o += 4) {
-            float4 const q = __ldg(wr + o / 4);
-            wide_fold4(a + o, x, q);
+            for (int o = 0; o < H; o += 4) {
+                float4 const q = row[o / 4];
+                wide_fold4(a + o / 2, xa, q, nz);
+                wide_fold4(b + o / 2, xb, q, nz);
+            }
+            row = reinterpret_cast<float4 const*>(home);
+            i = i1;
+            i1 = i2;
         }
+        if (layer == 1) break;
+        __syncwarp();                             // (the last row of weights has been read)
+        // ReLU into the buffer; live = the units that are non-zero in some candidate
+        uint32_t live[2] = {0u, 0u};
+#pragma unroll
+        for (int o = 0; o < H; ++o) {
+            float2 const h = o & 1 ? make_float2(relu(a[o / 2].y), relu(b[o / 2].y)) : make_float2(relu(a[o / 2].x), relu(b[o / 2].x));
+            own[o * WARP] = h;
+            live[o >> 5] |= h.x != 0.0f || h.y != 0.0f ? 1u << (o & 31) : 0u;
+        }
+        if (skip) {
+            live[0] = __reduce_or_sync(FULL_MASK, live[0]);
+            live[1] = __reduce_or_sync(FULL_MASK, live[1]);
+        } else {
+            live[0] = live[1] = ~0u;
+        }
+        m = (uint64_t(live[1]) << 32) | live[0];
+        if (H < 64) m &= (uint64_t(1) << (H & 63)) - 1u;         // only the H units that exist
     }
     // layer 3: every term, ascending
-    float out = __ldg(w + D::B3);
+    float const b3 = __ldg(w + D::B3);
+    float2 out = make_float2(b3, b3);
 #pragma unroll
     for (int o = 0; o < H; o += 4) {
         float4 const q = __ldg(reinterpret_cast<float4 const*>(w + D::W3 + o));
-        float2 const t01 = f2_mul(make_float2(relu(a[o]), relu(a[o + 1])), make_float2(q.x, q.y));
-        float2 const t23 = f2_mul(make_float2(relu(a[o + 2]), relu(a[o + 3])), make_float2(q.z, q.w));
-        out = f_add(out, t01.x);
-        out = f_add(out, t01.y);
-        out = f_add(out, t23.x);
-        out = f_add(out, t23.y);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            float2 const wk = k ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
+            float2 const ta = f2_mul(make_float2(relu(a[o / 2 + k].x), relu(a[o / 2 + k].y)), wk);
+            float2 const tb = f2_mul(make_float2(relu(b[o / 2 + k].x), relu(b[o / 2 + k].y)), wk);
+            out.x = f_add(out.x, ta.x);
+            out.x = f_add(out.x, ta.y);
+            out.y = f_add(out.y, tb.x);
+            out.y = f_add(out.y, tb.y);
+        }
     }
     return out;
-}
-
-// fast path of the widened network: the same record words; every lane of the warp calls it
-template <int H>
-__device__ __forceinline__ int fast_candidate_wide(uint32_t const* __restrict__ rec, PlaceFast pf, bool held_i,
-                                                   float const* __restrict__ w, float* hb, int lane, float& v) {
-    RecView r;
-    load_view(rec, pf, r);
-    WideIn in;
-    bool const defer = fast_wide_inputs(r, rec[R_CLEARS], pf, held_i, in.v);
-    v = wide_value<H>(in, w, hb, lane);
-    return defer ? FAST_DEFER : FAST_OK;
 }
 
 // stats_v4::advance (tetris_stats.hpp:19-23 with metrics.hpp:196-229); bi: the board's metrics
@@ -555,7 +559,7 @@ struct alignas(16) WarpShared {
     Stats st;
     uint32_t illegal[16];              // per segment (a byte each) its placements that turned out illegal
     uint16_t seg_of[K2];               // per parent its lists' segments, list 1's << 8
-    uint16_t defer[64];                // queued (segment << 8 | flat placement index) for the full path
+    uint16_t defer[4 * WARP];          // queued (segment << 8 | flat placement index) for the full path
     // ---- the widened networks' warp areas end here (kWideWarpBytes)
     alignas(16) float wfull[NPARAMS + 3];   // the v11 model's weights (full path, record partial sums)
     alignas(8) uint64_t kbuf[WARP];    // a level's keys above the top-K threshold, not yet merged
@@ -682,10 +686,13 @@ __device__ __forceinline__ void warp_top2(uint64_t& b1, uint64_t& b2) {
     }
 }
 
+// a candidate's position in its level (beam.hpp:296,360,423) and its key (beam.hpp:217-219)
+__device__ __forceinline__ uint32_t seg_pos(uint32_t info, uint32_t i) { return ((info >> 8) & 63u) * MP + i; }
+__device__ __forceinline__ uint64_t position_key(bool leaf, float v, uint32_t pos) {
+    return (uint64_t(ordered_bits(v)) << 32) | uint64_t((leaf ? uint32_t(ORDER_SPAN) : 0xFFFFFFFFu) - pos);
+}
 __device__ __forceinline__ uint64_t candidate_key(bool leaf, float v, uint32_t info, uint32_t i) {
-    uint32_t const pos = ((info >> 8) & 63u) * MP + i;                     // beam.hpp:296,360,423
-    uint32_t const low = (leaf ? uint32_t(ORDER_SPAN) : 0xFFFFFFFFu) - pos;       // beam.hpp:217-219
-    return (uint64_t(ordered_bits(v)) << 32) | uint64_t(low);
+    return position_key(leaf, v, seg_pos(info, i));
 }
 __device__ __forceinline__ uint32_t seg_flat(uint32_t info) { return (info >> 16) & 0xFFu; }   // piece * MP
 __device__ __forceinline__ bool seg_held(uint32_t info) { return (info >> 24) & 1u; }
@@ -723,16 +730,117 @@ __device__ __noinline__ uint64_t full_key(WarpShared* ws, Luts lut, bool leaf, u
     return candidate_key(leaf, v, info, flat - seg_flat(info));
 }
 
-// The widened network's full path, first half: is the queued candidate legal,
-// and its inputs (all zero when it is not).
-__device__ __noinline__ bool full_inputs_wide(WarpShared* ws, Luts lut, uint32_t entry, WideIn& in) {
+// The widened network's inputs of one queued candidate by the full path into its column of the warp's buffer
+// (zeros when it is illegal): its position, or -1.
+__device__ __forceinline__ void store_wide_inputs(float* column, float const (&in)[NIN]) {
+#pragma unroll
+    for (int i = 0; i < NIN; ++i) column[i * 2 * WARP] = in[i];
+}
+__device__ __noinline__ int full_inputs_wide(WarpShared* ws, Luts lut, uint32_t entry, float* column, uint32_t& evals) {
     uint32_t const info = ws->seg[entry >> 8].y, flat = entry & 0xFFu;
     uint32_t const* rec = ws->rec[info & 63u];
     uint32_t const mv = lut.move[flat];
     Applied const a = apply_ints(rec + R_BOARD, mv & 0xFFFFu, int((mv >> 16) & 0xFu), nullptr);
-    if (!a.legal) return false;
-    wide_inputs(rec[R_CLEARS] + clear_bump(a.cleared), a.bi, seg_held(info), in.v);
-    return true;
+    float in[NIN] = {};
+    int pos = -1;
+    if (a.legal) {
+        wide_inputs(rec[R_CLEARS] + clear_bump(a.cleared), a.bi, seg_held(info), in);
+        pos = int(seg_pos(info, flat - seg_flat(info)));
+    } else {
+        count_illegal(ws, entry >> 8, info, evals);
+    }
+    store_wide_inputs(column, in);
+    return pos;
+}
+
+// keys of a round above the threshold from which one sort and merge (260 instructions) beats inserting each
+// (20 and a chain of shuffles)
+constexpr int kMergeAbove = 10;
+
+// One level of the widened network: rounds of 64 candidates, two a lane, by the fast path, or (once 64 are
+// queued, or at the level's end) 64 queued ones by the full path; either way the inputs go to the warp's
+// buffer and one call evaluates them. The keys enter the list at once.
+template <int H, bool KEYS>
+__device__ __forceinline__ LevelAcc level_pass_wide(WarpShared& ws, Luts lut, float neg_zero, float* hb, bool leaf,
+                                                    uint32_t total, int kl, int lane, uint32_t& evals) {
+    constexpr uint32_t BATCH = 2 * WARP;
+    uint16_t* const dq = ws.defer;
+    LevelAcc acc{0, 0, 0, 0};
+    uint32_t queued = 0;                   // < 64 at the start of every fast round: the queue holds 128
+    uint32_t c0 = 0;
+    int seg = -1;
+    uint2 sg = make_uint2(0u, 0u);         // this lane's segment (none yet)
+    for (;;) {
+        bool const more = c0 < total;
+        if (!more && queued == 0) break;
+        bool const drain = queued >= BATCH || !more;
+        uint32_t const n = queued < BATCH ? queued : BATCH;
+        int pos[2] = {-1, -1};             // the lane's candidates' positions, -1 = none
+        __syncwarp();
+#pragma unroll 1
+        for (int r = 0; r < 2; ++r) {
+            float* const column = hb + 2 * lane + r;
+            int at = -1;
+            if (drain) {
+                uint32_t const e = uint32_t(r * WARP + lane);
+                if (e < n) {
+                    at = full_inputs_wide(&ws, lut, dq[e], column, evals);
+                } else {
+                    float const none[NIN] = {};
+                    store_wide_inputs(column, none);
+                }
+            } else {
+                uint32_t const c = c0 + uint32_t(r * WARP + lane);
+                bool const valid = c < total;
+                uint32_t const cc = valid ? c : total - 1u;      // out of range: the last candidate, discarded
+                while ((sg.x >> 16) <= cc) sg = ws.seg[++seg];
+                uint32_t const info = sg.y;
+                uint32_t const idx = cc - (sg.x & 0xFFFFu), flat = seg_flat(info) + idx;
+                PlaceFast const pf = load_place(lut, flat);
+                uint32_t const* const rec = ws.rec[info & 63u];
+                RecView v;
+                load_view(rec, pf, v);
+                float in[NIN];
+                bool const defer = fast_wide_inputs(v, rec[R_CLEARS], pf, seg_held(info), in);
+                store_wide_inputs(column, in);
+                if (valid && !defer) at = int(seg_pos(info, idx));
+                uint32_t const dm = __ballot_sync(FULL_MASK, valid && defer);
+                if (dm) {
+                    if (valid && defer) dq[queued + __popc(dm & ((1u << lane) - 1u))] = uint16_t((uint32_t(seg) << 8) | flat);
+                    queued += __popc(dm);
+                }
+            }
+            if (r) pos[1] = at;
+            else pos[0] = at;
+        }
+        if (drain) {                       // the entries past the batch move to the front
+            uint32_t const rem = queued - n;
+            __syncwarp();
+            uint32_t const t0 = uint32_t(lane) < rem ? dq[n + lane] : 0u;
+            uint32_t const t1 = uint32_t(lane) + WARP < rem ? dq[n + WARP + lane] : 0u;
+            __syncwarp();
+            if (uint32_t(lane) < rem) dq[lane] = uint16_t(t0);
+            if (uint32_t(lane) + WARP < rem) dq[WARP + lane] = uint16_t(t1);
+            queued = rem;
+        } else {
+            c0 += BATCH;
+        }
+        float2 const v = wide_value<H>(ws.wglobal, reinterpret_cast<float2*>(hb), lane, neg_zero);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            uint64_t const key = pos[r] >= 0 ? position_key(leaf, r ? v.y : v.x, uint32_t(pos[r])) : 0ull;
+            if (leaf) {
+                if (KEYS) top2_insert(acc.best, acc.best2, key);
+                else acc.best = key > acc.best ? key : acc.best;
+            } else if (__popc(__ballot_sync(FULL_MASK, key > acc.thr)) > kMergeAbove) {
+                acc.list = merge_keys(acc.list, key, kl, lane);
+                acc.thr = shfl64(acc.list, kl - 1);
+            } else {
+                topk_fold(acc.list, acc.thr, key, kl, lane);
+            }
+        }
+    }
+    return acc;
 }
 
 // One level: every candidate of the segment table, on the fast path or queued
@@ -754,16 +862,12 @@ __device__ __noinline__ bool full_inputs_wide(WarpShared* ws, Luts lut, uint32_t
 // Measured with this loop, its records and placement data, start -> now: generation 341.6 -> 233.5 ms,
 // default generation 52.4 -> 36.0 ms, 30 champion games 17.9 -> 15.3 ms; 36,800 warp instructions a move of a
 // champion's game at 16 warps per SM (ncu).
-template <int NET, bool KEYS, int TEAM = 1>
-__device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, Luts lut, FastW const& fw, float* hb,
-                                               bool leaf, uint32_t total, int kl, int lane, uint32_t& evals,
-                                               uint32_t first = 0) {
-    constexpr bool WIDE = NET != 0;
-    constexpr int HW = WIDE ? NET : 64;     // the widened network's width (unused for v11)
+template <bool KEYS, int TEAM = 1>
+__device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, Luts lut, FastW const& fw, bool leaf,
+                                               uint32_t total, int kl, int lane, uint32_t& evals, uint32_t first = 0) {
     uint16_t* const dq = own.defer;
     uint64_t* const kb = own.kbuf;
     constexpr bool TEAMED = TEAM > 1;
-    constexpr bool LAZY = !WIDE;
     LevelAcc acc{0, 0, 0, 0};
     // Each iteration is one round of 32 fast-path candidates (one per lane) or, once 32 are
     // queued (or the level is done), one batch of up to 32 deferred candidates through the full
@@ -780,31 +884,14 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
         bool const more = c0 < total;
         // the level's candidates are done; a non-leaf level takes one more turn to merge its buffer
         bool const fin = !more && queued == 0;
-        if (fin && (leaf || !LAZY || kcnt == 0)) break;
+        if (fin && (leaf || kcnt == 0)) break;
         uint64_t key = 0;
         if (fin) {
         } else if (queued >= uint32_t(WARP) || !more) {
             // ---- a batch of deferred candidates through the full reference path
             uint32_t const n = queued < uint32_t(WARP) ? queued : uint32_t(WARP);
             __syncwarp();
-            if constexpr (WIDE) {
-                // the inputs per lane, then the network on all lanes together
-                WideIn in{};
-                uint32_t entry = 0;
-                bool legal = false;
-                if (uint32_t(lane) < n) {
-                    entry = dq[lane];
-                    legal = full_inputs_wide(&ws, lut, entry, in);
-                    if (!legal) in = WideIn{};
-                }
-                __syncwarp();
-                float const v = wide_value<HW>(in, ws.wglobal, hb, lane);
-                if (uint32_t(lane) < n) {
-                    uint32_t const info = ws.seg[entry >> 8].y;
-                    if (legal) key = candidate_key(leaf, v, info, (entry & 0xFFu) - seg_flat(info));
-                    else count_illegal(&ws, entry >> 8, info, evals);
-                }
-            } else if (uint32_t(lane) < n) {
+            if (uint32_t(lane) < n) {
                 uint32_t const entry = dq[lane];
                 key = full_key(&ws, lut, leaf, entry);
                 if (!key) count_illegal(&ws, entry >> 8, ws.seg[entry >> 8].y, evals);
@@ -827,10 +914,7 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
             uint32_t const idx = cc - (sg.x & 0xFFFFu), flat = seg_flat(info) + idx;
             float v;
             int st;
-            if constexpr (WIDE)
-                st = fast_candidate_wide<HW>(ws.rec[info & 63u], load_place(lut, flat), seg_held(info), ws.wglobal, hb, lane, v);
-            else
-                st = fast_candidate(ws.rec[info & 63u], load_place(lut, flat), seg_held(info), fw, v);
+            st = fast_candidate(ws.rec[info & 63u], load_place(lut, flat), seg_held(info), fw, v);
             bool const def = valid && st != FAST_OK;
             if (valid && st == FAST_OK) key = candidate_key(leaf, v, info, idx);
             uint32_t const dm = __ballot_sync(FULL_MASK, def);
@@ -843,8 +927,6 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
         if (leaf) {
             if (KEYS) top2_insert(acc.best, acc.best2, key);
             else acc.best = key > acc.best ? key : acc.best;
-        } else if (!LAZY) {
-            topk_fold(acc.list, acc.thr, key, kl, lane);
         } else {
             uint32_t m = __ballot_sync(FULL_MASK, key > acc.thr);
             uint32_t n = __popc(m);
@@ -1112,8 +1194,11 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
         // registers across the team barriers
         FastW fwl;
         if (TEAMED) load_fast_weights(GlobalW{ws.wglobal}, fwl, fw.nz);
-        LevelAcc a = level_pass<NET, KEYS, TEAM>(ws, pr[rank], lut, TEAMED ? fwl : fw, hb, leaf, total, kl, lane, evals,
-                                                 uint32_t(rank * WARP));
+        LevelAcc a;
+        if constexpr (WIDE)
+            a = level_pass_wide<NET, KEYS>(ws, lut, fw.nz, hb, leaf, total, kl, lane, evals);
+        else
+            a = level_pass<KEYS, TEAM>(ws, pr[rank], lut, TEAMED ? fwl : fw, leaf, total, kl, lane, evals, uint32_t(rank * WARP));
         if (TEAMED) {
             // a partner's results go through its own record area, which it never uses otherwise
             if (partner) {
@@ -1540,18 +1625,23 @@ enum NetKind { NET_V11 = 0, NET_W64 = 1, NET_W32 = 2, NUM_NETS = 3 };
 constexpr int net_width(int ni) { return ni == NET_W64 ? 64 : ni == NET_W32 ? 32 : 0; }
 // dynamic shared memory per warp: its WarpShared block, plus the widened network's hidden-unit buffer
 constexpr size_t warp_bytes(int ni) {
-    return ni == NET_V11 ? sizeof(WarpShared) : kWideWarpBytes + size_t(net_width(ni)) * WARP * sizeof(float);
+    return ni == NET_V11 ? sizeof(WarpShared) : kWideWarpBytes + size_t(net_width(ni)) * 2 * WARP * sizeof(float);
 }
-// the widened networks' launch shapes (more registers per lane than v11): width 64 at 2 blocks
-// of 4 warps per SM (255 registers), width 32 at 3
-Variant const kWideNet[NUM_NETS] = {{nullptr, 0, 0}, {eval_kernel<4, 2, 64>, 4, 2}, {eval_kernel<4, 3, 32>, 4, 3}};
+// the widened networks' launch shapes (more registers per lane than v11, and a buffer of 64 candidates'
+// hidden units per warp): 8 warps an SM
+Variant const kWideNet[NUM_NETS] = {{nullptr, 0, 0}, {eval_kernel<4, 2, 64>, 4, 2}, {eval_kernel<4, 2, 32>, 4, 2}};
+// width 32 with room for 12 warps an SM (168 registers, 20 bytes of spills): better once every slot has
+// several games (16,000 sims, cap 60: 194.6 against 208.7 ms), worse on fewer, where a game's own speed
+// counts (2,000 sims, cap 300: 175.7 against 135.4 ms; 200 sims: 80.0 against 72.4)
+Variant const kWide32Many = {eval_kernel<12, 1, 32>, 12, 1};
+constexpr uint32_t kManyPerSlot = 4;
 // the budget-checking flavours (shapes where the extra check spills nothing)
 Variant const kBudgetNet[NUM_NETS] = {{eval_kernel<4, 3, 0, true>, 4, 3}, {eval_kernel<4, 2, 64, true>, 4, 2},
-                                      {eval_kernel<4, 3, 32, true>, 4, 3}};
+                                      {eval_kernel<4, 2, 32, true>, 4, 2}};
 // the tracing flavours that record each move's two largest keys (without a time budget)
 Variant const kKeysNet[NUM_NETS] = {{eval_kernel<4, 3, 0, false, true>, 4, 3},
                                     {eval_kernel<4, 2, 64, false, true>, 4, 2},
-                                    {eval_kernel<4, 3, 32, false, true>, 4, 3}};
+                                    {eval_kernel<4, 2, 32, false, true>, 4, 2}};
 constexpr int kNoAllocVariant = 1;   // the allocation-free entry point keeps its fixed 4 x 4 launch shape
 constexpr int kSmallVariant = 10;  // the paired kernel: the default for batches of at most 4 games per SM
 constexpr int kResumeVariant = kSmallVariant;   // the team kernel that finishes a hand-off's games
@@ -1593,6 +1683,7 @@ struct ta3b_ctx {
     size_t cap_wpad = 0;
     unsigned long long budget_ns = 0; // per-launch time budget (0 = none)
     uint32_t net_grid[NUM_NETS] = {0, 0, 0};     // widened-network kernels (by NetKind), set up on first use
+    uint32_t wide32_many_grid = 0;               // width 32's kernel for large batches, set up on first use
     uint32_t budget_grid[NUM_NETS] = {0, 0, 0};  // budget flavours (by NetKind), set up on first use
     uint32_t keys_grid[NUM_NETS] = {0, 0, 0};    // key-tracing flavours (by NetKind), set up on first use
     bool auto_small = true;                      // small v11 batches run a team kernel (until a variant is selected)
@@ -1740,13 +1831,18 @@ int launch(ta3b_ctx* ctx, Params const& prm, cudaStream_t st, int ni = NET_V11) 
         if (int rc = setup_kernel(ctx, small, NET_V11, ctx->small_grid, "paired kernel")) return rc;
     if (use_tiny && !ctx->tiny_grid)
         if (int rc = setup_kernel(ctx, tiny, NET_V11, ctx->tiny_grid, "teams-of-four kernel")) return rc;
+    bool const many32 = ni == NET_W32 && !keys && !budget && prm.total_sims >= ctx->sms * kWide32Many.games() * kManyPerSlot;
+    if (many32 && !ctx->wide32_many_grid)
+        if (int rc = setup_kernel(ctx, kWide32Many, ni, ctx->wide32_many_grid, "widened kernel")) return rc;
     Variant const* const v = keys     ? &kKeysNet[ni]
                              : budget ? &kBudgetNet[ni]
+                             : many32 ? &kWide32Many
                              : ni != NET_V11 ? &kWideNet[ni]
                              : use_tiny ? &tiny : use_small ? &small : &kVariants[ctx->variant];
     uint32_t const warps = v->warps, games = v->games();
     uint32_t const max_grid = keys     ? ctx->keys_grid[ni]
                               : budget ? ctx->budget_grid[ni]
+                              : many32 ? ctx->wide32_many_grid
                               : ni != NET_V11 ? ctx->net_grid[ni]
                               : use_tiny ? ctx->tiny_grid : use_small ? ctx->small_grid : ctx->grid;
     // a batch that one block per SM can hold is spread over every SM, one block each (a game runs
