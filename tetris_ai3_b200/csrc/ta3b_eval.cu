@@ -48,19 +48,30 @@ constexpr uint64_t kMaxSims = 0xFFFFFFFFull;
 
 // ---------------------------------------------------------------- tables ---
 struct DevTables {
-    uint32_t nplace[NPIECE];
     uint32_t spawn_cols[NPIECE];
     uint32_t spawn_col0[NPIECE];
     uint32_t shape_cols[NPIECE][4];
     int32_t shape_left[NPIECE][4];
-    // per tree [held_empty][layer][node]: slot | held << 4 | root_hold << 8
+};
+// per tree [held_empty][layer][node]: slot | held << 4 | root_hold << 8 (global: lanes read different nodes)
+struct NodeTables {
     uint32_t node[2][DEPTH][16];
 };
+// placements per piece, 6 bits each
+constexpr uint64_t make_nplace_pack() {
+    uint64_t v = 0;
+    for (int p = 0; p < NPIECE; ++p) v |= uint64_t(TABLES.nplace[p]) << (6 * p);
+    return v;
+}
+constexpr uint64_t NPLACE_PACK = make_nplace_pack();
+__device__ __forceinline__ uint32_t piece_placements(uint32_t piece) { return uint32_t(NPLACE_PACK >> (6u * piece)) & 63u; }
+// The window's pieces (beam.hpp:226-237), a nibble per slot in one register: the held piece, the current one,
+// the preview; nibble HELD_NONE is no piece.
+__device__ __forceinline__ uint32_t slot_piece(uint32_t window, uint32_t slot) { return (window >> (4u * slot)) & 0xFu; }
 
 constexpr DevTables make_dev_tables() {
     DevTables d{};
     for (int p = 0; p < NPIECE; ++p) {
-        d.nplace[p] = TABLES.nplace[p];
         d.spawn_cols[p] = TABLES.spawn_cols[p];
         d.spawn_col0[p] = uint32_t(TABLES.spawn_col0[p]);
         for (int o = 0; o < 4; ++o) {
@@ -68,6 +79,10 @@ constexpr DevTables make_dev_tables() {
             d.shape_left[p][o] = TABLES.shape_left[p][o];
         }
     }
+    return d;
+}
+constexpr NodeTables make_node_tables() {
+    NodeTables d{};
     for (int he = 0; he < 2; ++he)
         for (int l = 0; l < DEPTH; ++l)
             for (int n = 0; n < 16; ++n) {
@@ -78,6 +93,10 @@ constexpr DevTables make_dev_tables() {
 }
 
 __constant__ DevTables c_tables = make_dev_tables();
+__device__ NodeTables const g_nodes = make_node_tables();
+__device__ __forceinline__ uint32_t tree_node(int tree, int level, uint32_t node) {
+    return __ldg(&g_nodes.node[tree][level][node]);
+}
 
 // Placement tables copied into shared memory per block, indexed piece * MP + placement: the
 // incremental-path data (PlaceFast, its two vectors apart so that consecutive lanes' 16-byte
@@ -718,6 +737,17 @@ __device__ __forceinline__ void count_illegal(WarpShared* ws, uint32_t seg, uint
     evals -= seg_lists(info);
 }
 
+// The root stage's candidate c (two segments) as a queue entry. In team kernels the root's at most 68
+// candidates go through the full path without a record: a batch of it per warp takes less time than a fast
+// round, the batch of what that defers and the record that the leader's one lane builds (30 champion games 14.5
+// against 15.1 ms). With 16 warps an SM the instructions count, not the time of one warp: there the record
+// stays (a generation takes 245 ms with it, 248 without).
+__device__ __forceinline__ uint32_t root_entry(WarpShared const& ws, uint32_t c) {
+    uint32_t const n0 = ws.seg[0].x >> 16;
+    uint32_t const s = c >= n0 ? 1u : 0u;
+    return (s << 8) | (seg_flat(ws.seg[s].y) + c - (s ? n0 : 0u));
+}
+
 // Full path for one queued candidate (segment << 8 | flat placement index): its key, or 0 if illegal.
 // A legal candidate's key is never 0 (its low word is a positive position).
 __device__ __noinline__ uint64_t full_key(WarpShared* ws, Luts lut, bool leaf, uint32_t entry) {
@@ -864,7 +894,8 @@ __device__ __forceinline__ LevelAcc level_pass_wide(WarpShared& ws, Luts lut, fl
 // champion's game at 16 warps per SM (ncu).
 template <bool KEYS, int TEAM = 1>
 __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, Luts lut, FastW const& fw, bool leaf,
-                                               uint32_t total, int kl, int lane, uint32_t& evals, uint32_t first = 0) {
+                                               uint32_t total, int kl, int lane, uint32_t& evals, bool root,
+                                               uint32_t first = 0) {
     uint16_t* const dq = own.defer;
     uint64_t* const kb = own.kbuf;
     constexpr bool TEAMED = TEAM > 1;
@@ -887,6 +918,15 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
         if (fin && (leaf || kcnt == 0)) break;
         uint64_t key = 0;
         if (fin) {
+        } else if (TEAMED && root && more) {
+            // ---- the root's candidates, in the same rounds, through the full reference path
+            uint32_t const c = c0 + uint32_t(lane);
+            c0 += uint32_t(TEAM * WARP);
+            if (c < total) {
+                uint32_t const entry = root_entry(ws, c);
+                key = full_key(&ws, lut, leaf, entry);
+                if (!key) count_illegal(&ws, entry >> 8, ws.seg[entry >> 8].y, evals);
+            }
         } else if (queued >= uint32_t(WARP) || !more) {
             // ---- a batch of deferred candidates through the full reference path
             uint32_t const n = queued < uint32_t(WARP) ? queued : uint32_t(WARP);
@@ -962,16 +1002,16 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
 // cap 200) 414.8 -> 335.1 ms, widened 32 (cap 300) 243.2 -> 194.0 ms.
 // dedup = false: every list stands for itself (the key-tracing flavour, whose second-best key may be a copy;
 // level 1 unless both root groups place the same piece, the only way to the same board there but for clears).
-__device__ __forceinline__ uint32_t build_segments(WarpShared& ws, uint32_t const* slot_piece, int tree, int level,
+__device__ __forceinline__ uint32_t build_segments(WarpShared& ws, uint32_t window, int tree, int level,
                                                    uint32_t fnode, int kept, bool dedup, int lane, uint32_t& evals) {
     bool const active = lane < kept;
     uint32_t piece[2], held[2];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-        uint32_t const nd = c_tables.node[tree][level][((2u * fnode) & 15u) + uint32_t(c)];
-        piece[c] = slot_piece[nd & 0xFu];
+        uint32_t const nd = tree_node(tree, level, ((2u * fnode) & 15u) + uint32_t(c));
+        piece[c] = slot_piece(window, nd & 0xFu);
         uint32_t const held_slot = (nd >> 4) & 0xFu;
-        held[c] = held_slot != HELD_NONE && slot_piece[held_slot] == 0u;
+        held[c] = slot_piece(window, held_slot) == 0u;
     }
     uint32_t const self = 1u << lane;
     uint32_t m0 = self, m1 = self, merged = 0;
@@ -1002,8 +1042,8 @@ __device__ __forceinline__ uint32_t build_segments(WarpShared& ws, uint32_t cons
         }
         if (v0 == v1) m1 = 0;
     }
-    uint32_t const cnt0 = active && (m0 & (self - 1u)) == 0 ? c_tables.nplace[piece[0]] : 0u;
-    uint32_t const cnt1 = active && m1 && (m1 & (self - 1u)) == 0 ? c_tables.nplace[piece[1]] : 0u;
+    uint32_t const cnt0 = active && (m0 & (self - 1u)) == 0 ? piece_placements(piece[0]) : 0u;
+    uint32_t const cnt1 = active && m1 && (m1 & (self - 1u)) == 0 ? piece_placements(piece[1]) : 0u;
     // candidates (low half) and segments (high half) before this lane's
     uint32_t const own = (cnt0 + cnt1) | ((uint32_t(cnt0 != 0) + uint32_t(cnt1 != 0)) << 16);
     uint32_t incl = own;
@@ -1083,7 +1123,8 @@ __device__ __noinline__ uint64_t expand_copies(WarpShared const* ws, uint64_t li
 }
 
 // lane j builds kept node j (when active): parent record `prec`, placement (piece, i); with
-// root, the active lane builds record 32 from the committed board (no placement, no clears)
+// root, the active lane builds record 32 from the committed board (no placement, no clears). One body for
+// both: the kernel is bound by instruction fetch as much as by issue
 template <bool WIDE>
 __device__ __noinline__ void materialize(WarpShared* ws, Luts lut, bool active, uint32_t prec, uint32_t piece,
                                          uint32_t i, int lane, bool root = false) {
@@ -1105,14 +1146,6 @@ __device__ __noinline__ void materialize(WarpShared* ws, Luts lut, bool active, 
     __syncwarp();
 }
 
-// the committed board's record (record 32): one lane builds it through materialize's body, so the
-// kernel holds one copy of the record builder (a second inlined copy measured 5 % slower on the
-// headline generation: the kernel is bound by instruction fetch as much as by issue)
-template <bool WIDE>
-__device__ __forceinline__ void root_record(WarpShared* ws, Luts lut, int lane) {
-    materialize<WIDE>(ws, lut, lane == 0, 0u, 0u, 0u, lane, true);
-}
-
 // search_move_beam (beam.hpp:484-570) for the warp's committed game.
 // TEAM > 1: ws is the team's game (the leader's area, the partners' follow it). The leader runs
 // the search and posts each stage; a partner stays in here for the whole game, runs the stages it
@@ -1128,19 +1161,18 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
     WarpShared* const pr = &ws;
     Move mv{0, 0, 0, true, 0, 0};
     if (!partner && ws.eng.over) return mv;
-    uint32_t slot_piece[NSLOTS];                                  // beam.hpp:226-237
+    uint32_t window = 0xFu << (4 * HELD_NONE);
     int tree = 0;
     uint32_t r0 = 0, r1 = 0, p0 = 0, p1 = 0;
     if (!partner) {
-        slot_piece[0] = ws.eng.held;
-        slot_piece[1] = ws.eng.queue[0];
+        window |= ws.eng.held | (ws.eng.queue[0] << 4);
 #pragma unroll
-        for (int i = 0; i < DEPTH; ++i) slot_piece[2 + i] = ws.eng.queue[1 + i];
+        for (int i = 0; i < DEPTH; ++i) window |= ws.eng.queue[1 + i] << (8 + 4 * i);
         tree = ws.eng.held == NO_PIECE ? 1 : 0;
-        r0 = c_tables.node[tree][0][0];
-        r1 = c_tables.node[tree][0][1];
-        p0 = slot_piece[r0 & 0xFu];
-        p1 = slot_piece[r1 & 0xFu];
+        r0 = tree_node(tree, 0, 0);
+        r1 = tree_node(tree, 0, 1);
+        p0 = slot_piece(window, r0 & 0xFu);
+        p1 = slot_piece(window, r1 & 0xFu);
     }
 
     int kept = 1;                              // frontier size feeding the next stage
@@ -1161,13 +1193,18 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
         } else if (stage == DEPTH) {
             break;
         } else if (stage == 0) {               // two root groups over the committed board (beam.hpp:283-301)
-            root_record<WIDE>(&ws, lut, lane);
-            uint32_t const n0 = c_tables.nplace[p0];
-            total = n0 + c_tables.nplace[p1];
+            if (TEAMED) {                      // a team's root candidates take the full path: the board and its clears
+                if (lane < W) ws.rec[32][R_BOARD + lane] = ws.eng.board[lane];
+                if (lane == 0) ws.rec[32][R_CLEARS] = 0;
+            } else {
+                materialize<WIDE>(&ws, lut, lane == 0, 0u, 0u, 0u, lane, true);
+            }
+            uint32_t const n0 = piece_placements(p0);
+            total = n0 + piece_placements(p1);
             if (lane < 2) {
                 uint32_t const nd = lane ? r1 : r0;
                 uint32_t const held_slot = (nd >> 4) & 0xFu;
-                uint32_t const held_i = held_slot != HELD_NONE && slot_piece[held_slot] == 0u;
+                uint32_t const held_i = slot_piece(window, held_slot) == 0u;
                 ws.seg[lane] = make_uint2(lane ? n0 | (total << 16) : n0 << 16,
                                           make_seg_info(32u, uint32_t(lane), lane ? p1 : p0, held_i, 1u));
             }
@@ -1178,7 +1215,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             __syncwarp();
         } else {
             dedup = !KEYS && (stage > 1 || p0 == p1);
-            total = build_segments(ws, slot_piece, tree, stage, fnode, kept, dedup, lane, evals);
+            total = build_segments(ws, window, tree, stage, fnode, kept, dedup, lane, evals);
         }
         if (TEAMED && !partner) {                // post the stage
             if (lane == 0) {
@@ -1198,7 +1235,8 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
         if constexpr (WIDE)
             a = level_pass_wide<NET, KEYS>(ws, lut, fw.nz, hb, leaf, total, kl, lane, evals);
         else
-            a = level_pass<KEYS, TEAM>(ws, pr[rank], lut, TEAMED ? fwl : fw, leaf, total, kl, lane, evals, uint32_t(rank * WARP));
+            a = level_pass<KEYS, TEAM>(ws, pr[rank], lut, TEAMED ? fwl : fw, leaf, total, kl, lane, evals, stage == 0,
+                                       uint32_t(rank * WARP));
         if (TEAMED) {
             // a partner's results go through its own record area, which it never uses otherwise
             if (partner) {
@@ -1242,7 +1280,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
             uint32_t const par_node = __shfl_sync(FULL_MASK, fnode, int(pk));
             uint32_t const par_rank = __shfl_sync(FULL_MASK, frank, int(pk));
             uint32_t const cnode = (2u * par_node + child) & 15u;
-            uint32_t const piece = slot_piece[c_tables.node[tree][stage][cnode] & 0xFu];
+            uint32_t const piece = slot_piece(window, tree_node(tree, stage, cnode) & 0xFu);
             materialize<WIDE>(&ws, lut, lane < next, pk, piece, sslot % MP, lane);
             fscore = uint32_t(a.list >> 32);
             fnode = lane < next ? cnode : 0u;
@@ -1287,7 +1325,7 @@ __device__ __forceinline__ Move search_move(WarpShared& ws, Luts lut, FastW cons
     uint32_t const pa = lut.move[(g ? p1 : p0) * uint32_t(MP) + rs % MP];
     mv.orient = int((pa >> 20) & 3u);
     mv.x = int((pa >> 24) & 0xFu) - 2;
-    mv.hold = int((c_tables.node[tree][0][g] >> 8) & 1u);
+    mv.hold = int((tree_node(tree, 0, g) >> 8) & 1u);
     mv.none = ordered_bits_inv(uint32_t(best >> 32)) == -__int_as_float(0x7f800000);   // search.hpp:41
     return mv;
 }
