@@ -736,6 +736,15 @@ __global__ void adam_kernel(float* __restrict__ param, float* __restrict__ m, fl
     store_bf16(i, w, w1b, w2b);
 }
 
+// a pass's gradient (and loss, rows) from the CTA partials, in CTA order
+__global__ void sum_kernel(float const* __restrict__ partial, int nparts, float* __restrict__ out) {
+    int const i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= PARTIAL) return;
+    float g = 0.f;
+    for (int k = 0; k < nparts; ++k) g += partial[size_t(k) * PARTIAL + i];
+    out[i] = g;
+}
+
 // BF16 weight copies from the FP32 parameters
 __global__ void refresh_kernel(float const* __restrict__ param, __nv_bfloat16* __restrict__ w1b,
                                __nv_bfloat16* __restrict__ w2b) {
@@ -781,8 +790,13 @@ struct ta3s_model {
     float* d_y = nullptr;
     int32_t* d_idx = nullptr;
     size_t cap_idx = 0;
-    float* d_out = nullptr;
+    float* d_grad = nullptr;      // [PARTIAL]: a pass's summed gradient, loss and rows
     float* d_stats = nullptr;     // mean[128], inv_std[128]
+    // page-locked and mapped: the status word, then predictions [rows][2], which the kernel writes there
+    // itself (two copies into pageable memory cost a prediction of 800 rows 20 of its 80 us)
+    uint32_t* h_status = nullptr;
+    float* h_out = nullptr;
+    size_t cap_out = 0;
     float* d_corr = nullptr;      // a training call's bias corrections
     size_t cap_corr = 0;
     float y_mean = 0.f, y_std = 1.f;
@@ -816,11 +830,25 @@ int grow(ta3s_model* m, T*& ptr, size_t& cap, size_t n, char const* what) {
     return 0;
 }
 
+// waits for the call's kernels; the status word is zero between calls
 int check_status(ta3s_model* m) {
-    uint32_t st = 0;
-    TA3S_CUDA(m, cudaMemcpyAsync(&st, m->d_status, 4, cudaMemcpyDeviceToHost, m->stream), "status");
+    TA3S_CUDA(m, cudaMemcpyAsync(m->h_status, m->d_status, 4, cudaMemcpyDeviceToHost, m->stream), "status");
     TA3S_CUDA(m, cudaStreamSynchronize(m->stream), "surrogate kernels");
-    if (st) return fail(m, "surrogate: a tensor-core wait timed out");
+    if (*m->h_status) {
+        TA3S_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
+        return fail(m, "surrogate: a tensor-core wait timed out");
+    }
+    return 0;
+}
+
+// page-locked room for n rows' predictions
+int grow_out(ta3s_model* m, size_t n) {
+    if (n <= m->cap_out) return 0;
+    if (m->h_out) cudaFreeHost(m->h_out);
+    m->h_out = nullptr;
+    m->cap_out = 0;
+    TA3S_CUDA(m, cudaHostAlloc(&m->h_out, n * 2 * sizeof(float), cudaHostAllocMapped), "alloc predictions");
+    m->cap_out = n;
     return 0;
 }
 
@@ -833,8 +861,6 @@ int upload_rows(ta3s_model* m, float const* x, uint32_t n, bool standardize) {
         if (grow(m, m->d_xraw, c1, size_t(n) * IN, "alloc rows") || grow(m, m->d_x, c2, size_t(n) * 128, "alloc rows") ||
             grow(m, m->d_y, c3, n, "alloc targets"))
             return 1;
-        size_t c4 = cap;
-        if (grow(m, m->d_out, c4, size_t(n) * 2, "alloc outputs")) return 1;
         m->cap_rows = n;
     }
     TA3S_CUDA(m, cudaMemcpyAsync(m->d_xraw, x, size_t(n) * IN * 4, cudaMemcpyHostToDevice, m->stream), "copy rows");
@@ -855,7 +881,7 @@ Params make_params(ta3s_model* m, int batch, int32_t const* d_idx, int train) {
     prm.w1 = m->d_w1b;
     prm.w2 = m->d_w2b;
     prm.p32 = m->d_param;
-    prm.out = m->d_out;
+    prm.out = m->h_out;
     prm.partial = m->d_partial;
     prm.status = m->d_status;
     prm.inv_batch = 1.0f / float(batch);
@@ -909,7 +935,9 @@ ta3s_model* ta3s_create(int device, uint32_t seed) {
         (e = cudaMalloc(&m->d_w1b, 128 * 128 * 2)) != cudaSuccess ||
         (e = cudaMalloc(&m->d_w2b, 128 * 128 * 2)) != cudaSuccess ||
         (e = cudaMalloc(&m->d_partial, part * 4)) != cudaSuccess || (e = cudaMalloc(&m->d_status, 4)) != cudaSuccess ||
-        (e = cudaMalloc(&m->d_loss, 8)) != cudaSuccess || (e = cudaMalloc(&m->d_stats, 256 * 4)) != cudaSuccess)
+        (e = cudaMalloc(&m->d_loss, 8)) != cudaSuccess || (e = cudaMalloc(&m->d_stats, 256 * 4)) != cudaSuccess ||
+        (e = cudaMalloc(&m->d_grad, PARTIAL * 4)) != cudaSuccess ||
+        (e = cudaHostAlloc(&m->h_status, 16, cudaHostAllocDefault)) != cudaSuccess)
         return bad("alloc", e);
     // He-uniform init for the ReLU layers, small output layer; FP32 master copy
     std::vector<float> w(NPARAM, 0.f);
@@ -942,8 +970,10 @@ void ta3s_destroy(ta3s_model* m) {
     cudaSetDevice(m->device);
     for (void* p : {(void*)m->d_param, (void*)m->d_m, (void*)m->d_v, (void*)m->d_w1b, (void*)m->d_w2b,
                     (void*)m->d_partial, (void*)m->d_status, (void*)m->d_loss, (void*)m->d_xraw, (void*)m->d_x,
-                    (void*)m->d_y, (void*)m->d_idx, (void*)m->d_out, (void*)m->d_stats, (void*)m->d_corr})
+                    (void*)m->d_y, (void*)m->d_idx, (void*)m->d_grad, (void*)m->d_stats, (void*)m->d_corr})
         if (p) cudaFree(p);
+    if (m->h_status) cudaFreeHost(m->h_status);
+    if (m->h_out) cudaFreeHost(m->h_out);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
 }
@@ -1010,20 +1040,13 @@ int ta3s_gradients(ta3s_model* m, float* grad_out, float* loss_out) {
     if (!m || !grad_out) return fail(m, "ta3s_gradients: null argument");
     if (m->rows == 0) return fail(m, "ta3s_gradients: no data");
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
-    TA3S_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
     if (launch_mlp(m, int(m->rows), nullptr, 1)) return 1;
-    if (check_status(m)) return 1;
     int const grid = std::min(int((m->rows + ROWS - 1) / ROWS), m->sms);
-    std::vector<float> part(size_t(grid) * PARTIAL);
-    TA3S_CUDA(m, cudaMemcpy(part.data(), m->d_partial, part.size() * 4, cudaMemcpyDeviceToHost), "partials");
-    for (int i = 0; i < PARTIAL; ++i) {
-        float s = 0.f;
-        for (int k = 0; k < grid; ++k) s += part[size_t(k) * PARTIAL + i];
-        if (i < NPARAM)
-            grad_out[i] = s;
-        else if (i == NPARAM && loss_out)
-            *loss_out = s;
-    }
+    sum_kernel<<<(PARTIAL + 255) / 256, 256, 0, m->stream>>>(m->d_partial, grid, m->d_grad);
+    TA3S_CUDA(m, cudaGetLastError(), "gradient sum");
+    if (check_status(m)) return 1;
+    TA3S_CUDA(m, cudaMemcpy(grad_out, m->d_grad, NPARAM * 4, cudaMemcpyDeviceToHost), "gradients");
+    if (loss_out) TA3S_CUDA(m, cudaMemcpy(loss_out, m->d_grad + NPARAM, 4, cudaMemcpyDeviceToHost), "loss");
     return 0;
 }
 
@@ -1049,7 +1072,6 @@ int ta3s_train(ta3s_model* m, uint32_t epochs, uint32_t batch, float lr, float w
     }
     if (grow(m, m->d_idx, m->cap_idx, std::max<size_t>(total, 1), "alloc indices")) return 1;
     TA3S_CUDA(m, cudaMemcpyAsync(m->d_idx, idx.data(), total * 4, cudaMemcpyHostToDevice, m->stream), "indices");
-    TA3S_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
     AdamConst const ad{lr, 0.9f, 0.999f, 1e-8f, weight_decay};
     uint64_t const steps = uint64_t(epochs) * steps_per_epoch;
     // bias corrections of every step
@@ -1110,11 +1132,8 @@ int ta3s_predict(ta3s_model* m, const float* x, uint32_t n, float* mean_out, flo
     if (n == 0) return 0;
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
     if (upload_rows(m, x, n, false)) return 1;
-    TA3S_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
-    if (launch_mlp(m, int(n), nullptr, 0)) return 1;
-    std::vector<float> out(size_t(n) * 2);
-    TA3S_CUDA(m, cudaMemcpyAsync(out.data(), m->d_out, out.size() * 4, cudaMemcpyDeviceToHost, m->stream), "outputs");
-    if (check_status(m)) return 1;
+    if (grow_out(m, n) || launch_mlp(m, int(n), nullptr, 0) || check_status(m)) return 1;
+    float const* const out = m->h_out;
     for (uint32_t r = 0; r < n; ++r) {
         mean_out[r] = out[2 * r] * m->y_std + m->y_mean;
         if (logvar_out) logvar_out[r] = out[2 * r + 1] + 2.f * std::log(m->y_std);
