@@ -64,3 +64,14 @@ def test_training_with_a_ragged_last_minibatch_learns(rows, batch):
     s.train(x, y, epochs=60, batch=batch)
     assert np.isfinite(s.params).all() and np.isfinite(s.last_loss)
     assert so.spearman(s.predict(held), true) > 0.5
+
+
+@pytest.mark.parametrize("rows,batch", [(100, 1200), (300, 5000)])
+def test_minibatch_larger_than_the_rows(rows, batch):
+    """A minibatch is never larger than the rows there are, however large the argument (here beyond the eight
+    tiles that a cluster holds): one step an epoch over the same shuffle, so the results are bit-identical."""
+    x, y = _data(rows)
+    a, b = _model(), _model()
+    a.train(x, y, epochs=3, batch=batch, standardized=True)
+    b.train(x, y, epochs=3, batch=rows, standardized=True)
+    assert a.params.tobytes() == b.params.tobytes() and a.last_loss == b.last_loss

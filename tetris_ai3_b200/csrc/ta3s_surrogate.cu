@@ -650,7 +650,9 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS, 1) tr
     };
     auto tiles = [](Params const& p) { return (p.batch + ROWS - 1) / ROWS; };
     Params p = minibatch(0);
-    int const most = tiles(a.p);                        // CTAs that ever take a tile: their weights stay in shared memory
+    // CTAs that ever take a tile: their weights stay in shared memory (a minibatch has no more rows than there
+    // are, and the cluster no more CTAs than its tiles were checked for)
+    int const most = (min(a.p.batch, a.rows) + ROWS - 1) / ROWS;
     if (rank < most) b.load_weights(p);
     if (rank < tiles(p)) b.load_rows(p, rank);
     for (int s = 0; s < a.steps; ++s) {
@@ -660,6 +662,8 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS, 1) tr
             b.start();
             b.run_tile(p, rank);
             b.write_partial(p.partial + size_t(rank) * PARTIAL);
+        } else {
+            cp_async_wait();                            // (weights on their way must not land on the update's)
         }
         Params const next = s + 1 < a.steps ? minibatch(s + 1) : p;
         if (s + 1 < a.steps && rank < tiles(next)) b.load_rows(next, rank);     // on their way during the update
