@@ -888,7 +888,7 @@ __device__ __forceinline__ LevelAcc level_pass_wide(WarpShared& ws, Luts lut, fl
 // below the final list[kl-1] too. Team kernels sort in straight-line code (a warp alone on its scheduler
 // waits for every shuffle: 15.4 ms for 30 champion games, 16.9 ms with the loop), the single-warp kernels
 // in a loop (merge_keys: a generation takes 233 ms with it, 238 ms inserting each key at once). The
-// widened kernels insert each key at once (topk_fold; their warp areas have no buffer).
+// widened kernels insert or merge each round's keys at once (level_pass_wide; their warp areas have no buffer).
 // Measured with this loop, its records and placement data, start -> now: generation 341.6 -> 233.5 ms,
 // default generation 52.4 -> 36.0 ms, 30 champion games 17.9 -> 15.3 ms; 36,800 warp instructions a move of a
 // champion's game at 16 warps per SM (ncu).
