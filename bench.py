@@ -69,7 +69,7 @@ LANE_INSTR_PER_PLACEMENT = 358
 # (l1tex__data_pipe_lsu_wavefronts_mem_shared.sum.pct_of_peak_sustained_elapsed).
 NCU_FULL_OCCUPANCY = {"issue_slots_busy": 0.597, "warp_execution_efficiency": 0.881,
                       "shared_memory_throughput": 0.244}
-DRAM_BYTES_PER_LAUNCH = 1_181_184
+DRAM_BYTES_PER_LAUNCH = 776_448
 
 
 from tetris_ai3_b200.dist import rank_env as _dist_env, rank_seed, reduce_timing  # noqa: E402
