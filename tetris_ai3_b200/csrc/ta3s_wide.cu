@@ -161,6 +161,7 @@ struct GemmArgs {
     uint32_t* status;      // bit 0: a tensor-core wait timed out
     __nv_bfloat16 const* mask;   // EPI_MASK: out16 = BF16(mask > 0 ? C : 0), both [M][ldc]
     __nv_bfloat16* out16;        // EPI_MASK; EPI_ADAM: the BF16 copy of the updated weights [M][ldc]
+    int live_n;                  // EPI_ADAM: columns that are weights; the rest is padding, which stays zero
     int mapped;                  // the row map applies (to A's rows, or to B's with B_MN)
 };
 
@@ -318,6 +319,14 @@ __device__ __forceinline__ void gemm_tile(GemmArgs const& g, Adam const& ad, int
                     x.y = ad.step(x.y, mi.y, vi.y, w.y);
                     x.z = ad.step(x.z, mi.z, vi.z, w.z);
                     x.w = ad.step(x.w, mi.w, vi.w, w.w);
+                    // padding: its gradient is a sum of dH1 * 0, which is NaN where dH1 is not finite
+                    if (n0 + TN > g.live_n) {                     // (the row's last tiles: uniform over the CTA)
+                        int const live = g.live_n - (n0 + cc);
+                        if (live < 1) x.x = mi.x = vi.x = 0.f;
+                        if (live < 2) x.y = mi.y = vi.y = 0.f;
+                        if (live < 3) x.z = mi.z = vi.z = 0.f;
+                        if (live < 4) x.w = mi.w = vi.w = 0.f;
+                    }
                     *reinterpret_cast<float4*>(ad.m + at) = mi;
                     *reinterpret_cast<float4*>(ad.v + at) = vi;
                     *reinterpret_cast<float4*>(ad.param + at) = x;
@@ -810,7 +819,7 @@ int pass(ta3w_model* m, __nv_bfloat16 const* x, int32_t const* idx, int valid_ro
     GemmArgs dw1{};
     dw1.a = m->d_dh1b, dw1.lda = h, dw1.b = x, dw1.ldb = d.inp, dw1.map = rows, dw1.mapped = 1;
     dw1.c = m->d_grad + d.w1, dw1.ldc = d.inp, dw1.m = h, dw1.n = d.inp, dw1.k = R, dw1.k_split = R;
-    dw1.status = m->d_status, dw1.out16 = m->d_w1b;
+    dw1.status = m->d_status, dw1.out16 = m->d_w1b, dw1.live_n = d.in;
     SmallGrads const sg{R, h, m->d_dh1b, m->d_dh2b, m->d_h2f, m->d_gcols, m->d_rowloss, m->d_grad,
                         d.w3, d.b1, d.b2, d.b3, m->d_loss};
     int const tiles = (h / TILE) * (d.inp / TN), small = h / 32 + 1;
