@@ -1009,14 +1009,21 @@ int ta3s_get_params(ta3s_model* m, float* params_out) {
 int ta3s_set_data(ta3s_model* m, const float* x, const float* y, uint32_t n) {
     if (!m || !x || !y || n == 0) return fail(m, "ta3s_set_data: need n > 0 rows");
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
-    // per-column standardisation of the inputs (device) and of the target (host), FP64 sums
+    // per-column standardisation of the inputs and of the target, FP64 sums
     double s = 0, s2 = 0;
     for (uint32_t r = 0; r < n; ++r) s += y[r];
     double const mu = s / n;
     for (uint32_t r = 0; r < n; ++r) s2 += (y[r] - mu) * (y[r] - mu);
     m->y_mean = float(mu);
     m->y_std = s2 > 0 ? float(std::sqrt(s2 / n)) : 1.f;
-    if (upload_rows(m, x, n, true)) return 1;
+    bool const host_stats = ta3_stats::stats_on_host(n, IN);
+    std::vector<float> stats(256, 0.f);
+    if (host_stats) {
+        for (int c = 0; c < 128; ++c) stats[128 + c] = 1.f;
+        ta3_stats::host_column_stats(x, n, IN, stats.data(), stats.data() + 128);
+        TA3S_CUDA(m, cudaMemcpyAsync(m->d_stats, stats.data(), 256 * 4, cudaMemcpyHostToDevice, m->stream), "stats");
+    }
+    if (upload_rows(m, x, n, !host_stats)) return 1;
     std::vector<float> ys(n);
     for (uint32_t r = 0; r < n; ++r) ys[r] = (y[r] - m->y_mean) / m->y_std;
     TA3S_CUDA(m, cudaMemcpyAsync(m->d_y, ys.data(), size_t(n) * 4, cudaMemcpyHostToDevice, m->stream), "targets");

@@ -987,6 +987,8 @@ static int set_data_impl(ta3w_model* m, const float* x, const float* y, uint32_t
     std::fill(stats.begin() + d.inp, stats.end(), 1.f);
     m->y_mean = 0.f;
     m->y_std = 1.f;
+    bool const host_stats = standardize && ta3_stats::stats_on_host(n, size_t(d.in));
+    if (host_stats) ta3_stats::host_column_stats(x, n, size_t(d.in), stats.data(), stats.data() + d.inp);
     if (standardize) {
         double s = 0, s2 = 0;
         for (uint32_t r = 0; r < n; ++r) s += y[r];
@@ -997,7 +999,7 @@ static int set_data_impl(ta3w_model* m, const float* x, const float* y, uint32_t
     }
     TA3W_CUDA(m, cudaMemcpyAsync(m->d_stats, stats.data(), stats.size() * 4, cudaMemcpyHostToDevice, m->stream),
               "stats");
-    if (upload_rows(m, x, n, standardize)) return 1;
+    if (upload_rows(m, x, n, standardize && !host_stats)) return 1;
     std::vector<float> ys(n);
     for (uint32_t r = 0; r < n; ++r) ys[r] = (y[r] - m->y_mean) / m->y_std;
     TA3W_CUDA(m, cudaMemcpyAsync(m->d_y, ys.data(), size_t(n) * 4, cudaMemcpyHostToDevice, m->stream), "targets");
