@@ -78,3 +78,8 @@ class Model:
 
     def launches(self, kernel: str) -> int:
         return self.lib.fake_count(kernel.encode())
+
+    def captured(self, dtype, nth: int = 0):
+        """The captured argument's bytes in the nth launch (fake_capture)."""
+        buf = np.zeros(4096, np.uint8)
+        return buf[:self.lib.fake_arg(nth, _p(buf))].view(dtype)

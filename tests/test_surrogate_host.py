@@ -1,6 +1,7 @@
 """The surrogates' host side without a GPU, on a stand-in for the CUDA runtime."""
 from __future__ import annotations
 
+import numpy as np
 import pytest
 
 import fake_cuda
@@ -26,4 +27,26 @@ def test_narrow_or_small_training_sets_take_the_host_statistics(lib, in_dim, row
     lib.fake_reset()
     assert m.set_data(rows) == 0
     assert m.launches("column_stats_kernel") == device
+    m.close()
+
+
+KINDS = [("ta3s", 97), ("ta3w", 97)]
+
+
+@pytest.mark.parametrize("kind,in_dim", KINDS)
+@pytest.mark.parametrize("nth", [0, 1, 2])
+def test_no_memory_for_more_rows_leaves_room_for_none(lib, kind, in_dim, nth):
+    """The buffers of the rows grow one by one, each freed before its larger one is allocated: when one of them
+    fails, fewer rows need fresh buffers too, and no kernel gets a null pointer."""
+    m = fake_cuda.Model(lib, kind, in_dim)
+    assert m.set_data(100) == 0
+    lib.fake_fail(b"cudaMalloc", nth)
+    assert m.set_data(3000) == 1
+    lib.fake_reset()
+    x, out = {"ta3s": (0, 4), "ta3w": (0, 5)}[kind]                 # pack_kernel's rows and result
+    for arg in (x, out):
+        lib.fake_capture(b"pack_kernel", arg, 8)
+        assert m.predict(60) == 0
+        assert m.captured(np.uint64)[0] != 0
+        lib.fake_reset()
     m.close()

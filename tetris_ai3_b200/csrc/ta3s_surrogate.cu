@@ -859,9 +859,9 @@ int grow_out(ta3s_model* m, size_t n) {
 // the rows on the device, standardised in BF16 (with `standardize` by their own statistics, which stay for
 // later predictions)
 int upload_rows(ta3s_model* m, float const* x, uint32_t n, bool standardize) {
-    size_t cap = m->cap_rows;
-    if (n > cap) {
-        size_t c1 = cap, c2 = cap, c3 = cap;
+    if (n > m->cap_rows) {
+        size_t c1 = 0, c2 = 0, c3 = 0;
+        m->cap_rows = 0;      // (grow frees first: after a failure there is no room for any rows)
         if (grow(m, m->d_xraw, c1, size_t(n) * IN, "alloc rows") || grow(m, m->d_x, c2, size_t(n) * 128, "alloc rows") ||
             grow(m, m->d_y, c3, n, "alloc targets"))
             return 1;
