@@ -58,17 +58,19 @@ class Model:
 
     def set_data(self, rows: int, name="set_data"):
         x = np.random.default_rng(rows).standard_normal((rows, self.in_dim), dtype=np.float32)
-        return self.f(name)(self.h, _p(x), _p(x[:, 0].copy()), rows)
+        y = x[:, 0].copy()
+        return self.f(name)(self.h, _p(x), _p(y), rows)
 
     def gradients(self):
-        return self.f("gradients")(self.h, _p(np.zeros(self.nparam, np.float32)), None)
+        g = np.zeros(self.nparam, np.float32)
+        return self.f("gradients")(self.h, _p(g), None)
 
     def train(self, epochs: int, batch: int):
         return self.f("train")(self.h, epochs, batch, 1e-3, 0.0, 0, None)
 
     def predict(self, rows: int):
-        x = np.zeros((rows, self.in_dim), np.float32)
-        return self.f("predict")(self.h, _p(x), rows, _p(np.zeros(rows, np.float32)), None)
+        x, mean = np.zeros((rows, self.in_dim), np.float32), np.zeros(rows, np.float32)
+        return self.f("predict")(self.h, _p(x), rows, _p(mean), None)
 
     # the stand-in
     def log(self) -> list[str]:

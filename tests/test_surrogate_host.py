@@ -50,3 +50,37 @@ def test_no_memory_for_more_rows_leaves_room_for_none(lib, kind, in_dim, nth):
         assert m.captured(np.uint64)[0] != 0
         lib.fake_reset()
     m.close()
+
+
+@pytest.mark.parametrize("kind,in_dim", KINDS)
+@pytest.mark.parametrize("call,rows", [("predict", 40), ("predict", 3000), ("set_data", 40), ("set_data", 3000),
+                                       ("set_data_standardized", 3000)])
+def test_a_failed_call_leaves_no_training_set_behind(lib, kind, in_dim, call, rows):
+    """Prediction rows and a new training set take the old one's place on the device. Whichever runtime call
+    fails on the way, training afterwards is refused, unless nothing had been touched yet."""
+    def run(m):
+        return m.predict(rows) if call == "predict" else m.set_data(rows, call)
+
+    m = fake_cuda.Model(lib, kind, in_dim)
+    assert m.set_data(100) == 0 and m.train(1, 50) == 0
+    lib.fake_reset()
+    assert run(m) == 0
+    steps = m.log()
+    m.close()
+    seen: dict[str, int] = {}
+    for step in steps:
+        nth = seen[step] = seen.get(step, 0) + 1
+        if step in ("cudaFree", "cudaFreeHost"):            # (their results are not looked at)
+            continue
+        m = fake_cuda.Model(lib, kind, in_dim)
+        assert m.set_data(100) == 0 and m.train(1, 50) == 0
+        lib.fake_reset()
+        lib.fake_fail(step.encode(), nth - 1)
+        assert run(m) == 1, (step, nth)
+        untouched = step in ("cudaSetDevice", "cudaHostAlloc")
+        lib.fake_reset()
+        for again in (m.train(1, 50), m.gradients()):
+            assert again == (0 if untouched else 1), (step, nth)
+            assert untouched or "no data" in m.error()
+        assert m.set_data(60) == 0 and m.train(1, 50) == 0   # and a new set is taken
+        m.close()

@@ -857,8 +857,10 @@ int grow_out(ta3s_model* m, size_t n) {
 }
 
 // the rows on the device, standardised in BF16 (with `standardize` by their own statistics, which stay for
-// later predictions)
+// later predictions). They take the place of the training rows, also when it fails half-way: no training
+// set from here until a set_data call is complete.
 int upload_rows(ta3s_model* m, float const* x, uint32_t n, bool standardize) {
+    m->rows = 0;
     if (n > m->cap_rows) {
         size_t c1 = 0, c2 = 0, c3 = 0;
         m->cap_rows = 0;      // (grow frees first: after a failure there is no room for any rows)
@@ -1009,6 +1011,7 @@ int ta3s_get_params(ta3s_model* m, float* params_out) {
 int ta3s_set_data(ta3s_model* m, const float* x, const float* y, uint32_t n) {
     if (!m || !x || !y || n == 0) return fail(m, "ta3s_set_data: need n > 0 rows");
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
+    m->rows = 0;      // (until the call is complete)
     // per-column standardisation of the inputs and of the target, FP64 sums
     double s = 0, s2 = 0;
     for (uint32_t r = 0; r < n; ++r) s += y[r];
@@ -1037,6 +1040,7 @@ int ta3s_set_data_standardized(ta3s_model* m, const float* x, const float* y, ui
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
     std::vector<float> stats(256, 0.f);
     for (int c = 0; c < 128; ++c) stats[128 + c] = 1.f;
+    m->rows = 0;      // (until the call is complete)
     m->y_mean = 0.f;
     m->y_std = 1.f;
     TA3S_CUDA(m, cudaMemcpyAsync(m->d_stats, stats.data(), 256 * 4, cudaMemcpyHostToDevice, m->stream), "stats");
@@ -1142,14 +1146,12 @@ int ta3s_predict(ta3s_model* m, const float* x, uint32_t n, float* mean_out, flo
     if (!m || !x || !mean_out) return fail(m, "ta3s_predict: null argument");
     if (n == 0) return 0;
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
-    if (upload_rows(m, x, n, false)) return 1;
-    if (grow_out(m, n) || launch_mlp(m, int(n), nullptr, 0) || check_status(m)) return 1;
+    if (grow_out(m, n) || upload_rows(m, x, n, false) || launch_mlp(m, int(n), nullptr, 0) || check_status(m)) return 1;
     float const* const out = m->h_out;
     for (uint32_t r = 0; r < n; ++r) {
         mean_out[r] = out[2 * r] * m->y_std + m->y_mean;
         if (logvar_out) logvar_out[r] = out[2 * r + 1] + 2.f * std::log(m->y_std);
     }
-    m->rows = 0;   // the training rows were overwritten: a later train call needs set_data again
     return 0;
 }
 

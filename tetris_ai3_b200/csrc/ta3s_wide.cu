@@ -840,9 +840,11 @@ int check_status(ta3w_model* m) {
 }
 
 // the rows on the device, standardised in BF16 (with `standardize` by their own statistics, which stay for
-// later predictions)
+// later predictions). They take the place of the training rows, also when it fails half-way: no training
+// set from here until a set_data call is complete.
 int upload_rows(ta3w_model* m, float const* x, uint32_t n, bool standardize) {
     Dims const& d = m->d;
+    m->rows = 0;
     if (n > m->cap_rows) {
         size_t c1 = 0, c2 = 0, c3 = 0;
         if (m->d_xraw) cudaFree(m->d_xraw);
@@ -985,6 +987,7 @@ static int set_data_impl(ta3w_model* m, const float* x, const float* y, uint32_t
     TA3W_CUDA(m, cudaSetDevice(m->device), "set device");
     std::vector<float> stats(2 * size_t(d.inp), 0.f);
     std::fill(stats.begin() + d.inp, stats.end(), 1.f);
+    m->rows = 0;      // (until the call is complete)
     m->y_mean = 0.f;
     m->y_std = 1.f;
     bool const host_stats = standardize && ta3_stats::stats_on_host(n, size_t(d.in));
@@ -1094,7 +1097,6 @@ int ta3w_predict(ta3w_model* m, const float* x, uint32_t n, float* mean_out, flo
         mean_out[r] = out[2 * r] * m->y_std + m->y_mean;
         if (logvar_out) logvar_out[r] = out[2 * r + 1] + 2.f * std::log(m->y_std);
     }
-    m->rows = 0;   // the training rows were overwritten: a later train call needs set_data again
     return 0;
 }
 
