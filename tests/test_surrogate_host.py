@@ -1,6 +1,8 @@
 """The surrogates' host side without a GPU, on a stand-in for the CUDA runtime."""
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -84,3 +86,24 @@ def test_a_failed_call_leaves_no_training_set_behind(lib, kind, in_dim, call, ro
             assert untouched or "no data" in m.error()
         assert m.set_data(60) == 0 and m.train(1, 50) == 0   # and a new set is taken
         m.close()
+
+
+def test_a_status_that_no_call_has_read_is_not_the_next_calls(lib):
+    """A bit that a kernel set stays when the call fails before it reads the status (here at the launch behind
+    it); the next call starts from zero."""
+    m = fake_cuda.Model(lib, "ta3s")
+    assert m.set_data(100) == 0 and m.gradients() == 0
+    status = C.cast(lib.fake_block(4), C.POINTER(C.c_uint32))       # the only block of one word
+    lib.fake_reset()
+    for fails, nth, call in (("cudaLaunchKernel", 1, m.gradients), ("cudaMemcpyAsync", 0, m.gradients),
+                             ("cudaStreamSynchronize", 0, m.gradients), ("cudaMemcpyAsync", 2, lambda: m.train(1, 50))):
+        lib.fake_fail(fails.encode(), nth)
+        assert call() == 1
+        status[0] = 1                                                # as the kernel before it would have
+        lib.fake_reset()
+        assert m.gradients() == 0, (fails, m.error())
+        assert status[0] == 0
+    status[0] = 1                                                    # found by the call itself: reported once
+    assert m.gradients() == 1 and "timed out" in m.error()
+    assert m.gradients() == 0
+    m.close()

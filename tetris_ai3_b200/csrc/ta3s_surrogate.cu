@@ -799,6 +799,7 @@ struct ta3s_model {
     // page-locked and mapped: the status word, then predictions [rows][2], which the kernel writes there
     // itself (two copies into pageable memory cost a prediction of 800 rows 20 of its 80 us)
     uint32_t* h_status = nullptr;
+    bool unchecked = false;       // kernels launched whose status no call has found to be zero
     float* h_out = nullptr;
     size_t cap_out = 0;
     float* d_corr = nullptr;      // a training call's bias corrections
@@ -834,14 +835,18 @@ int grow(ta3s_model* m, T*& ptr, size_t& cap, size_t n, char const* what) {
     return 0;
 }
 
-// waits for the call's kernels; the status word is zero between calls
+// the status word is zero between calls; a call that failed between its kernels and check_status may have left a bit
+int begin_kernels(ta3s_model* m) {
+    if (m->unchecked) TA3S_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
+    m->unchecked = true;
+    return 0;
+}
+// waits for the call's kernels
 int check_status(ta3s_model* m) {
     TA3S_CUDA(m, cudaMemcpyAsync(m->h_status, m->d_status, 4, cudaMemcpyDeviceToHost, m->stream), "status");
     TA3S_CUDA(m, cudaStreamSynchronize(m->stream), "surrogate kernels");
-    if (*m->h_status) {
-        TA3S_CUDA(m, cudaMemsetAsync(m->d_status, 0, 4, m->stream), "status");
-        return fail(m, "surrogate: a tensor-core wait timed out");
-    }
+    if (*m->h_status) return fail(m, "surrogate: a tensor-core wait timed out");
+    m->unchecked = false;
     return 0;
 }
 
@@ -1055,7 +1060,7 @@ int ta3s_gradients(ta3s_model* m, float* grad_out, float* loss_out) {
     if (!m || !grad_out) return fail(m, "ta3s_gradients: null argument");
     if (m->rows == 0) return fail(m, "ta3s_gradients: no data");
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
-    if (launch_mlp(m, int(m->rows), nullptr, 1)) return 1;
+    if (begin_kernels(m) || launch_mlp(m, int(m->rows), nullptr, 1)) return 1;
     int const grid = std::min(int((m->rows + ROWS - 1) / ROWS), m->sms);
     sum_kernel<<<(PARTIAL + 255) / 256, 256, 0, m->stream>>>(m->d_partial, grid, m->d_grad);
     TA3S_CUDA(m, cudaGetLastError(), "gradient sum");
@@ -1096,6 +1101,7 @@ int ta3s_train(ta3s_model* m, uint32_t epochs, uint32_t batch, float lr, float w
         corr[k] = 1.f - std::pow(ad.b1, float(m->adam_t));
         corr[steps + k] = 1.f - std::pow(ad.b2, float(m->adam_t));
     }
+    if (begin_kernels(m)) return 1;
     if (std::min(batch, n) <= uint32_t(CLUSTER * ROWS)) {
         // minibatches of one cluster: whole runs of steps in one launch, bounded so that a launch stays short
         constexpr uint64_t kStepsPerLaunch = 4096;
@@ -1146,7 +1152,9 @@ int ta3s_predict(ta3s_model* m, const float* x, uint32_t n, float* mean_out, flo
     if (!m || !x || !mean_out) return fail(m, "ta3s_predict: null argument");
     if (n == 0) return 0;
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
-    if (grow_out(m, n) || upload_rows(m, x, n, false) || launch_mlp(m, int(n), nullptr, 0) || check_status(m)) return 1;
+    if (grow_out(m, n) || upload_rows(m, x, n, false) || begin_kernels(m) || launch_mlp(m, int(n), nullptr, 0) ||
+        check_status(m))
+        return 1;
     float const* const out = m->h_out;
     for (uint32_t r = 0; r < n; ++r) {
         mean_out[r] = out[2 * r] * m->y_std + m->y_mean;
