@@ -107,3 +107,45 @@ def test_a_status_that_no_call_has_read_is_not_the_next_calls(lib):
     assert m.gradients() == 1 and "timed out" in m.error()
     assert m.gradients() == 0
     m.close()
+
+
+def _corrections(m, epochs, batch, rows):
+    """The first and last step's bias correction 1 - 0.999^t of a training call that succeeds."""
+    lib = m.lib
+    if m.kind == "ta3w":                                             # last_kernel's Adam: three pointers, six floats, c2
+        lib.fake_capture(b"last_kernel", 2, 48)
+        assert m.train(epochs, batch) == 0
+        n = m.launches("last_kernel")
+        return m.captured(np.float32, 0)[11], m.captured(np.float32, n - 1)[11]
+    if batch > 1024:                                                 # adam_kernel's c2
+        lib.fake_capture(b"adam_kernel", 7, 4)
+        assert m.train(epochs, batch) == 0
+        n = m.launches("adam_kernel")
+        return m.captured(np.float32, 0)[0], m.captured(np.float32, n - 1)[0]
+    assert m.train(epochs, batch) == 0
+    steps = epochs * -(-rows // batch)
+    c = np.ctypeslib.as_array(C.cast(lib.fake_block(8 * steps), C.POINTER(C.c_float)), (2 * steps,))
+    return c[steps], c[2 * steps - 1]
+
+
+@pytest.mark.parametrize("kind,rows,batch,epochs,fails,nth,done", [
+    ("ta3s", 500, 100, 3, "cudaMalloc", 1, 0),                       # no room for the bias corrections
+    ("ta3s", 500, 100, 3, "cudaLaunchKernel", 0, 0),                 # all 15 steps are one launch
+    ("ta3s", 1, 64, 5000, "cudaLaunchKernel", 1, 4096),              # the second launch of two
+    ("ta3s", 2500, 1100, 3, "cudaLaunchKernel", 6, 3),               # two launches a step
+    ("ta3s", 2500, 1100, 3, "cudaLaunchKernel", 7, 3),
+    ("ta3w", 500, 100, 3, "cudaMalloc", 1, 0),                       # no room for the activations
+    ("ta3w", 500, 100, 3, "cudaLaunchKernelExC", 15, 2)])            # six launches a step
+def test_only_steps_that_ran_count_for_the_bias_corrections(lib, kind, rows, batch, epochs, fails, nth, done):
+    m = fake_cuda.Model(lib, kind)
+    assert m.set_data(rows) == 0
+    lib.fake_reset()
+    lib.fake_fail(fails.encode(), nth)
+    assert m.train(epochs, batch) == 1
+    lib.fake_reset()
+    steps = epochs * -(-rows // batch)
+    first, last = _corrections(m, epochs, batch, rows)
+    b2 = float(np.float32(0.999))
+    assert abs(first - (1 - b2 ** (done + 1))) < 1e-6
+    assert abs(last - (1 - b2 ** (done + steps))) < 1e-6
+    m.close()

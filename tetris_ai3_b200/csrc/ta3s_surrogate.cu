@@ -1097,9 +1097,9 @@ int ta3s_train(ta3s_model* m, uint32_t epochs, uint32_t batch, float lr, float w
     // bias corrections of every step
     std::vector<float> corr(2 * size_t(steps));
     for (uint64_t k = 0; k < steps; ++k) {
-        ++m->adam_t;
-        corr[k] = 1.f - std::pow(ad.b1, float(m->adam_t));
-        corr[steps + k] = 1.f - std::pow(ad.b2, float(m->adam_t));
+        float const t = float(m->adam_t + k + 1);
+        corr[k] = 1.f - std::pow(ad.b1, t);
+        corr[steps + k] = 1.f - std::pow(ad.b2, t);
     }
     if (begin_kernels(m)) return 1;
     if (std::min(batch, n) <= uint32_t(CLUSTER * ROWS)) {
@@ -1127,6 +1127,7 @@ int ta3s_train(ta3s_model* m, uint32_t epochs, uint32_t batch, float lr, float w
             a.loss_out = m->d_loss;
             train_kernel<<<CLUSTER, THREADS, SMEM_BYTES, m->stream>>>(a);
             TA3S_CUDA(m, cudaGetLastError(), "train launch");
+            m->adam_t += uint64_t(a.steps);
         }
     } else {
         for (uint64_t k = 0; k < steps; ++k) {
@@ -1137,6 +1138,7 @@ int ta3s_train(ta3s_model* m, uint32_t epochs, uint32_t batch, float lr, float w
                                                                       corr[k], corr[steps + k], m->d_w1b, m->d_w2b,
                                                                       m->d_loss);
             TA3S_CUDA(m, cudaGetLastError(), "adam launch");
+            ++m->adam_t;
         }
     }
     if (check_status(m)) return 1;

@@ -1064,10 +1064,11 @@ int ta3w_train(ta3w_model* m, uint32_t epochs, uint32_t batch, float lr, float w
     for (uint32_t e = 0; e < epochs; ++e)
         for (uint32_t s = 0; s < steps; ++s) {
             uint32_t const rows_here = std::min(batch, n - s * batch);
-            ++m->adam_t;
-            float const c1 = 1.f - std::pow(b1, float(m->adam_t)), c2 = 1.f - std::pow(b2, float(m->adam_t));
+            float const t = float(m->adam_t + 1);
+            float const c1 = 1.f - std::pow(b1, t), c2 = 1.f - std::pow(b2, t);
             Adam const ad{m->d_param, m->d_m, m->d_v, lr, b1, b2, eps, c1, c2, weight_decay};
             if (pass(m, m->d_x, m->d_idx + (size_t(e) * steps + s) * batch, int(rows_here), true, &ad)) return 1;
+            ++m->adam_t;
             last_rows = rows_here;
         }
     if (check_status(m)) return 1;
