@@ -149,3 +149,17 @@ def test_only_steps_that_ran_count_for_the_bias_corrections(lib, kind, rows, bat
     assert abs(first - (1 - b2 ** (done + 1))) < 1e-6
     assert abs(last - (1 - b2 ** (done + steps))) < 1e-6
     m.close()
+
+
+@pytest.mark.parametrize("batch", [101, 1200, 2**31 - 1, 2**31, 2**32 - 1])
+def test_a_minibatch_larger_than_the_rows_is_all_rows(lib, batch):
+    """Also where the argument does not fit an int, or the sum that rounds the steps up wraps around."""
+    m = fake_cuda.Model(lib, "ta3s")
+    assert m.set_data(100) == 0
+    lib.fake_reset()
+    lib.fake_capture(b"train_kernel", 0, 64)
+    assert m.train(3, batch) == 0
+    assert m.launches("train_kernel") == 1
+    assert m.captured(np.int32)[6] == 100                            # Params: three pointers, then the batch
+    assert lib.fake_block(4 * 3 * 100)                               # the shuffled rows of three epochs, no more
+    m.close()

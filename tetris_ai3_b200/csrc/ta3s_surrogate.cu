@@ -1076,6 +1076,7 @@ int ta3s_train(ta3s_model* m, uint32_t epochs, uint32_t batch, float lr, float w
     if (m->rows == 0) return fail(m, "ta3s_train: no data");
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
     uint32_t const n = m->rows;
+    batch = std::min(batch, n);          // (a minibatch has no more rows than there are, and fits an int)
     uint32_t const steps_per_epoch = (n + batch - 1) / batch;
     size_t const total = size_t(epochs) * steps_per_epoch * batch;
     std::vector<int32_t> idx(total);
@@ -1102,7 +1103,7 @@ int ta3s_train(ta3s_model* m, uint32_t epochs, uint32_t batch, float lr, float w
         corr[steps + k] = 1.f - std::pow(ad.b2, t);
     }
     if (begin_kernels(m)) return 1;
-    if (std::min(batch, n) <= uint32_t(CLUSTER * ROWS)) {
+    if (batch <= uint32_t(CLUSTER * ROWS)) {
         // minibatches of one cluster: whole runs of steps in one launch, bounded so that a launch stays short
         constexpr uint64_t kStepsPerLaunch = 4096;
         if (steps && grow(m, m->d_corr, m->cap_corr, corr.size(), "alloc bias corrections")) return 1;
