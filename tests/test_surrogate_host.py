@@ -163,3 +163,14 @@ def test_a_minibatch_larger_than_the_rows_is_all_rows(lib, batch):
     assert m.captured(np.int32)[6] == 100                            # Params: three pointers, then the batch
     assert lib.fake_block(4 * 3 * 100)                               # the shuffled rows of three epochs, no more
     m.close()
+
+
+@pytest.mark.parametrize("rows,locked", [(800, 1), (262_144, 1), (262_145, 0)])
+def test_page_locked_results_are_bounded(lib, rows, locked):
+    """A model locks at most 2 MB of memory for its predictions; larger ones come through device memory."""
+    m = fake_cuda.Model(lib, "ta3s")
+    lib.fake_reset()
+    assert m.predict(rows) == 0
+    assert m.launches("cudaHostAlloc") == locked
+    assert bool(lib.fake_block(8 * rows)) == (not locked)
+    m.close()

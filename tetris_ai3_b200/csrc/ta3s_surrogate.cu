@@ -802,6 +802,8 @@ struct ta3s_model {
     bool unchecked = false;       // kernels launched whose status no call has found to be zero
     float* h_out = nullptr;
     size_t cap_out = 0;
+    float* d_out = nullptr;       // predictions of more rows than kMappedRows
+    size_t cap_dout = 0;
     float* d_corr = nullptr;      // a training call's bias corrections
     size_t cap_corr = 0;
     float y_mean = 0.f, y_std = 1.f;
@@ -850,6 +852,12 @@ int check_status(ta3s_model* m) {
     return 0;
 }
 
+// Predictions of up to this many rows go into page-locked memory, 8 bytes a row (2 MB at most); more of them through
+// device memory and a copy. Page-locking saves the copy on every call but costs a model's first one: 200,000 rows
+// take 5.7 ms (6.0 with the copy), the first time 7.4 (8.2); 300,000 rows 10.3 (10.6) and 13.8 (12.1); 1,000,000 rows
+// 36.5 (37.1) and 45 (39).
+constexpr uint32_t kMappedRows = 262144;
+
 // page-locked room for n rows' predictions
 int grow_out(ta3s_model* m, size_t n) {
     if (n <= m->cap_out) return 0;
@@ -883,7 +891,7 @@ int upload_rows(ta3s_model* m, float const* x, uint32_t n, bool standardize) {
     return 0;
 }
 
-Params make_params(ta3s_model* m, int batch, int32_t const* d_idx, int train) {
+Params make_params(ta3s_model* m, int batch, int32_t const* d_idx, int train, float* out = nullptr) {
     Params prm{};
     prm.x = m->d_x;
     prm.y = m->d_y;
@@ -892,7 +900,7 @@ Params make_params(ta3s_model* m, int batch, int32_t const* d_idx, int train) {
     prm.w1 = m->d_w1b;
     prm.w2 = m->d_w2b;
     prm.p32 = m->d_param;
-    prm.out = m->h_out;
+    prm.out = out;
     prm.partial = m->d_partial;
     prm.status = m->d_status;
     prm.inv_batch = 1.0f / float(batch);
@@ -900,10 +908,10 @@ Params make_params(ta3s_model* m, int batch, int32_t const* d_idx, int train) {
     return prm;
 }
 
-int launch_mlp(ta3s_model* m, int batch, int32_t const* d_idx, int train) {
+int launch_mlp(ta3s_model* m, int batch, int32_t const* d_idx, int train, float* out = nullptr) {
     int const ntiles = (batch + ROWS - 1) / ROWS;
     int const grid = std::min(ntiles, m->sms);
-    mlp_kernel<<<grid, THREADS, SMEM_BYTES, m->stream>>>(make_params(m, batch, d_idx, train));
+    mlp_kernel<<<grid, THREADS, SMEM_BYTES, m->stream>>>(make_params(m, batch, d_idx, train, out));
     TA3S_CUDA(m, cudaGetLastError(), "surrogate mlp launch");
     return 0;
 }
@@ -981,7 +989,7 @@ void ta3s_destroy(ta3s_model* m) {
     cudaSetDevice(m->device);
     for (void* p : {(void*)m->d_param, (void*)m->d_m, (void*)m->d_v, (void*)m->d_w1b, (void*)m->d_w2b,
                     (void*)m->d_partial, (void*)m->d_status, (void*)m->d_loss, (void*)m->d_xraw, (void*)m->d_x,
-                    (void*)m->d_y, (void*)m->d_idx, (void*)m->d_grad, (void*)m->d_stats, (void*)m->d_corr})
+                    (void*)m->d_y, (void*)m->d_idx, (void*)m->d_grad, (void*)m->d_out, (void*)m->d_stats, (void*)m->d_corr})
         if (p) cudaFree(p);
     if (m->h_status) cudaFreeHost(m->h_status);
     if (m->h_out) cudaFreeHost(m->h_out);
@@ -1155,10 +1163,15 @@ int ta3s_predict(ta3s_model* m, const float* x, uint32_t n, float* mean_out, flo
     if (!m || !x || !mean_out) return fail(m, "ta3s_predict: null argument");
     if (n == 0) return 0;
     TA3S_CUDA(m, cudaSetDevice(m->device), "set device");
-    if (grow_out(m, n) || upload_rows(m, x, n, false) || begin_kernels(m) || launch_mlp(m, int(n), nullptr, 0) ||
-        check_status(m))
+    bool const mapped = n <= kMappedRows;
+    if (mapped ? grow_out(m, n) : grow(m, m->d_out, m->cap_dout, size_t(n) * 2, "alloc predictions")) return 1;
+    if (upload_rows(m, x, n, false) || begin_kernels(m) || launch_mlp(m, int(n), nullptr, 0, mapped ? m->h_out : m->d_out))
         return 1;
-    float const* const out = m->h_out;
+    std::vector<float> copied(mapped ? 0 : size_t(n) * 2);
+    if (!mapped)
+        TA3S_CUDA(m, cudaMemcpyAsync(copied.data(), m->d_out, copied.size() * 4, cudaMemcpyDeviceToHost, m->stream), "outputs");
+    if (check_status(m)) return 1;
+    float const* const out = mapped ? m->h_out : copied.data();
     for (uint32_t r = 0; r < n; ++r) {
         mean_out[r] = out[2 * r] * m->y_std + m->y_mean;
         if (logvar_out) logvar_out[r] = out[2 * r + 1] + 2.f * std::log(m->y_std);
