@@ -102,6 +102,7 @@ void __cudaUnregisterFatBinary(void**) {}
 void __cudaRegisterFunction(void**, char const* fn, char*, char const* name, int, uint3*, uint3*, dim3*, dim3*, int*) {
     kernels()[fn] = name;
 }
+void __cudaRegisterVar(void**, char*, char*, char const*, int, size_t, int, int) {}
 unsigned __cudaPushCallConfiguration(dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {
     g_config = {grid, block, smem, stream};
     return 0;
@@ -133,6 +134,34 @@ cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp* p, int) {
     return call("cudaGetDeviceProperties");
 }
 cudaError_t cudaFuncSetAttribute(void const*, cudaFuncAttribute, int) { return call("cudaFuncSetAttribute"); }
+cudaError_t cudaGetDevice(int* d) {
+    *d = 0;
+    return call("cudaGetDevice");
+}
+cudaError_t cudaGetDeviceCount(int* n) {
+    *n = 1;
+    return call("cudaGetDeviceCount");
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
+    *v = a == cudaDevAttrMaxSharedMemoryPerMultiprocessor ? 233472
+         : a == cudaDevAttrReservedSharedMemoryPerBlock   ? 1024
+         : a == cudaDevAttrMultiProcessorCount            ? 148
+                                                          : 0;
+    return call("cudaDeviceGetAttribute");
+}
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, void const*) {
+    std::memset(a, 0, sizeof *a);
+    return call("cudaFuncGetAttributes");
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, void const*, int, size_t, unsigned) {
+    *n = 1;
+    return call("cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+}
+cudaError_t cudaGetSymbolAddress(void** p, void const*) {
+    static unsigned char word[4096];
+    *p = word;
+    return call("cudaGetSymbolAddress");
+}
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     *s = nullptr;
     return call("cudaStreamCreateWithFlags");
@@ -162,11 +191,13 @@ cudaError_t cudaFreeHost(void* p) {
 }
 cudaError_t cudaMemcpy(void* dst, void const* src, size_t bytes, cudaMemcpyKind) {
     if (cudaError_t e = call("cudaMemcpy")) return e;
+    if (bytes && (!dst || !src)) return g_last = cudaErrorInvalidValue;
     std::memcpy(dst, src, bytes);
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* dst, void const* src, size_t bytes, cudaMemcpyKind, cudaStream_t) {
     if (cudaError_t e = call("cudaMemcpyAsync")) return e;
+    if (bytes && (!dst || !src)) return g_last = cudaErrorInvalidValue;
     std::memcpy(dst, src, bytes);
     return cudaSuccess;
 }

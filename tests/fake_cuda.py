@@ -1,4 +1,4 @@
-"""The surrogates' host side on a stand-in for the CUDA runtime (tests/cpp/fake_cudart.cpp): no GPU, kernels do
+"""The library's host side on a stand-in for the CUDA runtime (tests/cpp/fake_cudart.cpp): no GPU, kernels do
 nothing, and any runtime call can be made to fail."""
 from __future__ import annotations
 
@@ -11,21 +11,24 @@ import numpy as np
 from conftest import ROOT
 
 
-def build(out_dir) -> C.CDLL:
+def build(out_dir, sources=("ta3s_surrogate.cu", "ta3s_wide.cu")) -> C.CDLL:
     from tetris_ai3_b200 import build as b
-    from tetris_ai3_b200.surrogate import _SIG
-    so = os.path.join(str(out_dir), "libfake_surrogate.so")
+    from tetris_ai3_b200 import evaluator, surrogate
+    so = os.path.join(str(out_dir), "libfake_%s.so" % sources[0].split(".")[0])
     # the kernels never run: PTX alone, without the assembler's minute
     subprocess.run([b.nvcc(), "-gencode", "arch=compute_100a,code=compute_100a", "-O1", "-std=c++20", "-fmad=false",
                     "-Xcompiler", "-fPIC", "-shared", "-Xlinker", "-Bsymbolic",     # (torch's runtime may be loaded too)
                     "--expt-relaxed-constexpr", "-cudart", "none",
                     "-I", os.path.join(ROOT, "include"), "-I", b.CSRC, "-o", so,
-                    os.path.join(b.CSRC, "ta3s_surrogate.cu"), os.path.join(b.CSRC, "ta3s_wide.cu"),
+                    *(os.path.join(b.CSRC, s) for s in sources),
                     os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp")], check=True)
-    lib = C.CDLL(so)
-    for name, (res, args) in _SIG.items():
-        f = getattr(lib, name)
-        f.restype, f.argtypes = res, args
+    if "ta3b_eval.cu" in sources:
+        lib = evaluator.library(so)
+    else:
+        lib = C.CDLL(so)
+        for name, (res, args) in surrogate._SIG.items():
+            f = getattr(lib, name)
+            f.restype, f.argtypes = res, args
     lib.fake_block.restype = C.c_void_p
     lib.fake_block.argtypes = [C.c_size_t]
     lib.fake_capture.argtypes = [C.c_char_p, C.c_int, C.c_size_t]

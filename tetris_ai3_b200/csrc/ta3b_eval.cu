@@ -1954,13 +1954,14 @@ int host_eval(ta3b_ctx* ctx, float const* weights, uint32_t num_islands, uint32_
     if (int rc = grow(ctx, ctx->d_w, ctx->cap_w, models * num_params, "alloc weights")) return rc;
     if (int rc = grow(ctx, ctx->d_seeds, ctx->cap_seeds, uint64_t(num_islands) * num_games, "alloc seeds")) return rc;
     if (ctx->cap_sims < sims) {
-        size_t c = ctx->cap_sims;
+        ctx->cap_sims = 0;                // (grow frees first: after a failure there is no room for any sims)
+        size_t c = 0;
         if (int rc = grow(ctx, ctx->d_score, c, sims, "alloc score")) return rc;
-        c = ctx->cap_sims;
+        c = 0;
         if (int rc = grow(ctx, ctx->d_pieces, c, sims, "alloc pieces")) return rc;
-        c = ctx->cap_sims;
+        c = 0;
         if (int rc = grow(ctx, ctx->d_lines, c, sims, "alloc lines")) return rc;
-        c = ctx->cap_sims;
+        c = 0;
         if (int rc = grow(ctx, ctx->d_evals, c, sims, "alloc evals")) return rc;
         ctx->cap_sims = sims;
     }
@@ -1972,9 +1973,10 @@ int host_eval(ta3b_ctx* ctx, float const* weights, uint32_t num_islands, uint32_
     if (tracing) {
         if (int rc = grow(ctx, ctx->d_trace, ctx->cap_trace, sims * max_moves * 3 + 1, "alloc trace")) return rc;
         if (ctx->cap_tb < sims) {
-            size_t c = ctx->cap_tb;
+            ctx->cap_tb = 0;
+            size_t c = 0;
             if (int rc = grow(ctx, ctx->d_nmoves, c, sims, "alloc n_moves")) return rc;
-            c = ctx->cap_tb;
+            c = 0;
             if (int rc = grow(ctx, ctx->d_board, c, sims * W, "alloc boards")) return rc;
             ctx->cap_tb = sims;
         }
