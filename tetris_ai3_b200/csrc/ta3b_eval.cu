@@ -17,8 +17,11 @@
 // candidates that clear a row or reach into the spawn rows are queued and
 // evaluated by the full reference algorithm in compacted 32-lane batches.
 // The top-K of a level is a warp-distributed sorted list (lane i holds the
-// i-th best packed key) maintained with ballots and shuffles, so level scores
-// never touch memory. Nothing in the move loop synchronises more than one warp.
+// i-th best packed key): keys above its threshold wait in a 32-entry buffer in
+// shared memory, which is sorted across the lanes and merged into the list when
+// it is full (v11), or enter the list at once (widened networks). Level scores
+// never leave the SM. Nothing in the move loop synchronises more than one warp
+// (a team's warps in the team kernels).
 #include "ta3b.h"
 #include "tables.h"
 #include "eval_core.h"
@@ -255,12 +258,10 @@ __device__ int engine_place(Engine& e, int o, int x, BoardInts& bi) {         //
 
 // ------------------------------------------------------------ candidates ---
 struct SmemW {                       // weights read from shared memory (broadcast loads)
-    static constexpr bool VEC4 = false;
     float const* p;
     __device__ __forceinline__ float operator()(int i) const { return p[i]; }
 };
 struct GlobalW {
-    static constexpr bool VEC4 = false;
     float const* p;
     __device__ __forceinline__ float operator()(int i) const { return __ldg(p + i); }
 };
@@ -741,7 +742,7 @@ __device__ __forceinline__ void count_illegal(WarpShared* ws, uint32_t seg, uint
 // candidates go through the full path without a record: a batch of it per warp takes less time than a fast
 // round, the batch of what that defers and the record that the leader's one lane builds (30 champion games 14.5
 // against 15.1 ms). With 16 warps an SM the instructions count, not the time of one warp: there the record
-// stays (a generation takes 245 ms with it, 248 without).
+// stays (a generation takes 1 % longer without it).
 __device__ __forceinline__ uint32_t root_entry(WarpShared const& ws, uint32_t c) {
     uint32_t const n0 = ws.seg[0].x >> 16;
     uint32_t const s = c >= n0 ? 1u : 0u;
@@ -784,7 +785,8 @@ __device__ __noinline__ int full_inputs_wide(WarpShared* ws, Luts lut, uint32_t 
 }
 
 // keys of a round above the threshold from which one sort and merge (260 instructions) beats inserting each
-// (20 and a chain of shuffles)
+// (20 and a chain of shuffles). Flat: with 5, 20 or never merging the widened cases take the same within 1 %,
+// always merging costs 3 % on the short games (wide 32, 16,000 sims, cap 60: 206 against 200 ms)
 constexpr int kMergeAbove = 10;
 
 // One level of the widened network: rounds of 64 candidates, two a lane, by the fast path, or (once 64 are
@@ -875,8 +877,9 @@ __device__ __forceinline__ LevelAcc level_pass_wide(WarpShared& ws, Luts lut, fl
 
 // One level: every candidate of the segment table, on the fast path or queued
 // for the full path (evaluated in compacted 32-lane batches). leaf: fold into
-// the argmax key and per-list legality; otherwise into the top-kl list and
-// per-parent legality. ws is the game's area, own the warp's own (its queue of deferred
+// the argmax key; otherwise into the top-kl list. Legality is not folded: only
+// the full path meets illegal candidates, and counts them per segment
+// (count_illegal; list_legal reads the counts). ws is the game's area, own the warp's own (its queue of deferred
 // candidates and its key buffer; the same area except in team kernels).
 // TEAM > 1: this warp takes every TEAM-th 32-candidate round, starting at candidate `first`.
 //
@@ -887,11 +890,11 @@ __device__ __forceinline__ LevelAcc level_pass_wide(WarpShared& ws, Luts lut, fl
 // sorted across the lanes and merged into the list, which raises thr; a key at or below a stale thr is
 // below the final list[kl-1] too. Team kernels sort in straight-line code (a warp alone on its scheduler
 // waits for every shuffle: 15.4 ms for 30 champion games, 16.9 ms with the loop), the single-warp kernels
-// in a loop (merge_keys: a generation takes 233 ms with it, 238 ms inserting each key at once). The
-// widened kernels insert or merge each round's keys at once (level_pass_wide; their warp areas have no buffer).
-// Measured with this loop, its records and placement data, start -> now: generation 341.6 -> 233.5 ms,
-// default generation 52.4 -> 36.0 ms, 30 champion games 17.9 -> 15.3 ms; 36,800 warp instructions a move of a
-// champion's game at 16 warps per SM (ncu).
+// in a loop (merge_keys: a generation 2 % faster than inserting each key at once). The widened kernels
+// insert or merge each round's keys at once (level_pass_wide; their warp areas have no buffer).
+// With this loop, its records and placement data 30 champion games went from 17.9 to 15.3 ms, a generation
+// (10,000 sims, cap 2,000) from 341.6 to 233.5 ms where the whole call takes 217 to 258 ms today depending on
+// the models drawn; a champion's move is 36,800 warp instructions at 16 warps per SM (ncu).
 template <bool KEYS, int TEAM = 1>
 __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, Luts lut, FastW const& fw, bool leaf,
                                                uint32_t total, int kl, int lane, uint32_t& evals, bool root,
@@ -905,7 +908,8 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
     // path; either way its keys are folded at one place. Keys are unique within a level, so the
     // fold order does not change the kept set. One drain site and one fold site keep the loop's
     // code small (the kernel is bound by instruction fetch as much as by issue). Two candidates
-    // per lane in straight-line code measured slower (681 ms vs 486 ms per full generation).
+    // per lane in straight-line code measured 40 % slower on an early build of this loop (not tried
+    // since; the widened networks gain by it, because their weights' loads serve both).
     uint32_t queued = 0;          // < 32 at the start of every fast round: the queue holds 64
     uint32_t kcnt = 0;            // keys in the key buffer (non-leaf levels)
     int seg = -1;
@@ -998,8 +1002,8 @@ __device__ __forceinline__ LevelAcc level_pass(WarpShared& ws, WarpShared& own, 
 // kept keys enter the top-K afterwards (expand_copies). Equality is exact: nodes are grouped by a hash of
 // the record's board words and compared word by word with their group's first node. On the generation
 // 21 % of all candidates are such copies (5 / 20 / 29 % at levels 1 / 2 / 3; 26 % in a champion's games).
-// Measured, start -> grouped: generation (10,000 sims, cap 2,000) 330.5 -> 311.5 ms, widened 64 (2,000 sims,
-// cap 200) 414.8 -> 335.1 ms, widened 32 (cap 300) 243.2 -> 194.0 ms.
+// Grouping alone, on the build it came to: generation (10,000 sims, cap 2,000) 330.5 -> 311.5 ms, widened 64
+// (2,000 sims, cap 200) 414.8 -> 335.1 ms, widened 32 (cap 300) 243.2 -> 194.0 ms.
 // dedup = false: every list stands for itself (the key-tracing flavour, whose second-best key may be a copy;
 // level 1 unless both root groups place the same piece, the only way to the same board there but for clears).
 __device__ __forceinline__ uint32_t build_segments(WarpShared& ws, uint32_t window, int tree, int level,
@@ -1643,19 +1647,25 @@ struct Variant {
 Variant const kVariants[] = {
     {eval_kernel<4, 3>, 4, 3}, {eval_kernel<4, 4>, 4, 4}, {eval_kernel<4, 5>, 4, 5}, {eval_kernel<4, 6>, 4, 6},
     {eval_kernel<2, 10>, 2, 10}, {eval_kernel<2, 12>, 2, 12},
-    // larger blocks (8 and 16 games per block, 256 / 512 threads), same 128-register cap
+    // larger blocks (8 and 16 games per block, 256 / 512 threads), same 128-register cap. 16 x 1 is the
+    // fastest on every full batch measured (10,000 sims, cap 300: 58.1 ms; 4 x 3 and 4 x 4 65, 8 x 2 65,
+    // 20 x 1 60, the others 70 to 78)
     {eval_kernel<8, 2>, 8, 2}, {eval_kernel<16, 1>, 16, 1},
-    // 20 warps per SM (the 68-word records leave room for them) at a ~100-register cap
+    // 20 warps per SM at a ~100-register cap. Shared memory holds the second shape's block once per SM, but
+    // only one of the first's (118,816 bytes each): it runs 10 warps an SM. Likewise seven of the 2-warp
+    // shapes' blocks are resident, four of the 4-warp ones
     {eval_kernel<10, 2>, 10, 2}, {eval_kernel<20, 1>, 20, 1},
     // two warps per game, 4 games per block (one block per SM, no register cap): batches of at
     // most 4 games per SM run on it by default
     {eval_kernel<8, 1, 0, false, false, 2>, 8, 1, 2},
-    // four warps per game (2 games per block): 55 vs 65 us per move at one game per SM, 63 vs 67 at
-    // two (eight warps per game measured 69 us: the per-warp top-K and the merges stop the gain)
+    // four warps per game (2 games per block): 49 us a move against 51 with two warps at one game per SM,
+    // 50.5 against 52 at two (eight warps per game were slower than four on an earlier build: the per-warp
+    // top-K and the merges stop the gain)
     {eval_kernel<8, 1, 0, false, false, 4>, 8, 1, 4},
 };
 // the default variant's hand-off flavour: its launch's tail (at most 4 games per SM) goes to the
-// paired kernel
+// paired kernel. 10,000 sims, cap 2,000: 257.5 ms (277 to 281 without); handing over at 2, 3 or 6 games per SM
+// 259.8, 258 and 257.4 ms; 10,010 uneven sims, cap 1,000: 222.7 (235), 224.7, 223.6 and 222.8 ms
 Variant const kHandoffVariant = {eval_kernel<16, 1, 0, false, false, 1, true>, 16, 1};
 constexpr int kNumVariants = int(sizeof(kVariants) / sizeof(kVariants[0]));
 // the networks a launch can run: v11, or the widened 10 -> H -> H -> 1 for H = 64 or 32
@@ -1668,9 +1678,13 @@ constexpr size_t warp_bytes(int ni) {
 // the widened networks' launch shapes (more registers per lane than v11, and a buffer of 64 candidates'
 // hidden units per warp): 8 warps an SM
 Variant const kWideNet[NUM_NETS] = {{nullptr, 0, 0}, {eval_kernel<4, 2, 64>, 4, 2}, {eval_kernel<4, 2, 32>, 4, 2}};
-// width 32 with room for 12 warps an SM (168 registers, 20 bytes of spills): better once every slot has
-// several games (16,000 sims, cap 60: 194.6 against 208.7 ms), worse on fewer, where a game's own speed
-// counts (2,000 sims, cap 300: 175.7 against 135.4 ms; 200 sims: 80.0 against 72.4)
+// width 32 with room for 12 warps an SM (168 registers, 20 bytes of spills) against 8 warps, the times of both:
+//   2,000 sims, cap 300: 175.7 / 135.4 ms; 200 sims: 80.0 / 72.4 (a game's own speed counts)
+//   4,000 sims: cap 60 63.2 / 62.9 ms, cap 300 208 / 258, cap 2,000 1.23 / 1.56 s
+//   7,200 sims: cap 60 98 / 107 ms, cap 300 351 / 378, cap 2,000 2.07 / 1.97 s
+//   16,000 sims: cap 60 200 / 216 ms, cap 300 715 / 770, cap 2,000 3.85 / 4.15 s; 80,000, cap 300 3.13 / 3.49 s
+// How the long games fall into waves decides between 2,000 and 10,000 sims; from four games a slot on (7,104 sims)
+// 12 warps win but for one case by 5 %
 Variant const kWide32Many = {eval_kernel<12, 1, 32>, 12, 1};
 constexpr uint32_t kManyPerSlot = 4;
 // the budget-checking flavours (shapes where the extra check spills nothing)
@@ -1680,6 +1694,13 @@ Variant const kBudgetNet[NUM_NETS] = {{eval_kernel<4, 3, 0, true>, 4, 3}, {eval_
 Variant const kKeysNet[NUM_NETS] = {{eval_kernel<4, 3, 0, false, true>, 4, 3},
                                     {eval_kernel<4, 2, 64, false, true>, 4, 2},
                                     {eval_kernel<4, 2, 32, false, true>, 4, 2}};
+// what a block asks for (its warps' areas and the placement tables) against a block's limit, 227 KB, and an SM's
+// 228 KB less 1 KB a block: the shapes that run by default have to be resident as declared
+constexpr size_t block_bytes(uint32_t warps, int ni) { return warps * warp_bytes(ni) + sizeof(LutTables); }
+static_assert(block_bytes(16, NET_V11) <= 232448 && block_bytes(20, NET_V11) <= 232448, "16 x 1, 20 x 1");
+static_assert(block_bytes(12, NET_W32) <= 232448, "width 32's large batches");
+static_assert(2 * (block_bytes(4, NET_W64) + 1024) <= 233472 && 2 * (block_bytes(4, NET_W32) + 1024) <= 233472, "widened, 4 x 2");
+static_assert(2 * (block_bytes(8, NET_V11) + 1024) <= 233472 && 4 * (block_bytes(4, NET_V11) + 1024) <= 233472, "8 x 2, teams, 4 x 4");
 constexpr int kNoAllocVariant = 1;   // the allocation-free entry point keeps its fixed 4 x 4 launch shape
 constexpr int kSmallVariant = 10;  // the paired kernel: the default for batches of at most 4 games per SM
 constexpr int kResumeVariant = kSmallVariant;   // the team kernel that finishes a hand-off's games
@@ -1858,8 +1879,9 @@ int launch(ta3b_ctx* ctx, Params const& prm, cudaStream_t st, int ni = NET_V11) 
     // with a time budget the budget-checking flavour runs, with key tracing the tracing flavour
     // (which runs without the budget); each has its own fixed launch shape
     // unless a variant was selected, a v11 batch of at most 4 games per SM runs on the paired kernel
-    // (two warps per game), whose moves take 0.62x the single-warp kernel's time at that load, and
-    // one of at most 2 games per SM on teams of four warps (0.53x)
+    // (two warps per game), one of at most 2 games per SM on teams of four. 300 moves of champions' games, in
+    // ms, single warps / pairs / fours: 1 game per SM 22.8 / 15.2 / 14.7; 2: 22.8 / 15.6 / 15.2; 3: 22.8 / 18.3
+    // / 29.3 (two waves); 4: 23.0 / 21.1 / 29.9; 6: 25.5 / 39.4
     Variant const& small = kVariants[kSmallVariant];
     Variant const& tiny = kVariants[kTinyVariant];
     bool const auto_small = ctx->auto_small && ni == NET_V11 && !keys && !budget;

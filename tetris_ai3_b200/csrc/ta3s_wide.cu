@@ -368,6 +368,7 @@ __global__ void __launch_bounds__(THREADS, 2) backward_kernel(GemmArgs dw2, Gemm
 }
 
 using GemmFn = void (*)(GemmArgs);
+// (layouts other than 0, 0 run in the backward kernels; as plain products only for ta3w_gemm_test)
 GemmFn gemm_fn(int a_mn, int b_mn) {
     return a_mn ? (b_mn ? gemm_kernel<1, 1> : gemm_kernel<1, 0>) : (b_mn ? gemm_kernel<0, 1> : gemm_kernel<0, 0>);
 }
@@ -465,7 +466,7 @@ __global__ void __launch_bounds__(HEAD_THREADS)
     // a warp moves whole rows (rows is a multiple of 128, h of 128): 16 bytes a lane, four rows in flight
     int const warp = tid >> 5, lane = tid & 31;
     for (int c = 4 * lane; c < h; c += 128) {
-        float const* const bp = p + off_b2 + c;                 // (the offset is even only)
+        float const* const bp = p + off_b2 + c;                 // (a multiple of 128: the widths before it are)
         float const b[4] = {bp[0], bp[1], bp[2], bp[3]};
         float4 q[HEAD_ROWS / 8];
 #pragma unroll
