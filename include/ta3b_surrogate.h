@@ -46,7 +46,8 @@ int ta3s_train(ta3s_model* m, uint32_t epochs, uint32_t batch, float lr, float w
                float* final_loss);
 /* predicted mean score (in target units) and log-variance for n rows [n][97].
  * Replaces the device copy of the training rows: call ta3s_set_data again
- * before the next ta3s_train. */
+ * before the next ta3s_train (which is refused otherwise, also after a
+ * prediction or a set_data call that failed). */
 int ta3s_predict(ta3s_model* m, const float* x, uint32_t n, float* mean_out, float* logvar_out);
 
 /* ---- the same scheme for any parameter-vector size (ta3w_*) ----
