@@ -1,6 +1,6 @@
 """Several AdamW steps in a row, where moments, weights and the minibatches' rows carry over from step to step:
 the v11 surrogate's cluster launch over ragged epochs and over more steps than one launch takes, and the
-widened surrogate's update in the epilogue. A step's gradients (which other tests hold against the checkers) are
+widened surrogate's update in the epilogue. A step's gradients (which other tests hold against float64) are
 those of gradients() over the same rows in the same order, and AdamW is float32 operations rounded one by one, so
 the parameters are equal bit for bit."""
 from __future__ import annotations
